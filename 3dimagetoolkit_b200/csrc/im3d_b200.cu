@@ -751,6 +751,12 @@ GsCoef<T> make_coef(double hx, double hy, double hz, double dt, double bc, int n
     c.ihy2d = 1.0 / (hy * hy);
     c.ihz2d = 1.0 / (hz * hz);
     c.diagd = 1.0 / dt + 2.0 * c.ihx2d + 2.0 * c.ihy2d + 2.0 * c.ihz2d;
+    c.pow2 = 0;
+    const double hs[3] = {hx, hy, hz};
+    for (int a = 0; a < 3; ++a) {
+        int e = 0;
+        if (std::frexp(hs[a] * hs[a], &e) == 0.5 && e > -1000 && e < 1000) c.pow2 |= 1 << a;
+    }
     return c;
 }
 
@@ -842,31 +848,56 @@ inline bool fits_int32(const Dims& d)
     return 2 * d.npk() < (1ll << 31);
 }
 
+// Planes per thread of the half-sweep: NI where its grid fills the GPU once (8 blocks per
+// SM), else 2, which splits a small volume over more blocks (FP32, us per half-sweep with 2
+// and 3 planes: 128^3 2.83 / 3.53, 160^3 4.63 / 3.79, 256^3 16.5 / 14.5, with 4 planes 14.6;
+// FP64, 2 and 4: 90x80x71 Neumann 2.9 / 4.2, 200^3 19.0 / 17.8).
+template <typename T> struct RbNI { static constexpr int v = sizeof(T) == 4 ? 3 : 4; };
+// blocks per SM of the half-sweep: 8 (64 registers); 7 and 9 measured slower
+constexpr int kRbMinB = 8;
+
+template <typename T, int NI, int BC, typename IX>
+int rb_march_launch(im3d_ctx* ctx, T* U, const T* B, const Dims& d, const GsCoef<T>& c, int color, int first)
+{
+    const long long npk = d.npk();
+    // red walks the planes forward, black backward: each half-sweep starts on the planes
+    // the previous one wrote last, which are still in L2
+    return launch_dependent(ctx, rb_march_kernel<T, NI, BC, BC == RB_NEU ? 1 : kRbMinB, IX>,
+                            grid_rb_flat<T>(d, kBlkVec, 1, NI), kBlkVec, U + (color ? npk : 0),
+                            (const T*)(U + (color ? 0 : npk)), B + (color ? npk : 0), d, c, color, color, first);
+}
+
+template <typename T, typename IX>
+int rb_march(im3d_ctx* ctx, T* U, const T* B, const Dims& d, const GsCoef<T>& c, int color, int first)
+{
+    constexpr int NI = RbNI<T>::v;
+    const dim3 g = grid_rb_flat<T>(d, kBlkVec, 1, NI);
+    const bool large = (long long)g.x * g.z >= 8ll * ctx->num_sms;
+    if (c.neu && c.bc != T(0)) return rb_march_launch<T, 1, RB_NEU, IX>(ctx, U, B, d, c, color, first);
+    if (c.neu)
+        return large ? rb_march_launch<T, NI, RB_NEU0, IX>(ctx, U, B, d, c, color, first)
+                     : rb_march_launch<T, 2, RB_NEU0, IX>(ctx, U, B, d, c, color, first);
+    return large ? rb_march_launch<T, NI, RB_DIR, IX>(ctx, U, B, d, c, color, first)
+                 : rb_march_launch<T, 2, RB_DIR, IX>(ctx, U, B, d, c, color, first);
+}
+
+// One sweep (red, then black). use_self / omega != 1: the general kernel, which reads the
+// own value; else the residual solve's half-sweep on b_eff. first: B was written by the
+// kernel launched just before.
 template <typename T>
 int rb_sweep(im3d_ctx* ctx, T* U, const T* B, const Dims& d, const GsCoef<T>& c, int use_self,
-             double omega)
+             double omega, int first = 0)
 {
-    // the b_eff solve (no own value, omega 1) gets instantiations without the unused
-    // paths; with Dirichlet conditions and FP32 it fits 8 blocks per SM
     const bool self = use_self || omega != 1.0;
-    const dim3 grid = grid_rb_flat<T>(d, kBlkVec);
     for (int color = 0; color < 2; ++color) {
         const int pf = prof_begin(ctx, "rb_half");
-        // red walks the planes forward, black backward: each half-sweep starts on the
-        // planes the previous one wrote last, which are still in L2
-        const int reverse = color;
         if (self)
-            IM3D_TRY(launch_dependent(ctx, rb_half_vec_kernel<T, kNV, true, true>, grid, kBlkVec, U,
-                                      B, d, c, color, use_self, (T)omega, reverse));
-        else if (c.neu)
-            IM3D_TRY(launch_dependent(ctx, rb_half_vec_kernel<T, kNV, false, true>, grid, kBlkVec,
-                                      U, B, d, c, color, 0, T(1), reverse));
+            IM3D_TRY(launch_dependent(ctx, rb_half_vec_kernel<T, kNV>, grid_rb_flat<T>(d, kBlkVec), kBlkVec, U, B, d,
+                                      c, color, use_self, (T)omega, color));
         else if (fits_int32(d))
-            IM3D_TRY(launch_dependent(ctx, rb_half_vec_kernel<T, kNV, false, false, sizeof(T) == 4 ? 8 : 1, int>,
-                                      grid, kBlkVec, U, B, d, c, color, 0, T(1), reverse));
+            IM3D_TRY((rb_march<T, int>(ctx, U, B, d, c, color, first && !color)));
         else
-            IM3D_TRY(launch_dependent(ctx, rb_half_vec_kernel<T, kNV, false, false, sizeof(T) == 4 ? 8 : 1>,
-                                      grid, kBlkVec, U, B, d, c, color, 0, T(1), reverse));
+            IM3D_TRY((rb_march<T, long long>(ctx, U, B, d, c, color, first && !color)));
         prof_end(ctx, pf);
         IM3D_TRY(check_launch(ctx, "rb_half"));
     }
@@ -970,7 +1001,7 @@ int rb_solve(im3d_ctx* ctx, T* U, const T* B, const Dims& d, const GsCoef<T>& c,
     *conv = false;
     *rel = -1;
     while (s < max_sweeps) {
-        IM3D_TRY(rb_sweep(ctx, U, B, d, c, 0, omega));
+        IM3D_TRY(rb_sweep(ctx, U, B, d, c, 0, omega, s == 0));
         ++s;
         if (s >= next || s == max_sweeps) {
             double r = 0;
@@ -2265,9 +2296,9 @@ int worklist_group(im3d_ctx* ctx, const std::vector<int>& ids, const im3d_volume
     using KRhs = ConvKWinJob<T, 2, S, kKwT, kKwR, LdVec<T, 2>, StRhs<T>, KWinRG<T, 2>::v>;
     using FitM = FitMarchJob<S, kMarchJB, kMarchD, kMarchU, MarchMinB<S>::v>;
     using FitW = FitWinJob<T, S, TW, TY, TileA<T>::v>;
-    constexpr int RB_MINB = sizeof(T) == 4 ? 8 : 1;
-    using RbD = RbHalfJob<T, kNV, false, RB_MINB>;
-    using RbN = RbHalfJob<T, kNV, true, 1>;
+    constexpr int RB_MINB = kRbMinB, RB_NI = RbNI<T>::v;
+    using RbD = RbHalfJob<T, RB_NI, RB_DIR>;
+    using RbN = RbHalfJob<T, RB_NI, RB_NEU0>;
     using Res = RbResidualJob<T, kNVres>;
     using ClV = ClampTolJob<T, kNV, true>;
     using ClS = ClampTolJob<T, kNI, false>;
@@ -2323,7 +2354,7 @@ int worklist_group(im3d_ctx* ctx, const std::vector<int>& ids, const im3d_volume
         } else {
             jfw.h.push_back({FitW{v.W2, v.P1, v.f1_d, v.f2_d, d, v.tp.w[0], l1, l2}, fit_win_grid<T>(d)});
         }
-        const dim3 gpk = grid_rb_flat<T>(d, kBlkVec);
+        const dim3 gpk = grid_rb_flat<T>(d, kBlkVec, 1, RB_NI);
         for (int c = 0; c < 2; ++c) {
             // red walks the planes forward, black backward (rb_sweep)
             jrd[c].h.push_back({RbD{v.upk, v.bpk, d, v.coef, c, c}, gpk});
@@ -2451,6 +2482,8 @@ int worklist_group(im3d_ctx* ctx, const std::vector<int>& ids, const im3d_volume
         // control blocks are one range
         auto solve_group = [&](im3d_ctx* sc, const std::vector<int>& grp) -> int {
             std::vector<int> solving = grp, due, flags, still;
+            const std::vector<int> ones(grp.size(), 1);
+            bool first = true;
             const int q0 = grp.front(), q1 = grp.back() + 1;
             while (!solving.empty()) {
                 int k = maxs;
@@ -2458,12 +2491,14 @@ int worklist_group(im3d_ctx* ctx, const std::vector<int>& ids, const im3d_volume
                 k = std::max(k, 1);
                 for (int i = 0; i < k; ++i)
                     for (int c = 0; c < 2; ++c) {
+                        // the subgroup's first half-sweep follows the forcing terms
+                        const int* fl = first && i == 0 && c == 0 ? ones.data() : nullptr;
                         if (neu)
-                            IM3D_TRY((wl_launch<RbN, 128, 1>(sc, jrn[c], solving, nullptr, kBlkVec, 0, "rb_half", true)));
+                            IM3D_TRY((wl_launch<RbN, 128, RB_MINB>(sc, jrn[c], solving, fl, kBlkVec, 0, "rb_half", true)));
                         else
-                            IM3D_TRY((wl_launch<RbD, 128, RB_MINB>(sc, jrd[c], solving, nullptr, kBlkVec, 0, "rb_half",
-                                                                   true)));
+                            IM3D_TRY((wl_launch<RbD, 128, RB_MINB>(sc, jrd[c], solving, fl, kBlkVec, 0, "rb_half", true)));
                     }
+                first = false;
                 due.clear();
                 flags.clear();
                 for (int q : solving) {

@@ -1104,7 +1104,19 @@ struct GsCoef {
     int neu;
     // FP64 forms for the residual: 1/h^2 and the diagonal 1/dt + 2/hx^2 + 2/hy^2 + 2/hz^2
     double ihx2d, ihy2d, ihz2d, diagd;
+    // bit a set: h^2 of axis a is a power of two, so that x / h^2 == x * (1 / h^2) exactly
+    int pow2;
 };
+
+// The neighbour terms of the FP64 update divide by h^2 (poisson_imp.hxx:400); where h^2 is
+// a power of two the product with its (exact) reciprocal is the same number.
+template <int AXIS, typename T>
+__device__ __forceinline__ double over_h2(double x, const GsCoef<T>& c)
+{
+    const double h = AXIS == 0 ? c.hx : AXIS == 1 ? c.hy : c.hz;
+    const double r = AXIS == 0 ? c.ihx2d : AXIS == 1 ? c.ihy2d : c.ihz2d;
+    return (c.pow2 >> AXIS & 1) ? x * r : x / (h * h);
+}
 
 // One Gauss-Seidel point value (sum of neighbour terms + b + self/dt) * htilde;
 // `self_dt` is self/dt (beff mode folds u_in/dt into b and passes 0).
@@ -1250,16 +1262,15 @@ __device__ __forceinline__ void flat_pair(const uint3 blockIdx, unsigned groups,
 // All points of a packed row share the parity of k, so their k neighbours are the
 // other colour at (m-1, m) (k even) or (m, m+1) (k odd): one 16-byte vector plus one
 // scalar. The i neighbours come from a register window of vectors along i.
-// SELF: the point's own old value is read (use_self or omega != 1); the Poisson solve
-// on b_eff needs neither. NEU: the Neumann boundary rule is compiled in (c.neu must
-// match). Without both the kernel needs fewer registers and fits MINB blocks per SM.
+// General form: the point's own old value (use_self or omega != 1) and both boundary
+// rules; the residual solve with omega 1 runs rb_march_kernel instead.
 // reverse: the blocks take the planes of i from the last to the first, so that a
 // half-sweep following one in the other direction starts on the planes that are still
-// in L2. IX: the type of the cell offsets, int where both colours' cells number less
-// than 2^31 (fewer instructions per address), else long long.
-template <typename T, int NI, bool SELF = true, bool NEU = true, int MINB = 1, typename IX = long long>
-__device__ __forceinline__ void rb_half_vec_body(const uint3 blockIdx, const dim3 gridDim, T* __restrict__ U, const T* __restrict__ B, Dims d, GsCoef<T> c, int color, int use_self, T omega, int reverse)
+// in L2.
+template <typename T, int NI>
+__global__ void __launch_bounds__(128) rb_half_vec_kernel(T* __restrict__ U, const T* __restrict__ B, Dims d, GsCoef<T> c, int color, int use_self, T omega, int reverse)
 {
+    typedef long long IX;
     typedef V16<T> VT;
     typedef typename VT::type VV;
     constexpr int W = VT::W;
@@ -1281,8 +1292,7 @@ __device__ __forceinline__ void rb_half_vec_body(const uint3 blockIdx, const dim
     const T* bb = B + (color ? npk : 0);
     const bool jint = j >= 1 && j <= d.ny - 2;
     const IX q0 = ((IX)i0 * d.ny + j) * hz + m0;
-    const bool relax = SELF && omega != T(1);
-    if (!SELF) use_self = 0;
+    const bool relax = omega != T(1);
     // Every load of the NI planes is issued before the first store: the stores go to
     // the same array, so loads placed after one could not be moved ahead of it and each
     // thread would pay one memory round trip per plane.
@@ -1308,7 +1318,7 @@ __device__ __forceinline__ void rb_half_vec_body(const uint3 blockIdx, const dim
             // the k neighbour not in the centre vector: m0-1 (k even) or m0+W (k odd)
             const bool e_ok = par ? (m0 + W < hz) : (m0 >= 1);
             if (e_ok) exv[t] = oth[par ? q + W : q - 1];
-            if (SELF && (use_self || relax)) sfv[t] = *reinterpret_cast<const VV*>(own + q);
+            if (use_self || relax) sfv[t] = *reinterpret_cast<const VV*>(own + q);
         }
     }
 #pragma unroll
@@ -1344,7 +1354,7 @@ __device__ __forceinline__ void rb_half_vec_body(const uint3 blockIdx, const dim
                 const T sf = VT::get(self, cc);
                 T v;
                 if (std::is_same<T, double>::value) {
-                    double acc = sx / (c.hx * c.hx) + sy / (c.hy * c.hy) + sz / (c.hz * c.hz) + b;
+                    double acc = over_h2<0>(sx, c) + over_h2<1>(sy, c) + over_h2<2>(sz, c) + b;
                     if (use_self) acc = acc + sf / c.dt;
                     v = T(acc * (double)c.htilde[7]);
                 } else {
@@ -1365,7 +1375,7 @@ __device__ __forceinline__ void rb_half_vec_body(const uint3 blockIdx, const dim
                 }
             }
         }
-        if (NEU && c.neu) {
+        if (c.neu) {
             // Neumann: boundary points (faces of i, j or k) through the generic rule
 #pragma unroll
             for (int cc = 0; cc < W; ++cc) {
@@ -1382,10 +1392,231 @@ __device__ __forceinline__ void rb_half_vec_body(const uint3 blockIdx, const dim
     }
 }
 
-template <typename T, int NI, bool SELF = true, bool NEU = true, int MINB = 1, typename IX = long long>
-__global__ void __launch_bounds__(128, MINB) rb_half_vec_kernel(T* __restrict__ U, const T* __restrict__ B, Dims d, GsCoef<T> c, int color, int use_self, T omega, int reverse = 0)
+// The W cells of one packed row group: neighbour sums in, updated values out. FP32 runs
+// on the paired FP32 instructions (per component the scalar operations).
+template <typename T>
+struct RbRow;
+template <>
+struct RbRow<float> {
+    static __device__ __forceinline__ float4 update(const GsCoef<float>& c, const float4& xm, const float4& xp,
+                                                    const float4& ym, const float4& yp, const float4& zc,
+                                                    const float4& zn, const float4& b, const float (&ht)[4],
+                                                    const float (&hl)[4])
+    {
+        auto pair = [&](float2 a0, float2 a1, float2 b0, float2 b1, float2 c0, float2 c1, float2 bv, float2 h,
+                        float2 l) {
+            const float2 sx = __fadd2_rn(a0, a1), sy = __fadd2_rn(b0, b1), sz = __fadd2_rn(c0, c1);
+            const float2 acc = __ffma2_rn(sx, make_float2(c.ihx2, c.ihx2),
+                                          __ffma2_rn(sy, make_float2(c.ihy2, c.ihy2),
+                                                     __ffma2_rn(sz, make_float2(c.ihz2, c.ihz2), bv)));
+            return __ffma2_rn(acc, h, __fmul2_rn(acc, l));
+        };
+        const float2 lo = pair(make_float2(xm.x, xm.y), make_float2(xp.x, xp.y), make_float2(ym.x, ym.y),
+                               make_float2(yp.x, yp.y), make_float2(zc.x, zc.y), make_float2(zn.x, zn.y),
+                               make_float2(b.x, b.y), make_float2(ht[0], ht[1]), make_float2(hl[0], hl[1]));
+        const float2 hi = pair(make_float2(xm.z, xm.w), make_float2(xp.z, xp.w), make_float2(ym.z, ym.w),
+                               make_float2(yp.z, yp.w), make_float2(zc.z, zc.w), make_float2(zn.z, zn.w),
+                               make_float2(b.z, b.w), make_float2(ht[2], ht[3]), make_float2(hl[2], hl[3]));
+        return make_float4(lo.x, lo.y, hi.x, hi.y);
+    }
+};
+template <>
+struct RbRow<double> {
+    static __device__ __forceinline__ double2 update(const GsCoef<double>& c, const double2& xm, const double2& xp,
+                                                     const double2& ym, const double2& yp, const double2& zc,
+                                                     const double2& zn, const double2& b, const double (&ht)[2],
+                                                     const double (&)[2])
+    {
+        double2 o;
+        o.x = (over_h2<0>(xm.x + xp.x, c) + over_h2<1>(ym.x + yp.x, c) + over_h2<2>(zc.x + zn.x, c) + b.x) * ht[0];
+        o.y = (over_h2<0>(xm.y + xp.y, c) + over_h2<1>(ym.y + yp.y, c) + over_h2<2>(zc.y + zn.y, c) + b.y) * ht[1];
+        return o;
+    }
+};
+
+// 16-byte accesses with an L2 eviction policy (createpolicy).
+__device__ __forceinline__ uint64_t l2_evict_first()
 {
-    rb_half_vec_body<T, NI, SELF, NEU, MINB, IX>(blockIdx, gridDim, U, B, d, c, color, use_self, omega, reverse);
+    uint64_t p;
+    asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+    return p;
+}
+__device__ __forceinline__ uint64_t l2_evict_last()
+{
+    uint64_t p;
+    asm("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
+    return p;
+}
+__device__ __forceinline__ float4 ld16_hint(const float4* a, uint64_t policy)
+{
+    float4 v;
+    asm volatile("ld.global.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "l"(a), "l"(policy));
+    return v;
+}
+__device__ __forceinline__ void st16_hint(float4* a, const float4& v, uint64_t policy)
+{
+    asm volatile("st.global.L2::cache_hint.v4.f32 [%0], {%1, %2, %3, %4}, %5;"
+                 ::"l"(a), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "l"(policy)
+                 : "memory");
+}
+
+// Boundary rules of rb_march_kernel: Dirichlet; Neumann with value 0 (the segmentation
+// loop's); Neumann with any value.
+enum { RB_DIR = 0, RB_NEU0 = 1, RB_NEU = 2 };
+
+// Half-sweep of the residual solve: own value and relaxation out of the way, the updated
+// colour `own` and the other colour `oth` as separate pointers, so that no store holds a
+// load back. One thread per group of W = 16/sizeof(T) packed cells of row j, marching over
+// NI planes of i with the next plane's reads in flight. Every cell of a group is computed
+// by the interior formula, without a test per cell:
+//  * the k neighbours are the group itself and the group shifted by one cell (the parity of
+//    the row picks the direction);
+//  * Dirichlet: the cells on the k faces, which the interior formula does not apply to,
+//    are written with their value again (bc; the padding after the row stays 0), and rows
+//    on the other faces have no work;
+//  * Neumann: a missing neighbour is replaced before the sum by the ghost value -bcn h (low
+//    face) or +bcn h (high face) of NeuGaussSeidel (poisson_imp.hxx:23-336), which is 0 for
+//    RB_NEU0, and the diagonal is the face's.
+// first: the launch follows the kernel that wrote b_eff, so b_eff is read only after the
+// wait; later half-sweeps read it before (it was complete when the launch they depend on
+// passed its own wait), which overlaps the previous half-sweep's tail.
+// FP32: b_eff is read with evict_first and u written with evict_last, so that u (67 MB at
+// 256^3, which with b_eff's 67 MB exceeds the 126 MB L2) stays in L2 between half-sweeps:
+// 17.3 -> 14.6 us at 256^3. FP64 measured slower with the policies (4.9 -> 5.5 us at 128^3).
+// What bounds it: L2 bandwidth (about 15 B per cell from NI + 2 planes per NI and the rows
+// around a block), DRAM for b_eff. Measured us per half-sweep in sequence, against the
+// general kernel's form of it (54 instructions per cell): 256^3 FP32 17.0 -> 14.0,
+// 512x512x320 88.6 -> 83.4, 160^3 5.2 -> 4.0, 171x203x117 FP32 Neumann 14.0 -> 5.7,
+// 128^3 FP64 7.5 -> 4.9 and 200^3 FP64 28.4 -> 17.9 (no division per cell, over_h2).
+template <typename T, int NI, int BC, typename IX>
+__device__ __forceinline__ void rb_march_body(const uint3 blockIdx, const dim3 gridDim, T* __restrict__ own,
+                                              const T* __restrict__ oth, const T* __restrict__ bb, const Dims& d,
+                                              const GsCoef<T>& c, int color, int reverse, int first)
+{
+    typedef V16<T> VT;
+    typedef typename VT::type VV;
+    constexpr int W = VT::W;
+    constexpr bool NEU = BC != RB_DIR;
+    int g, j;
+    const int hz = d.hz();
+    flat_pair(blockIdx, (unsigned)(hz / W), g, j);
+    const int lo = NEU ? 0 : 1;
+    const int ib = (int)(reverse ? gridDim.z - 1 - blockIdx.z : blockIdx.z) * NI;
+    const int i0 = ib < lo ? lo : ib, i1 = min(ib + NI, d.nx - lo);
+    const int m0 = g * W;
+    const bool live = j >= lo && j < d.ny - lo && i0 < i1;
+    const IX plane = (IX)d.ny * hz;
+    const IX q0 = ((IX)i0 * d.ny + j) * hz + m0;
+    const T* pb = bb + q0;
+    auto ld_b = [](const T* p) {
+        if constexpr (sizeof(T) == 4) return ld16_hint(reinterpret_cast<const VV*>(p), l2_evict_first());
+        else return *reinterpret_cast<const VV*>(p);
+    };
+    VV bn = VV{};
+    if (!first && live) bn = ld_b(pb);
+    // Launched as a programmatic dependent of the previous half-sweep: wait until its
+    // writes are visible, then let the next half-sweep's blocks be scheduled while this
+    // one drains (both are no-ops in an ordinary launch).
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (!live) return;
+    if (first) bn = ld_b(pb);
+    const T* po = oth + q0;
+    T* pw = own + q0;
+    const int cy = j == 0 ? 0 : (j == d.ny - 1 ? 2 : 1);
+    const bool has_ym = !NEU || cy != 0, has_yp = !NEU || cy != 2;
+    int par = (i0 + j + color) & 1;
+    // the reads of one plane: the group's y neighbours and the k neighbour outside the group
+    VV xm = VV{}, xc, ymn = VV{}, ypn = VV{};
+    T en = T(0);
+    auto side = [&](const T* p, int pr) {
+        if (has_ym) ymn = *reinterpret_cast<const VV*>(p - hz);
+        if (has_yp) ypn = *reinterpret_cast<const VV*>(p + hz);
+        const bool e_ok = pr ? m0 + W < hz : m0 >= 1;
+        en = e_ok ? p[pr ? W : -1] : T(0);
+    };
+    if (!NEU || i0 >= 1) xm = *reinterpret_cast<const VV*>(po - plane);
+    xc = *reinterpret_cast<const VV*>(po);
+    side(po, par);
+#pragma unroll
+    for (int t = 0; t < NI; ++t) {
+        const int i = i0 + t;
+        if (i >= i1) break;
+        VV ym = ymn, yp = ypn, xp = VV{};
+        const VV bv = bn;
+        const T extra = en;
+        if (!NEU || i + 1 < d.nx) xp = *reinterpret_cast<const VV*>(po + plane);
+        if (t + 1 < NI && i + 1 < i1) {
+            side(po + plane, par ^ 1);
+            pb += plane;
+            bn = ld_b(pb);
+        }
+        VV zc = xc, zn;
+#pragma unroll
+        for (int cc = 0; cc < W; ++cc)
+            VT::set(zn, cc, par ? (cc + 1 < W ? VT::get(xc, cc + 1) : extra) : (cc >= 1 ? VT::get(xc, cc - 1) : extra));
+        // cells of the group on the faces k = 0 and k = nz - 1, and past the row
+        const bool first_k = par == 0 && m0 == 0;         // cell 0 has k = 0
+        const int last = ((d.nz - 1 - par) >> 1) - m0;    // the last cell with k < nz
+        const bool last_k = ((d.nz - 1 - par) & 1) == 0;  // ... and whether its k is nz - 1
+        T ht[W], hl[W];
+        VV xa = xm, xb = xp;
+        if constexpr (!NEU) {
+#pragma unroll
+            for (int cc = 0; cc < W; ++cc) {
+                ht[cc] = c.htilde[7];
+                hl[cc] = c.htilde_lo[7];
+            }
+        } else {
+            const int cx = i == 0 ? 0 : (i == d.nx - 1 ? 2 : 1);
+            const int nb = (cx != 1) + (cy != 1), m = (cx == 1) | ((cy == 1) << 1);
+            const T hin = c.htilde[m | 4], hon = c.htilde[m], lin = c.htilde_lo[m | 4], lon = c.htilde_lo[m];
+#pragma unroll
+            for (int cc = 0; cc < W; ++cc) {
+                const bool at0 = cc == 0 && first_k, at1 = last_k && cc == last;
+                ht[cc] = at0 || at1 ? hon : hin;
+                hl[cc] = at0 || at1 ? lon : lin;
+                if constexpr (BC == RB_NEU) {
+                    const T bcn = c.bcn[at0 || at1 ? nb + 1 : nb];
+                    if (cx == 0) VT::set(xa, cc, -(bcn * T(c.hx)));
+                    if (cx == 2) VT::set(xb, cc, bcn * T(c.hx));
+                    if (cy == 0) VT::set(ym, cc, -(bcn * T(c.hy)));
+                    if (cy == 2) VT::set(yp, cc, bcn * T(c.hy));
+                    if (at0) VT::set(zn, cc, -(bcn * T(c.hz)));
+                    if (at1) {
+                        if (par) VT::set(zn, cc, bcn * T(c.hz));
+                        else VT::set(zc, cc, bcn * T(c.hz));
+                    }
+                } else {
+                    if (at1) {
+                        if (par) VT::set(zn, cc, T(0));
+                        else VT::set(zc, cc, T(0));
+                    }
+                }
+            }
+        }
+        VV v = RbRow<T>::update(c, xa, xb, ym, yp, zc, zn, bv, ht, hl);
+#pragma unroll
+        for (int cc = 0; cc < W; ++cc) {
+            if (!NEU && ((cc == 0 && first_k) || (last_k && cc == last))) VT::set(v, cc, c.bc);
+            if (cc > last) VT::set(v, cc, T(0));
+        }
+        if constexpr (sizeof(T) == 4) st16_hint(reinterpret_cast<VV*>(pw), v, l2_evict_last());
+        else *reinterpret_cast<VV*>(pw) = v;
+        pw += plane;
+        po += plane;
+        xm = xc;
+        xc = xp;
+        par ^= 1;
+    }
+}
+
+template <typename T, int NI, int BC, int MINB, typename IX>
+__global__ void __launch_bounds__(128, MINB) rb_march_kernel(T* __restrict__ own, const T* __restrict__ oth, const T* __restrict__ bb, Dims d, GsCoef<T> c, int color, int reverse, int first)
+{
+    rb_march_body<T, NI, BC, IX>(blockIdx, gridDim, own, oth, bb, d, c, color, reverse, first);
 }
 
 // Vectorised FP64 residual, same walk as rb_half_vec_kernel; blockIdx.z covers

@@ -118,17 +118,20 @@ struct FitWinJob {
     }
 };
 
-// A half-sweep of the residual solve (no own value, omega 1).
-template <typename T, int NI, bool NEU, int MINB>
+// A half-sweep of the residual solve (no own value, omega 1). flag: the launch follows the
+// kernel that wrote b_eff.
+template <typename T, int NI, int BC>
 struct RbHalfJob {
     T* U;
     const T* B;
     Dims d;
     GsCoef<T> c;
     int color, reverse;
-    __device__ __forceinline__ void operator()(uint3 b, dim3 g, int) const
+    __device__ __forceinline__ void operator()(uint3 b, dim3 g, int flag) const
     {
-        rb_half_vec_body<T, NI, false, NEU, MINB>(b, g, U, B, d, c, color, 0, T(1), reverse);
+        const long long npk = d.npk();
+        rb_march_body<T, NI, BC, long long>(b, g, U + (color ? npk : 0), U + (color ? 0 : npk), B + (color ? npk : 0),
+                                            d, c, color, reverse, flag);
     }
 };
 
