@@ -80,6 +80,7 @@ struct im3d_ctx {
     int batch_mode = IM3D_BATCH_AUTO;
     int tile_loads = 1;  // the FP32 Heaviside pass moves its rows with TMA where it can
     int num_sms = 148;
+    int lex_key[4] = {0, 0, 0, 0};  // tile counts and sweeps of the lexicographic task list held in "lex_tasks"
     int ifit_chunks = 0;  // i chunks of the marching fit stage (0: cost model)
     size_t mem_limit = 0;  // device bytes the context may hold in buffers (0: no limit)
     size_t mem_held = 0;   // device bytes it holds in buffers now
@@ -757,34 +758,95 @@ GsCoef<T> make_coef(double hx, double hy, double hz, double dt, double bc, int n
         int e = 0;
         if (std::frexp(hs[a] * hs[a], &e) == 0.5 && e > -1000 && e < 1000) c.pow2 |= 1 << a;
     }
+    int e = 0;
+    if (std::frexp(dt, &e) == 0.5 && e > -1000 && e < 1000) c.pow2 |= 8;
+    c.idtd = 1.0 / dt;
     return c;
 }
 
-// One lexicographic sweep, reference order, natural layout, in place.
+// Lexicographic sweeps, reference order, natural layout, in place (lex_tile_kernel). The
+// task list depends on the tile counts and the number of sweeps only; the context keeps the
+// last one. A wait that gave up raises ctrl flag 1.
 template <typename T>
-int lex_sweep(im3d_ctx* ctx, T* r, const T* b, const Dims& d, const GsCoef<T>& c)
+int lex_sweeps(im3d_ctx* ctx, T* r, const T* b, const Dims& d, const GsCoef<T>& c, int sweeps)
 {
+    if (sweeps < 1) return IM3D_OK;
     if (!c.neu) {
         dir_faces_kernel<T><<<grid_vol(d, kBlkVol), kBlkVol, 0, ctx->stream>>>(r, d, c.bc);
         IM3D_TRY(check_launch(ctx, "dir_faces"));
     }
-    const int lo = c.neu ? 0 : 1;
-    const int hix = d.nx - lo, hiy = d.ny - lo, hiz = d.nz - lo;
-    if (hix <= lo || hiy <= lo || hiz <= lo) return IM3D_OK;
-    const dim3 blk(32, 4);
+    LexArgs a;
+    a.lo = c.neu ? 0 : 1;
+    auto tiles = [&](int n) { return (n - 2 * a.lo + kLexT - 1) / kLexT; };
+    a.nti = tiles(d.nx);
+    a.ntj = tiles(d.ny);
+    a.ntk = tiles(d.nz);
+    const long long nt = (long long)a.nti * a.ntj * a.ntk;
+    // sweeps of one launch: the list stays below a few million tasks
+    const int per = (int)std::max<long long>(1, std::min<long long>(std::min(sweeps, 32768), (1ll << 22) / nt));
+    if (nt > 0x7fffffffLL / 2) return fail(ctx, IM3D_ERR_INVALID_ARG, "volume too large for the launch geometry");
+    int* state = nullptr;  // task counter, then the sweeps finished per tile
+    IM3D_TRY(tbuf<int>(ctx, "lex_state", (size_t)nt + 1, &state));
+    a.next = state;
+    a.done = state + 1;
+    a.err = &ctx->ctrl_d->flag[1];
+    // FP64 without a division where the spacings and dt allow it (FP32 never divides)
+    auto kern = sizeof(T) == 8 && c.pow2 == 15 ? lex_tile_kernel<T, true> : lex_tile_kernel<T, false>;
+    const size_t smem = lex_smem<T>();
+    IM3D_TRY(set_smem(ctx, kern, smem));
+    int occ = 0;
+    IM3D_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kLexT * kLexT, smem));
+    if (occ < 1) return fail(ctx, IM3D_ERR_UNSUPPORTED, "the lexicographic sweep does not fit an SM");
     const int pf = prof_begin(ctx, "lex_sweep");
-    for (int s = 3 * lo; s <= (hix - 1) + (hiy - 1) + (hiz - 1); ++s) {
-        const int i0 = std::max(lo, s - (hiy - 1) - (hiz - 1));
-        const int i1 = std::min(hix - 1, s - 2 * lo);
-        if (i0 > i1) continue;
-        const int j0 = std::max(lo, s - i1 - (hiz - 1));
-        const int j1 = std::min(hiy - 1, s - i0 - lo);
-        if (j0 > j1) continue;
-        dim3 grid((j1 - j0 + 1 + blk.x - 1) / blk.x, (i1 - i0 + 1 + blk.y - 1) / blk.y);
-        lex_plane_kernel<T><<<grid, blk, 0, ctx->stream>>>(r, b, d, c, s, lo, i0, j0);
-        IM3D_TRY(check_launch(ctx, "lex_plane"));
+    for (int s0 = 0; s0 < sweeps; s0 += per) {
+        const int ns = std::min(per, sweeps - s0);
+        const int key[4] = {a.nti, a.ntj, a.ntk, ns};
+        unsigned long long* tasks = nullptr;
+        const size_t count = (size_t)nt * ns;
+        IM3D_TRY(tbuf<unsigned long long>(ctx, "lex_tasks", count, &tasks));
+        if (std::memcmp(key, ctx->lex_key, sizeof key) != 0) {
+            // counting sort of (tile, sweep) by i + j + k + 2 sweep
+            const int levels = a.nti + a.ntj + a.ntk - 2 + 2 * (ns - 1);
+            std::vector<size_t> at(levels + 1, 0);
+            std::vector<unsigned long long> list(count);
+            for (int pass = 0; pass < 2; ++pass) {
+                for (int s = 0; s < ns; ++s)
+                    for (int i = 0; i < a.nti; ++i)
+                        for (int j = 0; j < a.ntj; ++j)
+                            for (int k = 0; k < a.ntk; ++k) {
+                                const int l = i + j + k + 2 * s;
+                                if (pass == 0) ++at[l + 1];
+                                else
+                                    list[at[l]++] = (unsigned long long)i | (unsigned long long)j << 16 |
+                                                    (unsigned long long)k << 32 | (unsigned long long)s << 48;
+                            }
+                if (pass == 0)
+                    for (int l = 0; l < levels; ++l) at[l + 1] += at[l];
+            }
+            ctx->lex_key[0] = 0;  // no list while the copy can fail
+            IM3D_CUDA(ctx, cudaMemcpyAsync(tasks, list.data(), count * sizeof(unsigned long long),
+                                           cudaMemcpyHostToDevice, ctx->stream));
+            IM3D_TRY(sync(ctx));  // the list must outlive the copy
+            std::memcpy(ctx->lex_key, key, sizeof key);
+        }
+        a.tasks = tasks;
+        a.ntasks = (int)count;
+        IM3D_CUDA(ctx, cudaMemsetAsync(state, 0, ((size_t)nt + 1) * sizeof(int), ctx->stream));
+        const long long blocks = std::min<long long>((long long)count, (long long)occ * ctx->num_sms);
+        kern<<<(unsigned)blocks, kLexT * kLexT, smem, ctx->stream>>>(r, b, d, c, a);
+        IM3D_TRY(check_launch(ctx, "lex_tile"));
     }
     prof_end(ctx, pf);
+    return IM3D_OK;
+}
+
+// Control-block flags raised by a kernel's wait that gave up.
+int check_flags(im3d_ctx* ctx)
+{
+    if (ctx->ctrl_h->flag[0])
+        return fail(ctx, IM3D_ERR_CUDA, "a TMA load of the Heaviside pass did not complete in time");
+    if (ctx->ctrl_h->flag[1])
+        return fail(ctx, IM3D_ERR_CUDA, "a tile of the lexicographic sweep did not become ready in time");
     return IM3D_OK;
 }
 
@@ -862,8 +924,11 @@ int rb_march_launch(im3d_ctx* ctx, T* U, const T* B, const Dims& d, const GsCoef
     const long long npk = d.npk();
     // red walks the planes forward, black backward: each half-sweep starts on the planes
     // the previous one wrote last, which are still in L2
-    return launch_dependent(ctx, rb_march_kernel<T, NI, BC, BC == RB_NEU ? 1 : kRbMinB, IX>,
-                            grid_rb_flat<T>(d, kBlkVec, 1, NI), kBlkVec, U + (color ? npk : 0),
+    constexpr int MINB = BC == RB_NEU ? 1 : kRbMinB;
+    auto kern = rb_march_kernel<T, NI, BC, MINB, IX, false>;
+    if constexpr (sizeof(T) == 8)  // no division where the spacings allow it
+        if ((c.pow2 & 7) == 7) kern = rb_march_kernel<T, NI, BC, MINB, IX, true>;
+    return launch_dependent(ctx, kern, grid_rb_flat<T>(d, kBlkVec, 1, NI), kBlkVec, U + (color ? npk : 0),
                             (const T*)(U + (color ? 0 : npk)), B + (color ? npk : 0), d, c, color, color, first);
 }
 
@@ -1619,7 +1684,12 @@ int rsfe_apply(im3d_ctx* ctx, const T* myim_user, const T* init_user, int nx, in
                 if (p->ls_tol != 0)
                     IM3D_CUDA(ctx, cudaMemcpyAsync(prev, work, cnt * sizeof(T), cudaMemcpyDeviceToDevice,
                                                    ctx->stream));
-                if (lex) IM3D_TRY(lex_sweep<T>(ctx, phi, rhs, d, coef));
+                if (lex && p->ls_tol == 0) {
+                    IM3D_TRY(lex_sweeps<T>(ctx, phi, rhs, d, coef, p->ls_steps));
+                    s = p->ls_steps;
+                    break;
+                }
+                if (lex) IM3D_TRY(lex_sweeps<T>(ctx, phi, rhs, d, coef, 1));
                 else IM3D_TRY(rb_sweep<T>(ctx, upk, bpk, d, coef, 1, 1.0));
                 if (p->ls_tol != 0 && s >= p->ls_steps - 1) {
                     const dim3 grid(flat_grid(cnt));
@@ -1718,8 +1788,7 @@ int rsfe_apply(im3d_ctx* ctx, const T* myim_user, const T* init_user, int nx, in
             IM3D_TRY(check_launch(ctx, "div"));
         }
         if (cudaEventSynchronize(ctx->ev[3]) != cudaSuccess) IM3D_TRY(sync(ctx));
-        if (ctx->ctrl_h->flag[0])
-            return fail(ctx, IM3D_ERR_CUDA, "a TMA load of the Heaviside pass did not complete in time");
+        IM3D_TRY(check_flags(ctx));
         tollerance = std::sqrt(hhh * ctx->ctrl_h->sum[SUM_DPHI2]) /
                      std::sqrt(hhh * ctx->ctrl_h->sum[SUM_PHIOLD2]);
         if (lex) std::swap(phi, other);
@@ -1861,7 +1930,8 @@ int poisson_sweeps(im3d_ctx* ctx, T* res_user, const T* b_user, int nx, int ny, 
         IM3D_CUDA(ctx, cudaMemcpyAsync(r, res_user, n * sizeof(T), cudaMemcpyHostToDevice, ctx->stream));
     }
     if (order == IM3D_SWEEP_LEXICOGRAPHIC) {
-        for (int s = 0; s < sweeps; ++s) IM3D_TRY(lex_sweep<T>(ctx, r, b, d, c));
+        IM3D_TRY(zero_ctrl(ctx));
+        IM3D_TRY(lex_sweeps<T>(ctx, r, b, d, c, sweeps));
     } else if (sweeps > 0) {
         // DirGaussSeidel assigns the boundary value before sweeping (poisson_imp.hxx:366-391)
         if (!c.neu) {
@@ -1881,6 +1951,10 @@ int poisson_sweeps(im3d_ctx* ctx, T* res_user, const T* b_user, int nx, int ny, 
     }
     if (r != res_user)
         IM3D_CUDA(ctx, cudaMemcpyAsync(res_user, r, n * sizeof(T), cudaMemcpyDeviceToHost, ctx->stream));
+    if (order == IM3D_SWEEP_LEXICOGRAPHIC && sweeps > 0) {
+        IM3D_TRY(read_ctrl(ctx));
+        return check_flags(ctx);
+    }
     return sync(ctx);
 }
 
