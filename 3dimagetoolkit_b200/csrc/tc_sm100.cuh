@@ -51,6 +51,11 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t by
                  : "memory");
 }
 
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar)
+{
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t phase)
 {
     uint32_t done = 0;
@@ -65,13 +70,18 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t phase)
 }
 
 // Waits for the phase with the given parity to complete; gives up after `limit_ns`
-// nanoseconds (and after a bounded number of polls) and returns false then.
+// nanoseconds (and after a bounded number of polls) and returns false then. The clock is
+// read only after 256 polls: reading it takes longer than most waits.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t phase, uint64_t limit_ns = 2000000000ull)
 {
-    const uint64_t t0 = global_ns();
+    uint64_t t0 = 0;
     for (long long it = 0; it < (1ll << 26); ++it) {
         if (mbar_try_wait(bar, phase)) return true;
-        if ((it & 255) == 255 && global_ns() - t0 > limit_ns) return false;
+        if ((it & 255) == 255) {
+            const uint64_t t = global_ns();
+            if (t0 == 0) t0 = t;
+            if (t - t0 > limit_ns) return false;
+        }
     }
     return false;
 }
@@ -167,6 +177,14 @@ __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
         ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
+}
+
+// D[tmem] += A * B^T
+__device__ __forceinline__ void mma_bf16_acc(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc)
+{
+    asm volatile("tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, 1;"
+                 ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc)
+                 : "memory");
 }
 
 // arrives on `bar` once every MMA this thread issued before has completed

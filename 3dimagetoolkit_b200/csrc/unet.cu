@@ -16,6 +16,7 @@
 #include <cudaTypedefs.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <cstring>
@@ -116,61 +117,67 @@ int pow2_at_least(int x)
     return p;
 }
 
-// Tiling of a 3x3x3 convolution over a W x H x D volume for a kernel staging `chunks`
-// 8-channel chunks and NOUT output channels.
-bool plan_conv(int D, int H, int W, int nsamp, int chunks, int wbytes, int nout, ConvGeom* g, int* smem)
+int g_num_sms = 148;
+
+// Tiling of a 3x3x3 convolution: 4 tile rows where two staged planes, the filter and four
+// output planes fit (measured at 128^3, 16 -> 16 channels: 8, 4, 2, 1 rows take 79, 79, 123,
+// 183 us; 64 -> 32 at 64^3: 4, 2, 1 take 71, 87, 138), else fewer; output planes per unit zc
+// such that the busiest CTA streams the fewest planes.
+template <int CIN, int NOUT>
+bool plan_march(int D, int H, int W, int nsamp, int nblocks, MarchGeom* g, int* smem)
 {
     if (W % 16 != 0) return false;
     const int TW = W <= 128 ? W : 128;
     if (W % TW != 0) return false;
     const int P = TW + 2;
-    for (int pass = 0; pass < 2; ++pass) {
-        const int cap = pass == 0 ? 113 * 1024 : 220 * 1024;
-        const int tcap = pass == 0 ? 256 : 512;
-        for (int TH : {8, 4, 2, 1}) {
-            if (TH > H && TH > 1) continue;
-            const int reg = align_up(3 * (TH + 2) * P * 16, 1024);
-            const int mt = TW == 128 ? TH : ((TH - 1) * P + TW + 127) / 128;
-            const int bytes = align_up(wbytes, 1024) + chunks * reg + kGuardBytes + 64 + 1024;
-            if (bytes > cap || mt * nout > tcap) continue;
-            g->D = D;
-            g->H = H;
-            g->W = W;
-            g->nsamp = nsamp;
-            g->TH = TH;
-            g->TW = TW;
-            g->tiles_w = W / TW;
-            g->tiles_h = (H + TH - 1) / TH;
-            g->ntiles = (long long)nsamp * D * g->tiles_h * g->tiles_w;
-            g->mtiles = mt;
-            g->reg_bytes = reg;
-            g->tmem_cols = pow2_at_least(mt * nout);
-            *smem = bytes;
-            return true;
+    const int ctas = std::max(1, g_num_sms / nblocks);
+    for (int TH : {4, 2, 1}) {
+        if (TH > H && TH > 1) continue;
+        const int reg = align_up((TH + 2) * P * 16, 128);
+        const int mt = TW == 128 ? TH : ((TH - 1) * P + TW + 127) / 128;
+        const int slots = std::min(kMarchSlots, 512 / (mt * NOUT));
+        if (slots < 4 || mt > kMarchMaxMT) continue;
+        int stages = 0;
+        for (int st = 2; st <= 5; ++st)
+            if (march_smem_bytes<CIN, NOUT>(reg, st) <= 226 * 1024) stages = st;
+        if (stages < 2) continue;
+        const int tiles_w = W / TW, tiles_h = (H + TH - 1) / TH;
+        const long long cols = (long long)nsamp * tiles_w * tiles_h;
+        long long best = -1;
+        int zc = D;
+        for (int n = 1; n <= D; ++n) {
+            const int c = (D + n - 1) / n;
+            const long long planes = (cols * ((D + c - 1) / c) + ctas - 1) / ctas * (c + 2);
+            if (best < 0 || planes < best) {
+                best = planes;
+                zc = c;
+            }
         }
+        const int nzc = (D + zc - 1) / zc;
+        *g = MarchGeom{D, H, W, TH, TW, tiles_w, tiles_h, zc, nzc, cols * nzc, mt, reg, stages, slots,
+                       pow2_at_least(mt * NOUT * slots)};
+        // one CTA per SM: it may hold all 512 TMEM columns
+        *smem = std::max(march_smem_bytes<CIN, NOUT>(reg, stages), 116 * 1024);
+        return true;
     }
     return false;
 }
-
-int g_num_sms = 148;
 
 template <int CIN, int NOUT, int MODE>
 int conv_launch(cudaStream_t st, const View& x, int in_coff, const bf16_t* wpk, int nblocks, const float* bias,
                 void* out, int out_pitch, int out_coff, const bf16_t* mask, int mask_pitch, int mask_coff, int* errf,
                 std::string& err)
 {
-    ConvGeom g;
+    ConvArgs a;
     int smem = 0;
-    if (!plan_conv(x.D, x.H, x.W, x.nsamp, CIN / 8, conv_weight_bytes<CIN, NOUT>(), NOUT, &g, &smem)) {
+    if (!plan_march<CIN, NOUT>(x.D, x.H, x.W, x.nsamp, nblocks, &a.g, &smem)) {
         err = "no convolution tiling fits this volume (W must be a multiple of 16, and of 128 above 128)";
         return IM3D_ERR_UNSUPPORTED;
     }
     CUtensorMap map;
-    UN_TRY(make_map(x, g.TW, g.TH, 3, &map, err));
-    auto kern = conv3_tc_kernel<CIN, NOUT, MODE>;
+    UN_TRY(make_map(x, a.g.TW, a.g.TH, 1, &map, err));
+    auto kern = conv3_march_kernel<CIN, NOUT, MODE>;
     UN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    ConvArgs a;
-    a.g = g;
     a.wpk = wpk;
     a.bias = bias;
     a.out = out;
@@ -181,16 +188,9 @@ int conv_launch(cudaStream_t st, const View& x, int in_coff, const bf16_t* wpk, 
     a.mask_coff = mask_coff;
     a.in_coff = in_coff;
     a.err = errf;
-    // at most 2 CTAs per SM with <= 256 TMEM columns each, else 1 with up to 512: the
-    // shared-memory request enforces it, so that no CTA's TMEM allocation has to wait
-    const int per_sm = smem <= 113 * 1024 && g.tmem_cols <= 256 ? 2 : 1;
-    if (per_sm == 2 && smem < 77 * 1024) smem = 77 * 1024;
-    if (per_sm == 1 && smem < 116 * 1024) smem = 116 * 1024;
-    UN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    long long gx = (long long)g_num_sms * per_sm;
-    if (gx > g.ntiles) gx = g.ntiles;
-    kern<<<dim3((unsigned)gx, (unsigned)nblocks), 128, smem, st>>>(map, a);
-    return launch_status(err, "conv3_tc_kernel");
+    const long long gx = std::min<long long>(std::max(1, g_num_sms / nblocks), a.g.units);
+    kern<<<dim3((unsigned)gx, (unsigned)nblocks), kMarchThreads, smem, st>>>(map, a);
+    return launch_status(err, "conv3_march_kernel");
 }
 
 // Dispatch on the staged input channels and the output block width.
@@ -213,20 +213,8 @@ int conv_any(cudaStream_t st, int cin, int nout, const View& x, int in_coff, con
     return IM3D_ERR_UNSUPPORTED;
 }
 
-// Output-channel block width for a layer: 32 where the filter and the staged block
-// fit beside each other, else 16.
-int nout_for(int cin, int cout, int W)
-{
-    if (cout < 32) return 16;
-    ConvGeom g;
-    int smem;
-    if (cin == 64) {
-        const int wb = 27 * 8 * 32 * 16;
-        if (!plan_conv(8, 8, W, 1, 8, wb, 32, &g, &smem)) return 16;
-        return g.TH >= 2 ? 32 : 16;
-    }
-    return 32;
-}
+// Output-channel block width for a layer.
+int nout_for(int cout) { return cout < 32 ? 16 : 32; }
 
 template <int CIN>
 int wgrad_launch(cudaStream_t st, const View& x, int xcoff, const View& dz, int zcoff, int cout, float* dw,
@@ -733,8 +721,8 @@ int im3d_unet_create(im3d_ctx* ctx, uint64_t seed, im3d_unet** out)
     for (int q = 0; q < 16; ++q) host[n->out_w + q] = 0.f;  // the network starts by predicting no correction
     size_t wf = 0, wd = 0;
     for (int l = 0; l < NCONV; ++l) {
-        n->nout_f[l] = nout_for(kCin[l], kCout[l], 128);
-        n->nout_d[l] = nout_for(kCout[l], kCin[l], 128);
+        n->nout_f[l] = nout_for(kCout[l]);
+        n->nout_d[l] = nout_for(kCin[l]);
         n->wf_off.push_back(wf);
         wf += (size_t)27 * kCin[l] * kCout[l];
         n->wd_off.push_back(wd);
@@ -873,7 +861,7 @@ int im3d_conv3d_bf16(im3d_ctx* ctx, const uint16_t* x, int c_pitch, int c_off, i
     cudaDeviceProp prop;
     UN_CUDA(cudaGetDeviceProperties(&prop, im3d_ctx_device(ctx)));
     g_num_sms = prop.multiProcessorCount;
-    const int nout = cout == 16 ? 16 : 32;
+    const int nout = nout_for(cout);
     bf16_t* wpk = nullptr;
     int* errf = nullptr;
     UN_CUDA(cudaMalloc(&wpk, (size_t)27 * cin * cout * 2));

@@ -9,16 +9,16 @@
 //
 // The 3x3x3 convolutions (forward, and the data gradient as a forward convolution with
 // the flipped, transposed filter) run as implicit GEMMs on the tensor cores
-// (conv3_tc_kernel): a CTA stages, by TMA, the halo block of one output tile -- 3
-// planes x (TH + 2) rows x (TW + 2) columns of every 8-channel chunk, "chunk-planar"
-// (see tc_sm100.cuh) -- with the out-of-volume halo zero-filled by the TMA unit, which
-// is the convolution's zero padding. Each of the 27 taps is then the same block read
-// at a row offset, so the A operand of every tap is a descriptor into one staged block:
-// no im2col buffer, one HBM read of the block per tile. M = 128 output positions of the
-// padded tile, N = the output channels of the launch (16 or 32), K = 16 input channels
-// per instruction; the FP32 accumulators live in TMEM and are drained by 4 warps
-// (bias + ReLU or the ReLU mask of the data gradient, BF16 store). The weight gradient
-// (wgrad_tc_kernel) reads the same staged blocks with MN-major descriptors: M = the
+// (conv3_march_kernel): a CTA stages, by TMA, one input plane of a tile after another --
+// (TH + 2) rows x (TW + 2) columns of every 8-channel chunk, "chunk-planar" (see
+// tc_sm100.cuh) -- with the out-of-volume halo zero-filled by the TMA unit, which is the
+// convolution's zero padding. Each of the 9 taps of a plane is then the same block read
+// at a row offset, so the A operand of every tap is a descriptor into one staged plane:
+// no im2col buffer, one read of each plane per tile. M = 128 output positions of the
+// padded tile, N = the output channels of the launch (16 or 32) of the three output planes
+// that the input plane feeds, K = 16 input channels per instruction; the FP32 accumulators
+// live in TMEM and are drained by 4 warps (bias + ReLU or the ReLU mask of the data
+// gradient, BF16 store). The weight gradient (wgrad_tc_kernel) stages blocks of three planes with MN-major descriptors: M = the
 // output channels (64 rows, padded), N = the input channels, K = 16 voxel positions,
 // accumulated in TMEM over all tiles of a CTA and added to the FP32 gradient once.
 // Pooling, the 2x2x2 transposed convolutions, the 1x1 output layer, the loss and Adam
@@ -43,6 +43,13 @@ __device__ __forceinline__ bf16_t to_bf(float v)
     return __bfloat16_as_ushort(__float2bfloat16_rn(v));
 }
 
+// two floats as packed BF16 (round to nearest), the first in the low half
+__device__ __forceinline__ uint32_t pack_bf(float lo, float hi)
+{
+    const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+    return (uint32_t)__bfloat16_as_ushort(v.x) | ((uint32_t)__bfloat16_as_ushort(v.y) << 16);
+}
+
 // Geometry of one tiled 3x3x3 convolution launch (host-filled).
 struct ConvGeom {
     int D, H, W;     // volume of one sample
@@ -55,30 +62,9 @@ struct ConvGeom {
     int tmem_cols;   // TMEM columns allocated (power of two >= 32)
 };
 
-// Position of M-tile m's first row in the padded tile plane (pitch P = TW + 2): one
-// interior row per M-tile when TW == 128, else 128 consecutive positions starting at
-// the first interior one (rows of the tile and the 2 halo columns between them).
-__device__ __forceinline__ int mtile_start(const ConvGeom& g, int m)
-{
-    const int P = g.TW + 2;
-    return g.TW == 128 ? (m + 1) * P + 1 : P + 1 + 128 * m;
-}
-
-struct ConvArgs {
-    ConvGeom g;
-    const bf16_t* wpk;     // [N-block][27][CIN/8][NOUT][8] BF16 filter of this launch
-    const float* bias;     // output channels' bias (MODE 0, 2) or NULL
-    void* out;             // BF16 (MODE 0, 1) or FP32 (MODE 2) channels-last
-    int out_pitch, out_coff;
-    const bf16_t* mask;    // MODE 1: result multiplied by (mask > 0), or NULL
-    int mask_pitch, mask_coff;
-    int in_coff;           // first input channel (a multiple of 8)
-    int* err;              // raised when a wait gives up
-};
-
 enum { CONV_BIAS_RELU = 0, CONV_MASK = 1, CONV_BIAS_F32 = 2 };
 
-constexpr int kGuardBytes = 8192;  // after the staged block: the last M-tile's overreach
+constexpr int kGuardBytes = 8192;  // after the staged blocks: the last M-tile's overreach
 
 __host__ __device__ constexpr int align_up(int x, int a) { return (x + a - 1) / a * a; }
 
@@ -88,27 +74,92 @@ __host__ __device__ constexpr int conv_weight_bytes()
     return 27 * (CIN / 8) * NOUT * 16;
 }
 
-// dynamic shared memory of conv3_tc_kernel<CIN, NOUT>
+// Plan of one convolution launch by conv3_march_kernel (host-filled).
+struct MarchGeom {
+    int D, H, W;      // volume of one sample
+    int TH, TW;       // tile rows (along H) and columns (along W; TW divides W, TW <= 128)
+    int tiles_w, tiles_h;
+    int zc, nzc;      // output planes of a unit, units along z
+    long long units;  // nsamp * nzc * tiles_h * tiles_w
+    int mtiles;       // 128-position MMA tiles of a plane
+    int reg_bytes;    // one chunk region of a staged plane
+    int stages;       // staged planes
+    int slots;        // output planes in TMEM (>= 4)
+    int tmem_cols;    // power of two >= slots * mtiles * NOUT
+};
+
+struct ConvArgs {
+    MarchGeom g;
+    const bf16_t* wpk;     // [N-block][9][CIN/8][3 NOUT][8] BF16 filter of this launch (pack_filter_kernel)
+    const float* bias;     // output channels' bias (MODE 0, 2) or NULL
+    void* out;             // BF16 (MODE 0, 1) or FP32 (MODE 2) channels-last
+    int out_pitch, out_coff;
+    const bf16_t* mask;    // MODE 1: result multiplied by (mask > 0), or NULL
+    int mask_pitch, mask_coff;
+    int in_coff;           // first input channel (a multiple of 8)
+    int* err;              // raised when a wait gives up
+};
+
+constexpr int kMarchStages = 8, kMarchSlots = 8;  // most staged planes, most TMEM planes
+constexpr int kMarchMaxMT = 4;    // most M-tiles of a plane
+// warps of a block: one loader, MMA issuers, accumulator drains (a multiple of 4)
+constexpr int kMarchIssuers = 4, kMarchDrains = 8;
+constexpr int kMarchThreads = 32 * (1 + kMarchIssuers + kMarchDrains);
+
+// dynamic shared memory of conv3_march_kernel<CIN, NOUT>
 template <int CIN, int NOUT>
-__host__ __device__ inline int conv_smem_bytes(int reg_bytes)
+__host__ __device__ inline int march_smem_bytes(int reg_bytes, int stages)
 {
-    return align_up(conv_weight_bytes<CIN, NOUT>(), 1024) + (CIN / 8) * reg_bytes + kGuardBytes + 64 + 1024;
+    return align_up(conv_weight_bytes<CIN, NOUT>(), 1024) + stages * (CIN / 8) * reg_bytes + kGuardBytes +
+           8 * (2 * kMarchStages + 2 * kMarchSlots) + 16 + 1024;
 }
 
-template <int CIN, int NOUT, int MODE>
-__global__ void __launch_bounds__(128, 1) conv3_tc_kernel(const __grid_constant__ CUtensorMap xmap, ConvArgs a)
+// Position of M-tile m's first row in a padded tile plane (pitch P = TW + 2): one interior
+// row per M-tile when TW == 128, else 128 consecutive positions starting at the first
+// interior one (rows of the tile and the 2 halo columns between them).
+__device__ __forceinline__ int mtile_start(int TW, int m)
 {
-    constexpr int KC = CIN / 8;
+    const int P = TW + 2;
+    return TW == 128 ? (m + 1) * P + 1 : P + 1 + 128 * m;
+}
+
+// 3x3x3 convolution, marching along z. A CTA takes units (a TH x TW column of tiles, zc
+// output planes) in turn and streams the input planes z0-1 .. z0+zc of a unit once each
+// through a ring in shared memory (TMA, one 8-channel chunk per load). Input plane z feeds
+// three output planes: their accumulators sit side by side in TMEM (a ring of `slots` planes
+// per M-tile), so one MMA of N = 3 NOUT columns adds a (dy, dx) tap of all three, with the
+// filter packed as [tap][chunk][dz 2, 1, 0][NOUT]. An output plane still receives its 27 taps
+// in the order dz, dy, dx, channel.
+// Roles: one thread loads, 4 warps issue the MMAs (each its own M-tiles), 8 warps drain
+// finished planes (bias + ReLU, or the ReLU mask of a data gradient) while the next planes are
+// multiplied.
+// What bounds it: the TMA moves 16-byte rows (8 channels of a voxel) at 2-3 cycles each, about
+// 3800 cycles per plane of 4 x 128 voxels of 16 channels, against 36 + N / 4 cycles per MMA
+// (measured, M = 128, K = 16: its operands go through shared memory), about 2000. Three dz taps
+// per MMA cost little more than one, and each plane is loaded once instead of three times.
+// 16-byte cp.async from 4 warps instead of the TMA measured slower (119 against 79 us).
+// Measured against one block of three planes per output plane, load, MMAs (N = NOUT) and drain
+// in turn (us): 16 -> 16 channels at 128^3 139 -> 74, 32 -> 16 406 -> 124, 64 -> 32 at 64^3
+// 154 + 154 (N = 16) -> 67.
+template <int CIN, int NOUT, int MODE>
+__global__ void __launch_bounds__(kMarchThreads, 1) conv3_march_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ ConvArgs a)
+{
+    constexpr int KC = CIN / 8, N3 = 3 * NOUT;
     constexpr int WB = conv_weight_bytes<CIN, NOUT>();
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    const ConvGeom& g = a.g;
-    const int tid = threadIdx.x, warp = tid >> 5;
+    const MarchGeom& g = a.g;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int stage_bytes = KC * g.reg_bytes;
     unsigned char* wsm = smem;
     unsigned char* act = smem + align_up(WB, 1024);
-    uint64_t* bars = reinterpret_cast<uint64_t*>(act + KC * g.reg_bytes + kGuardBytes);
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(bars + 2);
-    __shared__ int s_fail;
+    uint64_t* full = reinterpret_cast<uint64_t*>(act + g.stages * stage_bytes + kGuardBytes);  // plane loaded
+    uint64_t* empty = full + kMarchStages;   // plane multiplied
+    uint64_t* ready = empty + kMarchStages;  // output plane complete in TMEM
+    uint64_t* drained = ready + kMarchSlots; // ... and read out
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(drained + kMarchSlots);
+    __shared__ volatile int s_fail;
+    __shared__ float s_bias[NOUT];
     const int nb = blockIdx.y;  // block of NOUT output channels
 
     {
@@ -116,13 +167,20 @@ __global__ void __launch_bounds__(128, 1) conv3_tc_kernel(const __grid_constant_
         uint4* dst = reinterpret_cast<uint4*>(wsm);
         for (int q = tid; q < WB / 16; q += blockDim.x) dst[q] = src[q];
     }
+    if (tid < NOUT) s_bias[tid] = a.bias ? a.bias[nb * NOUT + tid] : 0.f;
     if (tid == 0) {
-        tc::mbar_init(&bars[0], 1);
-        tc::mbar_init(&bars[1], 1);
+        for (int q = 0; q < kMarchStages; ++q) {
+            tc::mbar_init(full + q, 1);
+            tc::mbar_init(empty + q, kMarchIssuers);
+        }
+        for (int q = 0; q < kMarchSlots; ++q) {
+            tc::mbar_init(ready + q, kMarchIssuers);
+            tc::mbar_init(drained + q, kMarchDrains);
+        }
         tc::fence_mbar_init();
         s_fail = 0;
     }
-    if (warp == 0) {
+    if (warp == 1) {
         tc::tmem_alloc(tslot, (uint32_t)g.tmem_cols);
         tc::tmem_relinquish();
     }
@@ -131,120 +189,245 @@ __global__ void __launch_bounds__(128, 1) conv3_tc_kernel(const __grid_constant_
     __syncthreads();
     tc::tc_fence_after_sync();
     const uint32_t tmem = *tslot;
+    const int P = g.TW + 2, plane = (g.TH + 2) * P;
+    // a unit's first tile row and column, first output plane, planes and sample
+    auto unit = [&](long long u, int& w0, int& h0, int& z0, int& zn, int& s) {
+        w0 = (int)(u % g.tiles_w) * g.TW;
+        u /= g.tiles_w;
+        h0 = (int)(u % g.tiles_h) * g.TH;
+        u /= g.tiles_h;
+        z0 = (int)(u % g.nzc) * g.zc;
+        s = (int)(u / g.nzc);
+        zn = min(g.zc, g.D - z0);
+    };
 
-    const int P = g.TW + 2;
-    const int plane = (g.TH + 2) * P;
-    const uint32_t box_bytes = 16u * (uint32_t)plane * 3u;
-    const uint32_t idesc = tc::idesc_bf16(128, NOUT, false, false);
-    const uint32_t act_s = tc::smem_u32(act), w_s = tc::smem_u32(wsm);
-    uint32_t ph_ld = 0, ph_mma = 0;
-    bool loads_in_flight = false;
-
-    for (long long tile = blockIdx.x; tile < g.ntiles; tile += gridDim.x) {
-        long long r = tile;
-        const int tw = (int)(r % g.tiles_w);
-        r /= g.tiles_w;
-        const int th = (int)(r % g.tiles_h);
-        r /= g.tiles_h;
-        const int z = (int)(r % g.D);
-        const int s = (int)(r / g.D);
-        const int w0 = tw * g.TW, h0 = th * g.TH;
-        if (tid == 0) {
-            tc::mbar_arrive_expect_tx(&bars[0], KC * box_bytes);
-            for (int c = 0; c < KC; ++c)
-                tc::tma_load_5d(act + c * g.reg_bytes, &xmap, &bars[0], a.in_coff + 8 * c, w0 - 1, h0 - 1, z - 1, s);
-        }
-        loads_in_flight = true;
-        if (!tc::mbar_wait(&bars[0], ph_ld)) s_fail = 1;
-        ph_ld ^= 1;
-        __syncthreads();
-        if (s_fail) break;
-        loads_in_flight = false;
-        tc::tc_fence_after_sync();
-        if (tid == 0) {
-            for (int m = 0; m < g.mtiles; ++m) {
-                const int qs = mtile_start(g, m);
-                for (int t = 0; t < 27; ++t) {
-                    const int dz = t / 9, dy = (t / 3) % 3, dx = t % 3;
-                    const int q = dz * plane + qs + (dy - 1) * P + (dx - 1);
-#pragma unroll
-                    for (int ks = 0; ks < KC / 2; ++ks) {
-                        const uint64_t ad = tc::smem_desc(act_s + (uint32_t)(2 * ks * g.reg_bytes + q * 16),
-                                                          (uint32_t)g.reg_bytes, 128);
-                        const uint64_t bd = tc::smem_desc(w_s + (uint32_t)((t * KC + 2 * ks) * NOUT * 16),
-                                                          (uint32_t)(NOUT * 16), 128);
-                        tc::mma_bf16(tmem + (uint32_t)(m * NOUT), ad, bd, idesc, (t | ks) != 0);
+    if (warp == 0) {
+        if (lane == 0) {
+            const uint32_t bytes = (uint32_t)KC * 16u * (uint32_t)plane;
+            int st = 0, loaded = 0;  // next stage; planes loaded (counted up to the stages)
+            uint32_t ph = 1;         // parity of a free stage: the first pass finds them free
+            bool ok = true;
+            for (long long u = blockIdx.x; u < g.units && ok; u += gridDim.x) {
+                int w0, h0, z0, zn, s;
+                unit(u, w0, h0, z0, zn, s);
+                for (int z = z0 - 1; z <= z0 + zn; ++z) {
+                    if (!tc::mbar_wait(empty + st, ph)) s_fail = 1;
+                    if (s_fail) {
+                        ok = false;
+                        break;
+                    }
+                    tc::mbar_arrive_expect_tx(full + st, bytes);
+                    for (int c = 0; c < KC; ++c)
+                        tc::tma_load_5d(act + st * stage_bytes + c * g.reg_bytes, &xmap, full + st, a.in_coff + 8 * c,
+                                        w0 - 1, h0 - 1, z, s);
+                    loaded = min(loaded + 1, g.stages);
+                    if (++st == g.stages) {
+                        st = 0;
+                        ph ^= 1u;
                     }
                 }
             }
-            tc::mma_commit(&bars[1]);
+            // after a failure the loads still in flight land before the block exits (the
+            // stages before st hold this pass's planes, the others the last one's)
+            if (!ok)
+                for (int q = 0; q < loaded; ++q) tc::mbar_wait(full + q, q < st ? ph ^ 1u : ph, 1000000000ull);
         }
-        if (!tc::mbar_wait(&bars[1], ph_mma)) s_fail = 1;
-        ph_mma ^= 1;
-        __syncthreads();
-        if (s_fail) break;
-        tc::tc_fence_after_sync();
-        // epilogue: accumulator row tid of every M-tile
-        for (int m = 0; m < g.mtiles; ++m) {
-            const int q = mtile_start(g, m) + tid;
-            const int py = q / P, px = q - (q / P) * P;
-            float v[NOUT];
+    } else if (warp < 1 + kMarchIssuers) {
+        // lane 0 of each warp issues the MMAs of every kMarchIssuers-th M-tile
+        if (lane == 0) {
+            const uint32_t act_s = tc::smem_u32(act), w_s = tc::smem_u32(wsm);
+            int st = 0;                // stage of the plane
+            uint32_t ph = 0;           // ... and the parity of its load
+            int sa = 0, sf = 0;        // TMEM slots of output planes max(z - 1, z0) and of the next fresh plane
+            uint32_t phf = 1;          // parity of a drained fresh slot: the first pass finds them free
+            bool ok = true;
+            for (long long u = blockIdx.x; u < g.units && ok; u += gridDim.x) {
+                int w0, h0, z0, zn, s;
+                unit(u, w0, h0, z0, zn, s);
+                for (int z = z0 - 1; z <= z0 + zn; ++z) {
+                    // output planes z-1 .. z+1 of this unit, as offsets from z0
+                    const int o0 = max(z - 1 - z0, 0), o1 = min(z + 1 - z0, zn - 1);
+                    const bool fresh = o1 == z + 1 - z0;  // plane z + 1 receives its first tap
+                    if (fresh) {
+                        ok = tc::mbar_wait(drained + sf, phf);
+                        if (++sf == g.slots) {
+                            sf = 0;
+                            phf ^= 1u;
+                        }
+                    }
+                    if (!ok || !tc::mbar_wait(full + st, ph) || s_fail) {
+                        s_fail = 1;
+                        ok = false;
+                        break;
+                    }
+                    tc::tc_fence_after_sync();
+                    // the planes o0 .. o1 are consecutive TMEM slots, split where the ring wraps;
+                    // their filter rows start at dz = 1 - (o0 + z0 - z). Descriptors advance by
+                    // additions to their low words (addresses below 256 KB: no carry)
+                    const int cnt = o1 - o0 + 1;
+                    const int n0 = min(cnt, g.slots - sa), n1 = cnt - n0;
+                    const uint64_t bd0 = tc::smem_desc(w_s + (uint32_t)((o0 + z0 - (z - 1)) * NOUT * 16), (uint32_t)(N3 * 16), 128);
+                    const uint64_t ad0 = tc::smem_desc(act_s + (uint32_t)(st * stage_bytes), (uint32_t)g.reg_bytes, 128);
+                    const uint32_t id0 = tc::idesc_bf16(128, n0 * NOUT, false, false);
+                    const uint32_t id1 = tc::idesc_bf16(128, n1 * NOUT, false, false);
+                    const uint32_t ida = tc::idesc_bf16(128, NOUT, false, false);
+                    const uint32_t kstep = (uint32_t)((2 * g.reg_bytes) >> 4);
+                    for (int m = warp - 1; m < g.mtiles; m += kMarchIssuers) {
+                        const uint64_t am = ad0 + (uint32_t)(mtile_start(g.TW, m) - P - 1);
+                        const uint32_t dm = tmem + (uint32_t)(m * g.slots * NOUT);
+                        const uint32_t d0 = dm + (uint32_t)(sa * NOUT);
+                        if (fresh) {
+                            // the fresh plane's first tap does not accumulate
+                            for (int o = 0; o < cnt; ++o) {
+                                const int so = sa + o < g.slots ? sa + o : sa + o - g.slots;
+                                tc::mma_bf16(dm + (uint32_t)(so * NOUT), am, bd0 + (uint32_t)(o * NOUT), ida, o < cnt - 1);
+                            }
+                        }
 #pragma unroll
-            for (int c0 = 0; c0 < NOUT; c0 += 16) {
-                float part[16];
-                tc::tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(m * NOUT + c0), part);
+                        for (int t = 0; t < 9; ++t) {
 #pragma unroll
-                for (int u = 0; u < 16; ++u) v[c0 + u] = part[u];
-            }
-            const int y = h0 + py - 1, x = w0 + px - 1;
-            if (py < 1 || py > g.TH || px < 1 || px > g.TW || y >= g.H) continue;
-            const long long vox = (((long long)s * g.D + z) * g.H + y) * g.W + x;
-            const int c_first = nb * NOUT;
-            if (MODE == CONV_BIAS_F32) {
-                float* o = reinterpret_cast<float*>(a.out) + vox * a.out_pitch + a.out_coff + c_first;
-#pragma unroll
-                for (int n = 0; n < NOUT; ++n) o[n] = v[n] + (a.bias ? a.bias[c_first + n] : 0.f);
-                continue;
-            }
-            if (MODE == CONV_BIAS_RELU) {
-#pragma unroll
-                for (int n = 0; n < NOUT; ++n) v[n] = fmaxf(v[n] + a.bias[c_first + n], 0.f);
-            } else if (a.mask) {
-                const uint4* mp = reinterpret_cast<const uint4*>(a.mask + vox * a.mask_pitch + a.mask_coff + c_first);
-#pragma unroll
-                for (int n8 = 0; n8 < NOUT / 8; ++n8) {
-                    const uint4 mv = mp[n8];
-                    const uint32_t w4[4] = {mv.x, mv.y, mv.z, mv.w};
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        if (!(bf((bf16_t)(w4[u] & 0xffff)) > 0.f)) v[n8 * 8 + 2 * u] = 0.f;
-                        if (!(bf((bf16_t)(w4[u] >> 16)) > 0.f)) v[n8 * 8 + 2 * u + 1] = 0.f;
+                            for (int ks = 0; ks < KC / 2; ++ks) {
+                                if (t == 0 && ks == 0 && fresh) continue;
+                                const uint64_t ad = am + (uint32_t)((t / 3) * P + t % 3) + ks * kstep;
+                                const uint64_t bd = bd0 + (uint32_t)((t * KC + 2 * ks) * N3);
+                                tc::mma_bf16_acc(d0, ad, bd, id0);
+                                if (n1) tc::mma_bf16_acc(dm, ad, bd + (uint32_t)(n0 * NOUT), id1);
+                            }
+                        }
+                    }
+                    tc::mma_commit(empty + st);
+                    if (++st == g.stages) {
+                        st = 0;
+                        ph ^= 1u;
+                    }
+                    if (z > z0) {  // output plane z - 1 is complete
+                        tc::mma_commit(ready + sa);
+                        if (++sa == g.slots) sa = 0;
                     }
                 }
             }
-            uint4* o = reinterpret_cast<uint4*>(reinterpret_cast<bf16_t*>(a.out) + vox * a.out_pitch + a.out_coff + c_first);
+        }
+    } else {
+        const int lanes = (warp & 3) * 32;  // this warp's TMEM lanes
+        // this warp's M-tiles mfirst, mfirst + MS, ..., and where its lane's position of each
+        // lies: row py and column px of the tile, py < 0 for a halo position
+        constexpr int MS = kMarchDrains / 4, MT = kMarchMaxMT / MS;
+        const int mfirst = (warp - 1 - kMarchIssuers) >> 2;
+        int off[MT], py[MT];
 #pragma unroll
-            for (int n8 = 0; n8 < NOUT / 8; ++n8) {
-                uint4 pk;
-                pk.x = (uint32_t)to_bf(v[n8 * 8 + 0]) | ((uint32_t)to_bf(v[n8 * 8 + 1]) << 16);
-                pk.y = (uint32_t)to_bf(v[n8 * 8 + 2]) | ((uint32_t)to_bf(v[n8 * 8 + 3]) << 16);
-                pk.z = (uint32_t)to_bf(v[n8 * 8 + 4]) | ((uint32_t)to_bf(v[n8 * 8 + 5]) << 16);
-                pk.w = (uint32_t)to_bf(v[n8 * 8 + 6]) | ((uint32_t)to_bf(v[n8 * 8 + 7]) << 16);
-                o[n8] = pk;
+        for (int e = 0; e < MT; ++e) {
+            const int pq = mtile_start(g.TW, mfirst + e * MS) + lanes + lane;
+            const int r = pq / P, px = pq - r * P;
+            py[e] = mfirst + e * MS < g.mtiles && r >= 1 && r <= g.TH && px >= 1 && px <= g.TW ? r - 1 : -1;
+            off[e] = (r - 1) * g.W + px - 1;
+        }
+        const int c_first = nb * NOUT;
+        const uint4* mask = MODE == CONV_MASK ? reinterpret_cast<const uint4*>(a.mask) : nullptr;
+        int slot = 0;
+        uint32_t ph = 0;
+        bool ok = true;
+        for (long long u = blockIdx.x; u < g.units && ok; u += gridDim.x) {
+            int w0, h0, z0, zn, s;
+            unit(u, w0, h0, z0, zn, s);
+            for (int z = z0; z < z0 + zn; ++z) {
+                const long long vbase = (((long long)s * g.D + z) * g.H + h0) * g.W + w0;
+                // the ReLU mask of an M-tile is read one M-tile ahead (the first before the wait)
+                uint4 mk[NOUT / 8], mkn[NOUT / 8];
+                auto live = [&](int e) { return py[e] >= 0 && h0 + py[e] < g.H; };
+                auto ld_mask = [&](int e) {
+#pragma unroll
+                    for (int n8 = 0; n8 < NOUT / 8; ++n8) {
+                        mkn[n8] = make_uint4(0, 0, 0, 0);
+                        if (mask && live(e))
+                            mkn[n8] = *(reinterpret_cast<const uint4*>(a.mask + (vbase + off[e]) * a.mask_pitch +
+                                                                       a.mask_coff + c_first) + n8);
+                    }
+                };
+                if (MODE == CONV_MASK) ld_mask(0);
+                if (!tc::mbar_wait(ready + slot, ph) || s_fail) {
+                    s_fail = 1;
+                    ok = false;
+                    break;
+                }
+                tc::tc_fence_after_sync();
+                __syncwarp();
+#pragma unroll
+                for (int e = 0; e < MT; ++e) {
+                    const int m = mfirst + e * MS;
+                    if (m >= g.mtiles) break;
+                    if (MODE == CONV_MASK) {
+#pragma unroll
+                        for (int n8 = 0; n8 < NOUT / 8; ++n8) mk[n8] = mkn[n8];
+                        if (e + 1 < MT) ld_mask(e + 1);
+                    }
+                    float v[NOUT];
+                    __syncwarp();
+#pragma unroll
+                    for (int c0 = 0; c0 < NOUT; c0 += 16) {
+                        float part[16];
+                        tc::tmem_ld16(tmem + ((uint32_t)lanes << 16) + (uint32_t)((m * g.slots + slot) * NOUT + c0), part);
+#pragma unroll
+                        for (int n = 0; n < 16; ++n) v[c0 + n] = part[n];
+                    }
+                    if (!live(e)) continue;
+                    const long long vox = vbase + off[e];
+                    if (MODE != CONV_MASK) {
+#pragma unroll
+                        for (int n = 0; n < NOUT; ++n) v[n] += s_bias[n];
+                    }
+                    if (MODE == CONV_BIAS_F32) {
+                        float* o = reinterpret_cast<float*>(a.out) + vox * a.out_pitch + a.out_coff + c_first;
+                        if ((reinterpret_cast<uintptr_t>(o) & 15) == 0) {
+#pragma unroll
+                            for (int n = 0; n < NOUT; n += 4)
+                                reinterpret_cast<float4*>(o)[n / 4] = make_float4(v[n], v[n + 1], v[n + 2], v[n + 3]);
+                        } else {
+#pragma unroll
+                            for (int n = 0; n < NOUT; ++n) o[n] = v[n];
+                        }
+                        continue;
+                    }
+                    if (MODE == CONV_BIAS_RELU) {
+#pragma unroll
+                        for (int n = 0; n < NOUT; ++n) v[n] = fmaxf(v[n], 0.f);
+                    } else if (mask) {
+#pragma unroll
+                        for (int n8 = 0; n8 < NOUT / 8; ++n8) {
+                            const uint32_t w4[4] = {mk[n8].x, mk[n8].y, mk[n8].z, mk[n8].w};
+#pragma unroll
+                            for (int n = 0; n < 4; ++n) {
+                                if (!(bf((bf16_t)(w4[n] & 0xffff)) > 0.f)) v[n8 * 8 + 2 * n] = 0.f;
+                                if (!(bf((bf16_t)(w4[n] >> 16)) > 0.f)) v[n8 * 8 + 2 * n + 1] = 0.f;
+                            }
+                        }
+                    }
+                    uint4* o = reinterpret_cast<uint4*>(reinterpret_cast<bf16_t*>(a.out) + vox * a.out_pitch + a.out_coff + c_first);
+#pragma unroll
+                    for (int n8 = 0; n8 < NOUT / 8; ++n8) {
+                        uint4 pk;
+                        pk.x = pack_bf(v[n8 * 8 + 0], v[n8 * 8 + 1]);
+                        pk.y = pack_bf(v[n8 * 8 + 2], v[n8 * 8 + 3]);
+                        pk.z = pack_bf(v[n8 * 8 + 4], v[n8 * 8 + 5]);
+                        pk.w = pack_bf(v[n8 * 8 + 6], v[n8 * 8 + 7]);
+                        o[n8] = pk;
+                    }
+                }
+                // this warp's part of the slot may be multiplied into again
+                __syncwarp();
+                tc::tc_fence_before_sync();
+                if (lane == 0) tc::mbar_arrive(drained + slot);
+                if (++slot == g.slots) {
+                    slot = 0;
+                    ph ^= 1u;
+                }
             }
         }
-        tc::tc_fence_before_sync();
-        __syncthreads();
     }
-    if (s_fail) {
-        if (tid == 0) atomicExch(a.err, 1);
-        // let the copies that may still be in flight land before the block exits
-        if (loads_in_flight) tc::mbar_wait(&bars[0], ph_ld ^ 1, 1000000000ull);
-        __syncthreads();
-    }
+    __syncwarp();
     tc::tc_fence_before_sync();
     __syncthreads();
-    if (warp == 0) tc::tmem_dealloc(tmem, (uint32_t)g.tmem_cols);
+    if (s_fail && tid == 0) atomicExch(a.err, 1);
+    if (warp == 1) tc::tmem_dealloc(tmem, (uint32_t)g.tmem_cols);
 }
 
 // ---------------------------------------------------------------- weight gradient
@@ -707,11 +890,12 @@ __global__ void adam_kernel(float* __restrict__ p, const float* __restrict__ g, 
     }
 }
 
-// FP32 filter W[co][ci][27] -> BF16 operand blocks of conv3_tc_kernel.
-//   forward (transpose = 0): block nb holds output channels nb*NOUT.. : [27][CIN/8][NOUT][8]
-//     with element (t, kc, n, e) = W[nb*NOUT + n][kc*8 + e][t]  (CIN = layer Cin)
+// FP32 filter W[co][ci][27] -> BF16 operand blocks of conv3_march_kernel: block nb holds
+// outputs nb*NOUT .. of the launch, [9 taps (dy, dx)][CIN/8][dz 2, 1, 0][NOUT][8]:
+//   forward (transpose = 0): element (t, kc, dz, n, e) = W[nb*NOUT + n][kc*8 + e][9 dz + t]
+//     (CIN = layer Cin)
 //   data gradient (transpose = 1): the flipped, transposed filter, CIN = layer Cout,
-//     outputs = layer Cin: element (t, kc, n, e) = W[kc*8 + e][nb*NOUT + n][26 - t]
+//     outputs = layer Cin: W[kc*8 + e][nb*NOUT + n][26 - (9 dz + t)]
 __global__ void pack_filter_kernel(const float* __restrict__ W, int cout, int cin, int nout, int transpose,
                                    bf16_t* __restrict__ out)
 {
@@ -724,10 +908,12 @@ __global__ void pack_filter_kernel(const float* __restrict__ W, int cout, int ci
         long long r = e / 8;
         const int n = (int)(r % nout);
         r /= nout;
+        const int dz = 2 - (int)(r % 3);
+        r /= 3;
         const int kc = (int)(r % (kcin / 8));
         r /= kcin / 8;
-        const int t = (int)(r % 27);
-        const int nb = (int)(r / 27);
+        const int t = 9 * dz + (int)(r % 9);
+        const int nb = (int)(r / 9);
         const int k = kc * 8 + el, nn = nb * nout + n;
         const float w = transpose ? W[((size_t)k * cin + nn) * 27 + (26 - t)] : W[((size_t)nn * cin + k) * 27 + t];
         out[e] = to_bf(w);
