@@ -85,8 +85,9 @@ struct View {
     int D, H, W, nsamp;
 };
 
-// Tensor map of a view for boxes of 8 channels x (TW + 2) x (TH + 2) x depth.
-int make_map(const View& v, int TW, int TH, int depth, CUtensorMap* map, std::string& err)
+// Tensor map of a view for boxes of `chans` channels x bw x bh of one plane. Boxes of 8
+// channels are not swizzled, those of 16 and 32 with the swizzle of their 32 or 64 bytes.
+int make_map(const View& v, int chans, int bw, int bh, CUtensorMap* map, std::string& err)
 {
     auto fn = encode_fn();
     if (!fn) {
@@ -98,10 +99,12 @@ int make_map(const View& v, int TW, int TH, int depth, CUtensorMap* map, std::st
                           (cuuint64_t)v.nsamp};
     cuuint64_t strides[4] = {v.pitch * es, v.pitch * es * v.W, v.pitch * es * v.W * v.H,
                              v.pitch * es * v.W * v.H * v.D};
-    cuuint32_t box[5] = {8, (cuuint32_t)(TW + 2), (cuuint32_t)(TH + 2), (cuuint32_t)depth, 1};
+    cuuint32_t box[5] = {(cuuint32_t)chans, (cuuint32_t)bw, (cuuint32_t)bh, 1, 1};
     cuuint32_t estr[5] = {1, 1, 1, 1, 1};
     const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<bf16_t*>(v.p), dims, strides, box, estr,
-                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                          CU_TENSOR_MAP_INTERLEAVE_NONE,
+                          chans == 8 ? CU_TENSOR_MAP_SWIZZLE_NONE
+                                     : (chans == 16 ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_64B),
                           CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) {
         err = "cuTensorMapEncodeTiled failed (" + std::to_string((int)r) + ")";
@@ -118,6 +121,23 @@ int pow2_at_least(int x)
 }
 
 int g_num_sms = 148;
+
+// Output planes per unit such that the busiest of `ctas` blocks streams the fewest input
+// planes (two more than its output planes per unit), for `cols` columns of D planes.
+int plan_zc(int D, long long cols, int ctas)
+{
+    long long best = -1;
+    int zc = D;
+    for (int n = 1; n <= D; ++n) {
+        const int c = (D + n - 1) / n;
+        const long long planes = (cols * ((D + c - 1) / c) + ctas - 1) / ctas * (c + 2);
+        if (best < 0 || planes < best) {
+            best = planes;
+            zc = c;
+        }
+    }
+    return zc;
+}
 
 // Tiling of a 3x3x3 convolution: 4 tile rows where two staged planes, the filter and four
 // output planes fit (measured at 128^3, 16 -> 16 channels: 8, 4, 2, 1 rows take 79, 79, 123,
@@ -143,16 +163,7 @@ bool plan_march(int D, int H, int W, int nsamp, int nblocks, MarchGeom* g, int* 
         if (stages < 2) continue;
         const int tiles_w = W / TW, tiles_h = (H + TH - 1) / TH;
         const long long cols = (long long)nsamp * tiles_w * tiles_h;
-        long long best = -1;
-        int zc = D;
-        for (int n = 1; n <= D; ++n) {
-            const int c = (D + n - 1) / n;
-            const long long planes = (cols * ((D + c - 1) / c) + ctas - 1) / ctas * (c + 2);
-            if (best < 0 || planes < best) {
-                best = planes;
-                zc = c;
-            }
-        }
+        const int zc = plan_zc(D, cols, ctas);
         const int nzc = (D + zc - 1) / zc;
         *g = MarchGeom{D, H, W, TH, TW, tiles_w, tiles_h, zc, nzc, cols * nzc, mt, reg, stages, slots,
                        pow2_at_least(mt * NOUT * slots)};
@@ -175,7 +186,7 @@ int conv_launch(cudaStream_t st, const View& x, int in_coff, const bf16_t* wpk, 
         return IM3D_ERR_UNSUPPORTED;
     }
     CUtensorMap map;
-    UN_TRY(make_map(x, a.g.TW, a.g.TH, 1, &map, err));
+    UN_TRY(make_map(x, 8, a.g.TW + 2, a.g.TH + 2, &map, err));
     auto kern = conv3_march_kernel<CIN, NOUT, MODE>;
     UN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     a.wpk = wpk;
@@ -216,79 +227,62 @@ int conv_any(cudaStream_t st, int cin, int nout, const View& x, int in_coff, con
 // Output-channel block width for a layer.
 int nout_for(int cout) { return cout < 32 ? 16 : 32; }
 
-template <int CIN>
-int wgrad_launch(cudaStream_t st, const View& x, int xcoff, const View& dz, int zcoff, int cout, float* dw,
+template <int CO, int CI>
+int wgrad_launch(cudaStream_t st, const View& x, int xcoff, int cin, const View& dz, int zcoff, int cout, float* dw,
                  int* errf, std::string& err)
 {
-    if (x.W % 16 != 0) {
-        err = "weight gradient: W must be a multiple of 16";
-        return IM3D_ERR_UNSUPPORTED;
-    }
     const int TW = x.W <= 128 ? x.W : 128;
-    const int P = TW + 2;
-    int TH = 0, reg_z = 0, reg_x = 0, smem = 0;
-    for (int th : {8, 4, 2, 1}) {
-        if (th > x.H && th > 1) continue;
-        const int rz = align_up((th + 2) * P * 16, 1024);
-        const int rx = align_up(3 * (th + 2) * P * 16, 1024);
-        // the 64-row A operand reads 8 chunk regions from the dZ block: keep them inside
-        const int over = (8 - cout / 8) * rz - (CIN / 8) * rx;
-        const int bytes = wgrad_smem_bytes<CIN>(cout, rz, rx) + (over > 0 ? over : 0);
-        if (bytes <= 220 * 1024) {
-            TH = th;
-            reg_z = rz;
-            reg_x = rx;
-            smem = bytes;
-            break;
-        }
-    }
-    if (!TH) {
-        err = "weight gradient: no tiling fits shared memory";
+    if (x.W % 16 != 0 || x.W % TW != 0) {
+        err = "weight gradient: W must be a multiple of 16, and of 128 above 128";
         return IM3D_ERR_UNSUPPORTED;
     }
-    ConvGeom g;
-    g.D = x.D;
-    g.H = x.H;
-    g.W = x.W;
-    g.nsamp = x.nsamp;
-    g.TH = TH;
-    g.TW = TW;
-    g.tiles_w = x.W / TW;
-    g.tiles_h = (x.H + TH - 1) / TH;
-    g.ntiles = (long long)x.nsamp * x.D * g.tiles_h * g.tiles_w;
-    g.mtiles = 0;
-    g.reg_bytes = reg_x;
-    g.tmem_cols = 512;
-    CUtensorMap xm, zm;
-    UN_TRY(make_map(x, TW, TH, 3, &xm, err));
-    UN_TRY(make_map(dz, TW, TH, 1, &zm, err));
-    WgradArgs a;
-    a.g = g;
-    a.zcoff = zcoff;
-    a.xcoff = xcoff;
-    a.tap0 = 0;
-    a.ntaps = 512 / CIN < 27 ? 512 / CIN : 27;
-    a.cout = cout;
-    a.dw = dw;
-    a.err = errf;
-    const int groups = (27 + a.ntaps - 1) / a.ntaps;
-    long long splits = (g_num_sms + groups - 1) / groups;
-    if (splits > g.ntiles) splits = g.ntiles;
-    auto kern = wgrad_tc_kernel<CIN>;
-    if (smem < 116 * 1024) smem = 116 * 1024;  // one CTA per SM: it allocates all 512 TMEM columns
-    UN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    kern<<<dim3((unsigned)groups, (unsigned)splits), 128, smem, st>>>(xm, zm, a, reg_z, reg_x);
-    return launch_status(err, "wgrad_tc_kernel");
+    const int nblocks = (cout / CO) * (cin / CI);
+    const int ctas = std::max(1, g_num_sms / nblocks);
+    for (int TH : {4, 2, 1}) {
+        if (TH > x.H && TH > 1) continue;
+        WgradArgs a;
+        a.xbytes = align_up((TH + 2) * (TW + 2) * 2 * CI, 1024);
+        a.zbytes = align_up(TH * TW * 2 * CO, 1024);
+        const int smem = 1024 + kWgXStages * a.xbytes + kWgZStages * a.zbytes + 16 * (kWgXStages + kWgZStages);
+        if (smem > 226 * 1024) continue;
+        a.D = x.D;
+        a.H = x.H;
+        a.W = x.W;
+        a.TH = TH;
+        a.TW = TW;
+        a.tiles_w = x.W / TW;
+        a.tiles_h = (x.H + TH - 1) / TH;
+        const long long cols = (long long)x.nsamp * a.tiles_w * a.tiles_h;
+        a.zc = plan_zc(x.D, cols, ctas);
+        a.nzc = (x.D + a.zc - 1) / a.zc;
+        a.units = cols * a.nzc;
+        a.zcoff = zcoff;
+        a.xcoff = xcoff;
+        a.cin = cin;
+        a.ciblocks = cin / CI;
+        a.dw = dw;
+        a.err = errf;
+        CUtensorMap xm, zm;
+        UN_TRY(make_map(x, CI, TW + 2, TH + 2, &xm, err));
+        UN_TRY(make_map(dz, CO, TW, TH, &zm, err));
+        auto kern = wgrad_mma_kernel<CO, CI>;
+        UN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        const long long gx = std::min<long long>(ctas, a.units);
+        kern<<<dim3((unsigned)gx, (unsigned)nblocks), kWgThreads, smem, st>>>(xm, zm, a);
+        return launch_status(err, "wgrad_mma_kernel");
+    }
+    err = "weight gradient: no tiling fits shared memory";
+    return IM3D_ERR_UNSUPPORTED;
 }
 
+// Blocks of 16 or 32 output and input channels.
 int wgrad_any(cudaStream_t st, int cin, const View& x, int xcoff, const View& dz, int zcoff, int cout, float* dw,
               int* errf, std::string& err)
 {
-    if (cin == 16) return wgrad_launch<16>(st, x, xcoff, dz, zcoff, cout, dw, errf, err);
-    if (cin == 32) return wgrad_launch<32>(st, x, xcoff, dz, zcoff, cout, dw, errf, err);
-    if (cin == 64) return wgrad_launch<64>(st, x, xcoff, dz, zcoff, cout, dw, errf, err);
-    err = "unsupported weight-gradient shape";
-    return IM3D_ERR_UNSUPPORTED;
+    if (cin == 16 && cout == 16) return wgrad_launch<16, 16>(st, x, xcoff, cin, dz, zcoff, cout, dw, errf, err);
+    if (cin == 16) return wgrad_launch<32, 16>(st, x, xcoff, cin, dz, zcoff, cout, dw, errf, err);
+    if (cout == 16) return wgrad_launch<16, 32>(st, x, xcoff, cin, dz, zcoff, cout, dw, errf, err);
+    return wgrad_launch<32, 32>(st, x, xcoff, cin, dz, zcoff, cout, dw, errf, err);
 }
 
 int flat_blocks(long long n, int per = 256)

@@ -18,9 +18,8 @@
 // padded tile, N = the output channels of the launch (16 or 32) of the three output planes
 // that the input plane feeds, K = 16 input channels per instruction; the FP32 accumulators
 // live in TMEM and are drained by 4 warps (bias + ReLU or the ReLU mask of the data
-// gradient, BF16 store). The weight gradient (wgrad_tc_kernel) stages blocks of three planes with MN-major descriptors: M = the
-// output channels (64 rows, padded), N = the input channels, K = 16 voxel positions,
-// accumulated in TMEM over all tiles of a CTA and added to the FP32 gradient once.
+// gradient, BF16 store). The weight gradient (wgrad_mma_kernel) marches the same way with its
+// accumulators in registers (mma.sync: its M, the output channels, is 16 or 32).
 // Pooling, the 2x2x2 transposed convolutions, the 1x1 output layer, the loss and Adam
 // are small SIMT kernels.
 #pragma once
@@ -49,18 +48,6 @@ __device__ __forceinline__ uint32_t pack_bf(float lo, float hi)
     const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
     return (uint32_t)__bfloat16_as_ushort(v.x) | ((uint32_t)__bfloat16_as_ushort(v.y) << 16);
 }
-
-// Geometry of one tiled 3x3x3 convolution launch (host-filled).
-struct ConvGeom {
-    int D, H, W;     // volume of one sample
-    int nsamp;       // samples
-    int TH, TW;      // tile rows (along H) and columns (along W; TW divides W, TW <= 128)
-    int tiles_w, tiles_h;
-    long long ntiles;  // nsamp * D * tiles_h * tiles_w
-    int mtiles;      // 128-position MMA tiles per CTA tile
-    int reg_bytes;   // one chunk region of the staged block (multiple of 1024)
-    int tmem_cols;   // TMEM columns allocated (power of two >= 32)
-};
 
 enum { CONV_BIAS_RELU = 0, CONV_MASK = 1, CONV_BIAS_F32 = 2 };
 
@@ -431,136 +418,230 @@ __global__ void __launch_bounds__(kMarchThreads, 1) conv3_march_kernel(const __g
 }
 
 // ---------------------------------------------------------------- weight gradient
+constexpr int kWgWarps = 9;                      // multiplying warps: one per (dz, dy)
+constexpr int kWgThreads = 32 * (kWgWarps + 1);  // and one that loads
+constexpr int kWgXStages = 5, kWgZStages = 3;      // planes of X and of dZ in shared memory
+
 struct WgradArgs {
-    ConvGeom g;      // the forward launch's tiling (TW multiple of 16)
-    int zcoff;       // first channel of dZ in its tensor
-    int xcoff;       // first input channel in X's tensor
-    int tap0, ntaps; // taps of this launch's blockIdx.x group: tap0 + blockIdx.x * ntaps ...
-    int cout;        // output channels (rows of dZ used)
-    float* dw;       // FP32 gradient [cout][CIN][27] (the parameter layout), accumulated with atomics
+    int D, H, W;      // volume of one sample
+    int TH, TW;       // tile rows and columns (TW divides W, TW <= 128, a multiple of 16)
+    int tiles_w, tiles_h;
+    int zc, nzc;      // planes of a unit, units along z
+    long long units;  // nsamp * nzc * tiles_h * tiles_w
+    int xbytes, zbytes;  // a staged plane of X (halo included) and of dZ, multiples of 1024
+    int zcoff, xcoff;    // first channel of dZ and of X in their tensors
+    int cin;             // input channels of the layer
+    int ciblocks;        // blocks of CI input channels (blockIdx.y = output block * ciblocks + input block)
+    float* dw;           // FP32 gradient [cout][cin][27] (the parameter layout), accumulated with atomics
     int* err;
 };
 
-template <int CIN>
-__host__ __device__ inline int wgrad_smem_bytes(int cout, int reg_z, int reg_x)
+__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t addr, uint32_t (&r)[4])
 {
-    return (cout / 8) * reg_z + (CIN / 8) * reg_x + kGuardBytes + 64 + 1024;
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr));
 }
 
-// grid.x: tap groups of a.ntaps taps; grid.y: splits of the tile list.
-template <int CIN>
-__global__ void __launch_bounds__(128, 1) wgrad_tc_kernel(const __grid_constant__ CUtensorMap xmap,
-                                                         const __grid_constant__ CUtensorMap zmap, WgradArgs a,
-                                                         int reg_z, int reg_x)
+// D (16 x 8, FP32) += A (16 x 16) * B (16 x 8), BF16
+__device__ __forceinline__ void mma_16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1)
 {
-    constexpr int KC = CIN / 8;
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+                 "{%0, %1, %2, %3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+// Byte offset of 16-byte chunk c of row r in a plane of rows of ROW bytes that the TMA wrote
+// with its ROW-byte swizzle (32: chunk bit 0 ^ address bit 7; 64: chunk bits ^ bits 7, 8).
+template <int ROW>
+__device__ __forceinline__ uint32_t swizzled(int r, int c)
+{
+    return (uint32_t)(r * ROW + ((ROW == 32 ? c ^ ((r >> 2) & 1) : c ^ ((r >> 1) & 3)) << 4));
+}
+
+// dW[co][ci][tap] = sum over voxels of dZ[v][co] X[v + tap][ci], for CO output and CI input
+// channels (blockIdx.y). A CTA marches along z through units of TH x TW columns: X planes and
+// dZ planes stream through rings in shared memory (TMA), each X plane serving three output
+// planes. Warp (dz, dy) keeps the accumulators of its three dx taps in registers over all its
+// units and adds them to the gradient once.
+// The products run on mma.sync (M = 16 output channels, N = 8 input channels, K = 16 voxels):
+// both operands are read transposed from channels-last rows by ldmatrix, and M = 16 fits 16
+// and 32 channels exactly, where tcgen05's smallest M (64) multiplies three quarters or half
+// of it for nothing and needs one MMA per tap of 16 or 32 columns.
+// What bounds it: the TMA's rows of 32 or 64 bytes (twice the multiplying warps measured the
+// same). us against the tcgen05 form (M = 64, N = CI, load and multiply in turn): 16 x 16 at
+// 128^3 929 -> 131, 16 x 32 at 128^3 about 950 -> 227, 32 x 32 at 64^3 about 420 -> 79.
+template <int CO, int CI>
+__global__ void __launch_bounds__(kWgThreads, 1) wgrad_mma_kernel(const __grid_constant__ CUtensorMap xmap,
+                                                                  const __grid_constant__ CUtensorMap zmap,
+                                                                  const __grid_constant__ WgradArgs a)
+{
+    constexpr int RX = 2 * CI, RZ = 2 * CO;  // bytes of a row (one voxel)
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    const ConvGeom& g = a.g;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int zc = a.cout / 8;
-    unsigned char* zblk = smem;                    // dZ: zc regions of one padded plane
-    unsigned char* xblk = smem + zc * reg_z;       // X: KC regions of 3 padded planes
-    uint64_t* bars = reinterpret_cast<uint64_t*>(xblk + KC * reg_x + kGuardBytes);
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(bars + 2);
-    __shared__ int s_fail;
-    const int t_first = a.tap0 + blockIdx.x * a.ntaps;
-    const int nt = min(a.ntaps, 27 - t_first);
+    unsigned char* xs = smem;
+    unsigned char* zs = xs + kWgXStages * a.xbytes;
+    uint64_t* fullx = reinterpret_cast<uint64_t*>(zs + kWgZStages * a.zbytes);
+    uint64_t* emptyx = fullx + kWgXStages;
+    uint64_t* fullz = emptyx + kWgXStages;
+    uint64_t* emptyz = fullz + kWgZStages;
+    __shared__ volatile int s_fail;
     if (tid == 0) {
-        tc::mbar_init(&bars[0], 1);
-        tc::mbar_init(&bars[1], 1);
+        for (int q = 0; q < kWgXStages; ++q) {
+            tc::mbar_init(fullx + q, 1);
+            tc::mbar_init(emptyx + q, kWgWarps);
+        }
+        for (int q = 0; q < kWgZStages; ++q) {
+            tc::mbar_init(fullz + q, 1);
+            tc::mbar_init(emptyz + q, kWgWarps);
+        }
         tc::fence_mbar_init();
         s_fail = 0;
     }
-    if (warp == 0) {
-        tc::tmem_alloc(tslot, 512u);
-        tc::tmem_relinquish();
-    }
-    tc::tc_fence_before_sync();
     __syncthreads();
-    tc::tc_fence_after_sync();
-    const uint32_t tmem = *tslot;
-    const int P = g.TW + 2;
-    const int plane = (g.TH + 2) * P;
-    const uint32_t zbox = 16u * (uint32_t)plane, xbox = 16u * (uint32_t)plane * 3u;
-    const uint32_t idesc = tc::idesc_bf16(64, CIN, true, true);
-    const uint32_t zs = tc::smem_u32(zblk), xs = tc::smem_u32(xblk);
-    uint32_t ph_ld = 0, ph_mma = 0;
-    bool first = true, loads_in_flight = false;
-    for (long long tile = blockIdx.y; tile < g.ntiles && nt > 0; tile += gridDim.y) {
-        long long r = tile;
-        const int tw = (int)(r % g.tiles_w);
-        r /= g.tiles_w;
-        const int th = (int)(r % g.tiles_h);
-        r /= g.tiles_h;
-        const int z = (int)(r % g.D);
-        const int s = (int)(r / g.D);
-        const int w0 = tw * g.TW, h0 = th * g.TH;
-        const int rows = min(g.TH, g.H - h0);
-        if (tid == 0) {
-            tc::mbar_arrive_expect_tx(&bars[0], zc * zbox + KC * xbox);
-            for (int c = 0; c < zc; ++c)
-                tc::tma_load_5d(zblk + c * reg_z, &zmap, &bars[0], a.zcoff + 8 * c, w0 - 1, h0 - 1, z, s);
-            for (int c = 0; c < KC; ++c)
-                tc::tma_load_5d(xblk + c * reg_x, &xmap, &bars[0], a.xcoff + 8 * c, w0 - 1, h0 - 1, z - 1, s);
-        }
-        loads_in_flight = true;
-        if (!tc::mbar_wait(&bars[0], ph_ld)) s_fail = 1;
-        ph_ld ^= 1;
-        __syncthreads();
-        if (s_fail) break;
-        loads_in_flight = false;
-        tc::tc_fence_after_sync();
-        if (tid == 0) {
-            for (int ti = 0; ti < nt; ++ti) {
-                const int t = t_first + ti;
-                const int dz = t / 9, dy = (t / 3) % 3, dx = t % 3;
-                for (int row = 0; row < rows; ++row) {
-                    const int q0 = (row + 1) * P + 1;
-                    for (int k0 = 0; k0 < g.TW; k0 += 16) {
-                        const int qz = q0 + k0;
-                        const int qx = dz * plane + qz + (dy - 1) * P + (dx - 1);
-                        const uint64_t ad = tc::smem_desc(zs + (uint32_t)(qz * 16), 128, (uint32_t)reg_z);
-                        const uint64_t bd = tc::smem_desc(xs + (uint32_t)(qx * 16), 128, (uint32_t)reg_x);
-                        tc::mma_bf16(tmem + (uint32_t)(ti * CIN), ad, bd, idesc, first && row == 0 && k0 == 0 ? 0u : 1u);
+    const int cob = blockIdx.y / a.ciblocks, cib = blockIdx.y % a.ciblocks;
+    const int P = a.TW + 2;
+    auto unit = [&](long long u, int& w0, int& h0, int& z0, int& zn, int& s) {
+        w0 = (int)(u % a.tiles_w) * a.TW;
+        u /= a.tiles_w;
+        h0 = (int)(u % a.tiles_h) * a.TH;
+        u /= a.tiles_h;
+        z0 = (int)(u % a.nzc) * a.zc;
+        s = (int)(u / a.nzc);
+        zn = min(a.zc, a.D - z0);
+    };
+    if (warp == kWgWarps) {
+        if (lane == 0) {
+            const uint32_t xb = (uint32_t)((a.TH + 2) * P * RX), zb = (uint32_t)(a.TH * a.TW * RZ);
+            int sx = 0, sz = 0, nx = 0, nzl = 0;  // next stages, loads issued (up to the stages)
+            uint32_t phx = 1, phz = 1;            // parity of a free stage: the first pass finds them free
+            bool ok = true;
+            for (long long u = blockIdx.x; u < a.units && ok; u += gridDim.x) {
+                int w0, h0, z0, zn, s;
+                unit(u, w0, h0, z0, zn, s);
+                // X planes z0 - 1 .. z0 + zn; the dZ plane z goes out with the X plane z + 1
+                for (int z = z0 - 1; z <= z0 + zn && ok; ++z) {
+                    ok = tc::mbar_wait(emptyx + sx, phx) && !s_fail;
+                    if (!ok) break;
+                    tc::mbar_arrive_expect_tx(fullx + sx, xb);
+                    tc::tma_load_5d(xs + sx * a.xbytes, &xmap, fullx + sx, a.xcoff + cib * CI, w0 - 1, h0 - 1, z, s);
+                    nx = min(nx + 1, kWgXStages);
+                    if (++sx == kWgXStages) {
+                        sx = 0;
+                        phx ^= 1u;
+                    }
+                    if (z <= z0) continue;
+                    ok = tc::mbar_wait(emptyz + sz, phz) && !s_fail;
+                    if (!ok) break;
+                    tc::mbar_arrive_expect_tx(fullz + sz, zb);
+                    tc::tma_load_5d(zs + sz * a.zbytes, &zmap, fullz + sz, a.zcoff + cob * CO, w0, h0, z - 1, s);
+                    nzl = min(nzl + 1, kWgZStages);
+                    if (++sz == kWgZStages) {
+                        sz = 0;
+                        phz ^= 1u;
                     }
                 }
             }
-            tc::mma_commit(&bars[1]);
+            if (!ok) {
+                // the loads still in flight land before the block exits
+                s_fail = 1;
+                for (int q = 0; q < nx; ++q) tc::mbar_wait(fullx + q, q < sx ? phx ^ 1u : phx, 1000000000ull);
+                for (int q = 0; q < nzl; ++q) tc::mbar_wait(fullz + q, q < sz ? phz ^ 1u : phz, 1000000000ull);
+            }
         }
-        first = false;
-        if (!tc::mbar_wait(&bars[1], ph_mma)) s_fail = 1;
-        ph_mma ^= 1;
-        tc::tc_fence_before_sync();
-        __syncthreads();
-        if (s_fail) break;
-    }
-    if (!s_fail && !first) {
-        tc::tc_fence_after_sync();
-        // M = 64 accumulator rows: row r sits in TMEM lane (r % 16) + 32 (r / 16)
-        const int co = warp * 16 + lane;
-        for (int ti = 0; ti < nt; ++ti) {
+    } else {
+        const int dz = warp / 3, dy = warp - 3 * dz;
+        float acc[3][CO / 16][CI / 8][4];
 #pragma unroll
-            for (int c0 = 0; c0 < CIN; c0 += 16) {
-                float v[16];
-                tc::tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(ti * CIN + c0), v);
-                if (lane < 16 && co < a.cout) {
-                    // the parameter layout [cout][CIN][27]
-                    float* d = a.dw + ((size_t)co * CIN + c0) * 27 + (t_first + ti);
+        for (int t = 0; t < 3; ++t)
 #pragma unroll
-                    for (int u = 0; u < 16; ++u) atomicAdd(d + u * 27, v[u]);
+            for (int m = 0; m < CO / 16; ++m)
+#pragma unroll
+                for (int n = 0; n < CI / 8; ++n)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) acc[t][m][n][e] = 0.f;
+        // ldmatrix rows of this lane: A (voxel, chunk of 8 output channels), B (voxel, chunk of
+        // 8 input channels) of the fragment order of mma.m16n8k16
+        const int av = (lane & 7) + ((lane >> 4) << 3), ac = (lane >> 3) & 1;
+        const int bv = (lane & 7) + (((lane >> 3) & 1) << 3), bc = lane >> 4;
+        int sx = 0, sz = 0;  // stages of X plane z - 1 and of dZ plane z
+        uint32_t wx = 0, wz = 0;  // parities of the next X stage to wait for and of dZ
+        int nwx = 0;              // next X stage to wait for
+        const uint32_t xs0 = tc::smem_u32(xs), zs0 = tc::smem_u32(zs);
+        bool ok = true;
+        for (long long u = blockIdx.x; u < a.units && ok; u += gridDim.x) {
+            int w0, h0, z0, zn, s;
+            unit(u, w0, h0, z0, zn, s);
+            for (int z = z0; z < z0 + zn; ++z) {
+                for (int q = z == z0 ? 0 : 2; q < 3 && ok; ++q) {
+                    ok = tc::mbar_wait(fullx + nwx, wx) && !s_fail;
+                    if (++nwx == kWgXStages) {
+                        nwx = 0;
+                        wx ^= 1u;
+                    }
+                }
+                ok = ok && tc::mbar_wait(fullz + sz, wz) && !s_fail;
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                const int sp = sx + dz < kWgXStages ? sx + dz : sx + dz - kWgXStages;
+                const uint32_t xp = xs0 + (uint32_t)(sp * a.xbytes), zp = zs0 + (uint32_t)(sz * a.zbytes);
+                for (int r = 0; r < a.TH; ++r) {
+                    const int zrow = r * a.TW, xrow = (r + dy) * P;
+#pragma unroll 2
+                    for (int k0 = 0; k0 < a.TW; k0 += 16) {
+                        uint32_t af[CO / 16][4];
+#pragma unroll
+                        for (int m = 0; m < CO / 16; ++m)
+                            ldmatrix_x4_trans(zp + swizzled<RZ>(zrow + k0 + av, 2 * m + ac), af[m]);
+#pragma unroll
+                        for (int t = 0; t < 3; ++t)
+#pragma unroll
+                            for (int n = 0; n < CI / 16; ++n) {
+                                uint32_t bf_[4];
+                                ldmatrix_x4_trans(xp + swizzled<RX>(xrow + k0 + t + bv, 2 * n + bc), bf_);
+#pragma unroll
+                                for (int m = 0; m < CO / 16; ++m) {
+                                    mma_16816(acc[t][m][2 * n], af[m], bf_[0], bf_[1]);
+                                    mma_16816(acc[t][m][2 * n + 1], af[m], bf_[2], bf_[3]);
+                                }
+                            }
+                    }
+                }
+                __syncwarp();
+                // X plane z - 1 (and at the unit's end z and z + 1) and dZ plane z are free
+                for (int q = 0; q < (z == z0 + zn - 1 ? 3 : 1); ++q) {
+                    if (lane == 0) tc::mbar_arrive(emptyx + sx);
+                    if (++sx == kWgXStages) sx = 0;
+                }
+                if (lane == 0) tc::mbar_arrive(emptyz + sz);
+                if (++sz == kWgZStages) {
+                    sz = 0;
+                    wz ^= 1u;
                 }
             }
         }
+        if (!ok) {
+            s_fail = 1;
+        } else {
+            const int g = lane >> 2, t4 = lane & 3;
+#pragma unroll
+            for (int t = 0; t < 3; ++t)
+#pragma unroll
+                for (int m = 0; m < CO / 16; ++m)
+#pragma unroll
+                    for (int n = 0; n < CI / 8; ++n)
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            const int co = cob * CO + m * 16 + g + (e >> 1) * 8;
+                            const int ci = cib * CI + n * 8 + 2 * t4 + (e & 1);
+                            atomicAdd(a.dw + ((size_t)co * a.cin + ci) * 27 + dz * 9 + dy * 3 + t, acc[t][m][n][e]);
+                        }
+        }
     }
-    if (s_fail) {
-        if (tid == 0) atomicExch(a.err, 2);
-        if (loads_in_flight) tc::mbar_wait(&bars[0], ph_ld ^ 1, 1000000000ull);
-        __syncthreads();
-    }
-    tc::tc_fence_before_sync();
     __syncthreads();
-    if (warp == 0) tc::tmem_dealloc(tmem, 512u);
+    if (s_fail && tid == 0) atomicExch(a.err, 2);
 }
 
 // ------------------------------------------------------------------ SIMT kernels
