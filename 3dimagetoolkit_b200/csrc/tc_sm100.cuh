@@ -134,6 +134,19 @@ __device__ __forceinline__ void bulk_wait0()
     asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 
+// 16-byte asynchronous copy to shared memory; 16 zero bytes when !valid (nothing is read then)
+__device__ __forceinline__ void cp_async16_zfill(void* smem, const void* gmem, bool valid)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(smem)), "l"(gmem), "r"(valid ? 16 : 0)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait()
+{
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
 // Generic-proxy writes to shared memory become visible to the tensor core (async proxy).
 __device__ __forceinline__ void fence_proxy_async_smem()
 {

@@ -401,20 +401,52 @@ int alloc_acts(im3d_unet* n, size_t n1, std::string& err)
     return IM3D_OK;
 }
 
+// Transposed convolution: forward; weight, bias and data gradient.
+template <int CI, int CO, int VX, int OG>
+int up_fwd(cudaStream_t st, const bf16_t* in, const bf16_t* U, const float* b, int D2, int H2, int W2, int nsamp,
+           bf16_t* out, int op, int ooff, std::string& err)
+{
+    const long long n = (long long)nsamp * D2 * H2 * W2;
+    auto kern = upconv_fwd_kernel<CI, CO, VX, OG>;
+    const int smem = OG * CI * CO * 4;
+    UN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    kern<<<dim3((unsigned)flat_blocks(n / VX, 128), 8 / OG), 128, smem, st>>>(in, U, b, D2, H2, W2, nsamp, out, op, ooff);
+    return launch_status(err, "upconv_fwd");
+}
+
+template <int CI, int CO, int CB>
+int up_bwd(cudaStream_t st, const bf16_t* in, const bf16_t* gout, int gp, int goff, const bf16_t* U, int D2, int H2,
+           int W2, int nsamp, float* dU, float* db, bf16_t* gin, std::string& err)
+{
+    const long long n = (long long)nsamp * D2 * H2 * W2;
+    {
+        auto kern = upconv_wgrad_kernel<CI, CO>;
+        const int smem = 2 * UpWgrad<CI, CO>::stage;
+        UN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        const long long blocks = std::min<long long>(2ll * g_num_sms, (n + UpWgrad<CI, CO>::TP - 1) / UpWgrad<CI, CO>::TP);
+        kern<<<(unsigned)blocks, 256, smem, st>>>(in, gout, gp, goff, D2, H2, W2, nsamp, dU, db);
+        UN_TRY(launch_status(err, "upconv_wgrad"));
+    }
+    auto kern = upconv_bwd_kernel<CI, CO, CB>;
+    const int smem = 8 * CO * CB * 4;
+    UN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    kern<<<dim3((unsigned)flat_blocks(n, 128), CI / CB), 128, smem, st>>>(gout, gp, goff, U, in, D2, H2, W2, nsamp, gin);
+    return launch_status(err, "upconv_bwd");
+}
+
 // BF16 operand copies of the FP32 filters
 int pack_params(im3d_unet* n, cudaStream_t st, std::string& err)
 {
     if (n->packed) return IM3D_OK;
+    PackJobs jobs;
+    int count = 0;
     for (int l = 0; l < NCONV; ++l) {
-        pack_filter_kernel<<<flat_blocks(27LL * kCin[l] * kCout[l]), 256, 0, st>>>(
-            n->p + n->w_off[l], kCout[l], kCin[l], n->nout_f[l], 0, n->wf + n->wf_off[l]);
-        UN_TRY(launch_status(err, "pack_filter"));
-        if (l != E1A) {
-            pack_filter_kernel<<<flat_blocks(27LL * kCin[l] * kCout[l]), 256, 0, st>>>(
-                n->p + n->w_off[l], kCout[l], kCin[l], n->nout_d[l], 1, n->wd + n->wd_off[l]);
-            UN_TRY(launch_status(err, "pack_filter"));
-        }
+        jobs.job[count++] = PackJob{n->p + n->w_off[l], n->wf + n->wf_off[l], kCout[l], kCin[l], n->nout_f[l], 0};
+        if (l != E1A)
+            jobs.job[count++] = PackJob{n->p + n->w_off[l], n->wd + n->wd_off[l], kCout[l], kCin[l], n->nout_d[l], 1};
     }
+    pack_filter_kernel<<<dim3(16, (unsigned)count), 256, 0, st>>>(jobs);
+    UN_TRY(launch_status(err, "pack_filter"));
     to_bf16_kernel<<<flat_blocks(8 * 64 * 32), 256, 0, st>>>(n->p + n->up2_w, n->upk + n->upk2, 8 * 64 * 32);
     to_bf16_kernel<<<flat_blocks(8 * 32 * 16), 256, 0, st>>>(n->p + n->up1_w, n->upk + n->upk1, 8 * 32 * 16);
     UN_TRY(launch_status(err, "to_bf16"));
@@ -456,31 +488,27 @@ int forward(im3d_unet* n, cudaStream_t st, int nsamp, int D, int H, int W, float
     UN_TRY(conv(E1A, v, 0, n->a1, 16, 0));
     v.p = n->a1;
     UN_TRY(conv(E1B, v, 0, n->cat1, 32, 16));                    // a -> cat1[16:32]
-    pool_fwd_kernel<<<flat_blocks(n2 * 16), 256, 0, st>>>(n->cat1, 32, 16, 16, D, H, W, nsamp, n->p1, n->idx1);
+    pool_fwd_kernel<<<flat_blocks(n2 * 2), 256, 0, st>>>(n->cat1, 32, 16, 16, D, H, W, nsamp, n->p1, n->idx1);
     UN_TRY(launch_status(err, "pool_fwd"));
     View v2{n->p1, 16, D2, H2, W2, nsamp};
     UN_TRY(conv(E2A, v2, 0, n->b1, 32, 0));
     v2.p = n->b1;
     v2.pitch = 32;
     UN_TRY(conv(E2B, v2, 0, n->cat2, 64, 32));                   // b -> cat2[32:64]
-    pool_fwd_kernel<<<flat_blocks(n3 * 32), 256, 0, st>>>(n->cat2, 64, 32, 32, D2, H2, W2, nsamp, n->p2, n->idx2);
+    pool_fwd_kernel<<<flat_blocks(n3 * 4), 256, 0, st>>>(n->cat2, 64, 32, 32, D2, H2, W2, nsamp, n->p2, n->idx2);
     UN_TRY(launch_status(err, "pool_fwd"));
     View v3{n->p2, 32, D3, H3, W3, nsamp};
     UN_TRY(conv(E3A, v3, 0, n->c1, 64, 0));
     v3.p = n->c1;
     v3.pitch = 64;
     UN_TRY(conv(E3B, v3, 0, n->c, 64, 0));
-    upconv_fwd_kernel<64, 32><<<flat_blocks(n2, 128), 128, 0, st>>>(n->c, n->upk + n->upk2, n->p + n->up2_b, D3, H3,
-                                                                    W3, nsamp, n->cat2, 64, 0);
-    UN_TRY(launch_status(err, "upconv_fwd"));
+    UN_TRY((up_fwd<64, 32, 2, 2>(st, n->c, n->upk + n->upk2, n->p + n->up2_b, D3, H3, W3, nsamp, n->cat2, 64, 0, err)));
     View c2{n->cat2, 64, D2, H2, W2, nsamp};
     UN_TRY(conv(D2A, c2, 0, n->d2a, 32, 0));
     c2.p = n->d2a;
     c2.pitch = 32;
     UN_TRY(conv(D2B, c2, 0, n->d2, 32, 0));
-    upconv_fwd_kernel<32, 16><<<flat_blocks(n1, 128), 128, 0, st>>>(n->d2, n->upk + n->upk1, n->p + n->up1_b, D2, H2,
-                                                                    W2, nsamp, n->cat1, 32, 0);
-    UN_TRY(launch_status(err, "upconv_fwd"));
+    UN_TRY((up_fwd<32, 16, 2, 4>(st, n->d2, n->upk + n->upk1, n->p + n->up1_b, D2, H2, W2, nsamp, n->cat1, 32, 0, err)));
     View c1v{n->cat1, 32, D, H, W, nsamp};
     UN_TRY(conv(D1A, c1v, 0, n->d1a, 16, 0));
     c1v.p = n->d1a;
@@ -503,7 +531,7 @@ int backward(im3d_unet* n, cudaStream_t st, int nsamp, int D, int H, int W, cons
     const long long n1 = (long long)nsamp * D * H * W, n2 = n1 / 8, n3 = n1 / 64;
     zero_f32_kernel<<<flat_blocks(n->nparams), 256, 0, st>>>(n->g, (long long)n->nparams);
     UN_CUDA(cudaMemsetAsync(n->loss_d, 0, sizeof(double), st));
-    out_layer_kernel<16><<<flat_blocks(n1), 256, 0, st>>>(n->d1, n->p + n->out_w, n->p + n->out_b, n1, y, target, wt,
+    out_layer_kernel<16><<<flat_blocks(n1, 256 * 4), 256, 0, st>>>(n->d1, n->p + n->out_w, n->p + n->out_b, n1, y, target, wt,
                                                           1.f / (float)n1, n->g_d1, n->g + n->out_w, n->g + n->out_b,
                                                           n->loss_d);
     UN_TRY(launch_status(err, "out_layer"));
@@ -516,7 +544,11 @@ int backward(im3d_unet* n, cudaStream_t st, int nsamp, int D, int H, int W, cons
         int s = wgrad_any(st, kCin[l], x, xo, dz, zo, kCout[l], n->g + n->w_off[l], n->errf, err);
         if (s != IM3D_OK) return s;
         const long long nv = (long long)dz.nsamp * dz.D * dz.H * dz.W;
-        bias_grad_kernel<<<flat_blocks(nv), 256, 0, st>>>(dz.p, dz.pitch, zo, kCout[l], nv, n->g + n->b_off[l]);
+        float* db = n->g + n->b_off[l];
+        const int blocks = flat_blocks(nv * (kCout[l] / 8), 256 * 8);
+        if (kCout[l] == 16) bias_grad_kernel<16><<<blocks, 256, 0, st>>>(dz.p, dz.pitch, zo, nv, db);
+        else if (kCout[l] == 32) bias_grad_kernel<32><<<blocks, 256, 0, st>>>(dz.p, dz.pitch, zo, nv, db);
+        else bias_grad_kernel<64><<<blocks, 256, 0, st>>>(dz.p, dz.pitch, zo, nv, db);
         return launch_status(err, "bias_grad");
     };
     // level 1 decoder
@@ -527,12 +559,8 @@ int backward(im3d_unet* n, cudaStream_t st, int nsamp, int D, int H, int W, cons
     UN_TRY(wgrad(D1A, View{n->cat1, 32, D, H, W, nsamp}, 0, gd1a, 0));
     UN_TRY(dgrad(D1A, gd1a, 0, n->g_cat1, 32, 0, nullptr, 0, 0));  // [d up1 | d a (skip, raw)]
     // transposed convolution 1
-    upconv_wgrad_kernel<32, 16><<<flat_blocks(n2, 32), 256, 0, st>>>(n->d2, n->g_cat1, 32, 0, D2, H2, W2, nsamp,
-                                                                      n->g + n->up1_w, n->g + n->up1_b);
-    UN_TRY(launch_status(err, "upconv_wgrad"));
-    upconv_bwd_kernel<32, 16><<<flat_blocks(n2, 128), 128, 0, st>>>(n->g_cat1, 32, 0, n->upk + n->upk1, n->d2, D2, H2,
-                                                                    W2, nsamp, n->g_d2);
-    UN_TRY(launch_status(err, "upconv_bwd"));
+    UN_TRY((up_bwd<32, 16, 32>(st, n->d2, n->g_cat1, 32, 0, n->upk + n->upk1, D2, H2, W2, nsamp, n->g + n->up1_w,
+                               n->g + n->up1_b, n->g_d2, err)));
     // level 2 decoder
     View gd2{n->g_d2, 32, D2, H2, W2, nsamp};
     UN_TRY(wgrad(D2B, View{n->d2a, 32, D2, H2, W2, nsamp}, 0, gd2, 0));
@@ -541,12 +569,8 @@ int backward(im3d_unet* n, cudaStream_t st, int nsamp, int D, int H, int W, cons
     UN_TRY(wgrad(D2A, View{n->cat2, 64, D2, H2, W2, nsamp}, 0, gd2a, 0));
     UN_TRY(dgrad(D2A, gd2a, 0, n->g_cat2, 64, 0, nullptr, 0, 0));  // [d up2 | d b (skip, raw)]
     // transposed convolution 2
-    upconv_wgrad_kernel<64, 32><<<flat_blocks(n3, 32), 256, 0, st>>>(n->c, n->g_cat2, 64, 0, D3, H3, W3, nsamp,
-                                                                      n->g + n->up2_w, n->g + n->up2_b);
-    UN_TRY(launch_status(err, "upconv_wgrad"));
-    upconv_bwd_kernel<64, 32><<<flat_blocks(n3, 128), 128, 0, st>>>(n->g_cat2, 64, 0, n->upk + n->upk2, n->c, D3, H3,
-                                                                    W3, nsamp, n->g_c);
-    UN_TRY(launch_status(err, "upconv_bwd"));
+    UN_TRY((up_bwd<64, 32, 32>(st, n->c, n->g_cat2, 64, 0, n->upk + n->upk2, D3, H3, W3, nsamp, n->g + n->up2_w,
+                               n->g + n->up2_b, n->g_c, err)));
     // level 3
     View gc{n->g_c, 64, D3, H3, W3, nsamp};
     UN_TRY(wgrad(E3B, View{n->c1, 64, D3, H3, W3, nsamp}, 0, gc, 0));
@@ -555,7 +579,7 @@ int backward(im3d_unet* n, cudaStream_t st, int nsamp, int D, int H, int W, cons
     UN_TRY(wgrad(E3A, View{n->p2, 32, D3, H3, W3, nsamp}, 0, gc1, 0));
     UN_TRY(dgrad(E3A, gc1, 0, n->g_p2, 32, 0, nullptr, 0, 0));
     // pooling 2: g_b = (g_skip + scatter(g_p2)) * (b > 0), in place in g_cat2[32:64]
-    pool_bwd_kernel<<<flat_blocks(n3 * 32), 256, 0, st>>>(n->g_p2, n->idx2, 32, D2, H2, W2, nsamp, n->g_cat2, 64, 32,
+    pool_bwd_kernel<<<flat_blocks(n3 * 4), 256, 0, st>>>(n->g_p2, n->idx2, 32, D2, H2, W2, nsamp, n->g_cat2, 64, 32,
                                                           n->cat2, 64, 32, n->g_cat2, 64, 32);
     UN_TRY(launch_status(err, "pool_bwd"));
     View gb{n->g_cat2, 64, D2, H2, W2, nsamp};
@@ -565,7 +589,7 @@ int backward(im3d_unet* n, cudaStream_t st, int nsamp, int D, int H, int W, cons
     UN_TRY(wgrad(E2A, View{n->p1, 16, D2, H2, W2, nsamp}, 0, gb1, 0));
     UN_TRY(dgrad(E2A, gb1, 0, n->g_p1, 16, 0, nullptr, 0, 0));
     // pooling 1: g_a in place in g_cat1[16:32]
-    pool_bwd_kernel<<<flat_blocks(n2 * 16), 256, 0, st>>>(n->g_p1, n->idx1, 16, D, H, W, nsamp, n->g_cat1, 32, 16,
+    pool_bwd_kernel<<<flat_blocks(n2 * 2), 256, 0, st>>>(n->g_p1, n->idx1, 16, D, H, W, nsamp, n->g_cat1, 32, 16,
                                                           n->cat1, 32, 16, n->g_cat1, 32, 16);
     UN_TRY(launch_status(err, "pool_bwd"));
     View ga{n->g_cat1, 32, D, H, W, nsamp};
@@ -865,7 +889,9 @@ int im3d_conv3d_bf16(im3d_ctx* ctx, const uint16_t* x, int c_pitch, int c_off, i
         return IM3D_ERR_OOM;
     }
     cudaMemsetAsync(errf, 0, sizeof(int), st);
-    pack_filter_kernel<<<flat_blocks(27LL * cin * cout), 256, 0, st>>>(w, cout, cin, nout, 0, wpk);
+    PackJobs jobs;
+    jobs.job[0] = PackJob{w, wpk, cout, cin, nout, 0};
+    pack_filter_kernel<<<flat_blocks(27LL * cin * cout), 256, 0, st>>>(jobs);
     int s = launch_status(err, "pack_filter");
     const View v{reinterpret_cast<const bf16_t*>(x), c_pitch, nx, ny, nz, nsamp};
     if (s == IM3D_OK)

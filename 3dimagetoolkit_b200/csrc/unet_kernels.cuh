@@ -645,243 +645,405 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_mma_kernel(const __grid_c
 }
 
 // ------------------------------------------------------------------ SIMT kernels
-// sum over voxels of dZ[v][c] (c < C) into db[c]
-__global__ void bias_grad_kernel(const bf16_t* __restrict__ dz, int pitch, int coff, int C, long long n, float* db)
+// 8 BF16 channels as floats
+__device__ __forceinline__ void unpack8(const uint4& q, float (&v)[8])
 {
-    __shared__ float acc[64];
-    for (int c = threadIdx.x; c < 64; c += blockDim.x) acc[c] = 0.f;
+    const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        v[2 * e] = __uint_as_float(w[e] << 16);
+        v[2 * e + 1] = __uint_as_float(w[e] & 0xffff0000u);
+    }
+}
+__device__ __forceinline__ uint4 pack8(const float (&v)[8])
+{
+    return make_uint4(pack_bf(v[0], v[1]), pack_bf(v[2], v[3]), pack_bf(v[4], v[5]), pack_bf(v[6], v[7]));
+}
+
+// sum over voxels of dZ[v][c] (c < C) into db[c]; 8 channels per thread and read, the block's
+// sums added once (a scalar read and a shared atomic per thread took 35 us at 128^3 x 16,
+// bandwidth 11)
+template <int C>
+__global__ void __launch_bounds__(256) bias_grad_kernel(const bf16_t* __restrict__ dz, int pitch, int coff, long long n,
+                                                        float* db)
+{
+    constexpr int G = C / 8, LANES = 256 / G;
+    __shared__ float part[8][C];
+    const int g = threadIdx.x % G;
+    float s[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) s[e] = 0.f;
+    for (long long v = (long long)blockIdx.x * LANES + threadIdx.x / G; v < n; v += (long long)gridDim.x * LANES) {
+        float x[8];
+        unpack8(*reinterpret_cast<const uint4*>(dz + v * pitch + coff + 8 * g), x);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) s[e] += x[e];
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+#pragma unroll
+        for (int o = G; o < 32; o <<= 1) s[e] += __shfl_xor_sync(0xffffffffu, s[e], o);
+    if ((threadIdx.x & 31) < G)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) part[threadIdx.x >> 5][8 * g + e] = s[e];
     __syncthreads();
-    const int c = threadIdx.x % C;
-    const int lanes = blockDim.x / C;
-    float s = 0.f;
-    for (long long v = (long long)blockIdx.x * lanes + threadIdx.x / C; v < n; v += (long long)gridDim.x * lanes)
-        if (threadIdx.x < lanes * C) s += bf(dz[v * pitch + coff + c]);
-    if (threadIdx.x < lanes * C) atomicAdd(&acc[c], s);
-    __syncthreads();
-    for (int q = threadIdx.x; q < C; q += blockDim.x) atomicAdd(db + q, acc[q]);
+    if (threadIdx.x < C) {
+        float t = 0.f;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) t += part[w][threadIdx.x];
+        atomicAdd(db + threadIdx.x, t);
+    }
 }
 
 // 2x2x2 max pooling of channels [coff, coff + C) of `in` (pitch ip) into out [n/8][C]
-// (pitch C); idx receives the argmax child (0..7) per output value.
+// (pitch C); idx receives the argmax child (0..7) per output value. 8 channels per thread.
 __global__ void pool_fwd_kernel(const bf16_t* __restrict__ in, int ip, int coff, int C, int D, int H, int W,
                                 int nsamp, bf16_t* __restrict__ out, uint8_t* __restrict__ idx)
 {
-    const int D2 = D / 2, H2 = H / 2, W2 = W / 2;
-    const long long total = (long long)nsamp * D2 * H2 * W2 * C;
+    const int D2 = D / 2, H2 = H / 2, W2 = W / 2, G = C / 8;
+    const long long total = (long long)nsamp * D2 * H2 * W2 * G;
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
-        const int c = (int)(e % C);
-        long long p = e / C;
+        const int g = (int)(e % G);
+        const long long p = e / G;
         const int x = (int)(p % W2);
         long long r = p / W2;
         const int y = (int)(r % H2);
         r /= H2;
         const int z = (int)(r % D2);
         const int s = (int)(r / D2);
-        float best = -3.0e38f;
-        int bi = 0;
+        uint4 q[8];
 #pragma unroll
         for (int o = 0; o < 8; ++o) {
             const long long v = (((long long)s * D + 2 * z + (o >> 2)) * H + 2 * y + ((o >> 1) & 1)) * W + 2 * x + (o & 1);
-            const float f = bf(in[v * ip + coff + c]);
-            if (f > best) {
-                best = f;
-                bi = o;
-            }
+            q[o] = *reinterpret_cast<const uint4*>(in + v * ip + coff + 8 * g);
         }
-        out[e] = to_bf(best);
-        idx[e] = (uint8_t)bi;
+        float best[8];
+        uint32_t bi[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            best[c] = -3.0e38f;
+            bi[c] = 0;
+        }
+#pragma unroll
+        for (int o = 0; o < 8; ++o) {
+            float f[8];
+            unpack8(q[o], f);
+#pragma unroll
+            for (int c = 0; c < 8; ++c)
+                if (f[c] > best[c]) {
+                    best[c] = f[c];
+                    bi[c] = (uint32_t)o;
+                }
+        }
+        reinterpret_cast<uint4*>(out)[e] = pack8(best);
+        reinterpret_cast<uint2*>(idx)[e] = make_uint2(bi[0] | bi[1] << 8 | bi[2] << 16 | bi[3] << 24,
+                                                      bi[4] | bi[5] << 8 | bi[6] << 16 | bi[7] << 24);
     }
 }
 
 // Gradient of the pooled skip tensor: for every child cell of a pooled cell,
 //   g[child] = (g_skip[child] + (child == argmax ? g_pool : 0)) * (act[child] > 0)
-// (act = the pooled ReLU output). g may alias g_skip (same pitch and offset).
+// (act = the pooled ReLU output). g may alias g_skip (same pitch and offset). 8 channels per
+// thread, every child's reads before the first store.
 __global__ void pool_bwd_kernel(const bf16_t* __restrict__ gpool, const uint8_t* __restrict__ idx, int C, int D,
                                 int H, int W, int nsamp, const bf16_t* gskip, int sp, int soff,
                                 const bf16_t* __restrict__ act, int ap, int aoff, bf16_t* g, int gp, int goff)
 {
-    const int D2 = D / 2, H2 = H / 2, W2 = W / 2;
-    const long long total = (long long)nsamp * D2 * H2 * W2 * C;
+    const int D2 = D / 2, H2 = H / 2, W2 = W / 2, G = C / 8;
+    const long long total = (long long)nsamp * D2 * H2 * W2 * G;
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
-        const int c = (int)(e % C);
-        long long p = e / C;
+        const int c8 = 8 * (int)(e % G);
+        const long long p = e / G;
         const int x = (int)(p % W2);
         long long r = p / W2;
         const int y = (int)(r % H2);
         r /= H2;
         const int z = (int)(r % D2);
         const int s = (int)(r / D2);
-        const float gp_v = bf(gpool[e]);
-        const int bi = idx[e];
+        float gv[8];
+        unpack8(reinterpret_cast<const uint4*>(gpool)[e], gv);
+        const uint2 ix = reinterpret_cast<const uint2*>(idx)[e];
+        const long long v0 = (((long long)s * D + 2 * z) * H + 2 * y) * W + 2 * x;
 #pragma unroll
-        for (int o = 0; o < 8; ++o) {
-            const long long v = (((long long)s * D + 2 * z + (o >> 2)) * H + 2 * y + ((o >> 1) & 1)) * W + 2 * x + (o & 1);
-            float val = gskip ? bf(gskip[v * sp + soff + c]) : 0.f;
-            if (o == bi) val += gp_v;
-            if (!(bf(act[v * ap + aoff + c]) > 0.f)) val = 0.f;
-            g[v * gp + goff + c] = to_bf(val);
+        for (int oz = 0; oz < 2; ++oz) {
+            uint4 qs[4], qa[4];
+#pragma unroll
+            for (int o = 0; o < 4; ++o) {
+                const long long v = v0 + ((long long)oz * H + (o >> 1)) * W + (o & 1);
+                qs[o] = gskip ? *reinterpret_cast<const uint4*>(gskip + v * sp + soff + c8) : make_uint4(0, 0, 0, 0);
+                qa[o] = *reinterpret_cast<const uint4*>(act + v * ap + aoff + c8);
+            }
+#pragma unroll
+            for (int o = 0; o < 4; ++o) {
+                const long long v = v0 + ((long long)oz * H + (o >> 1)) * W + (o & 1);
+                float val[8], av[8];
+                unpack8(qs[o], val);
+                unpack8(qa[o], av);
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                    const uint32_t bi = ((c < 4 ? ix.x : ix.y) >> (8 * (c & 3))) & 0xffu;
+                    if (bi == (uint32_t)(4 * oz + o)) val[c] += gv[c];
+                    if (!(av[c] > 0.f)) val[c] = 0.f;
+                }
+                *reinterpret_cast<uint4*>(g + v * gp + goff + c8) = pack8(val);
+            }
         }
     }
 }
 
 // 2x2x2 stride-2 transposed convolution: out[child(p, o)][co] = b[co] + sum_ci
-// in[p][ci] U[o][ci][co]. One thread per output voxel; U (BF16) staged in shared memory.
-template <int CI, int CO>
+// in[p][ci] U[o][ci][co], the sum in the order of ci. A thread holds the channels of VX coarse
+// voxels and goes through the children of its block (blockIdx.y: OG of them) and 16 output
+// channels at a time; the filter sits in shared memory as floats and is read as broadcast
+// 16-byte vectors, the sums run on the paired FP32 instructions. (One thread per output voxel
+// with a 2-byte shared read per product took 266 us for 32 -> 16 channels at 128^3.)
+template <int CI, int CO, int VX, int OG>
 __global__ void __launch_bounds__(128) upconv_fwd_kernel(const bf16_t* __restrict__ in, const bf16_t* __restrict__ U,
                                                          const float* __restrict__ b, int D2, int H2, int W2, int nsamp,
                                                          bf16_t* out, int op, int ooff)
 {
-    __shared__ bf16_t us[8 * CI * CO];
-    for (int q = threadIdx.x; q < 8 * CI * CO; q += blockDim.x) us[q] = U[q];
+    extern __shared__ __align__(16) float us[];  // [OG][CI][CO]
+    const int o0 = blockIdx.y * OG;
+    for (int q = threadIdx.x; q < OG * CI * CO; q += blockDim.x) us[q] = bf(U[o0 * CI * CO + q]);
     __syncthreads();
-    const int D = 2 * D2, H = 2 * H2, W = 2 * W2;
-    const long long total = (long long)nsamp * D * H * W;
-    for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < total; v += (long long)gridDim.x * blockDim.x) {
-        const int x = (int)(v % W);
-        long long r = v / W;
-        const int y = (int)(r % H);
-        r /= H;
-        const int z = (int)(r % D);
-        const int s = (int)(r / D);
-        const int o = ((z & 1) << 2) | ((y & 1) << 1) | (x & 1);
-        const long long p = (((long long)s * D2 + (z >> 1)) * H2 + (y >> 1)) * W2 + (x >> 1);
-        float acc[CO];
+    const int H = 2 * H2, W = 2 * W2;
+    const long long total = (long long)nsamp * D2 * H2 * W2;  // a multiple of VX
+    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t * VX < total; t += (long long)gridDim.x * blockDim.x) {
+        const long long p = t * VX;
+        uint4 xq[VX][CI / 8];
 #pragma unroll
-        for (int co = 0; co < CO; ++co) acc[co] = b[co];
-        const uint4* ip = reinterpret_cast<const uint4*>(in + p * CI);
-        for (int c8 = 0; c8 < CI / 8; ++c8) {
-            const uint4 w4 = ip[c8];
-            const uint32_t u4[4] = {w4.x, w4.y, w4.z, w4.w};
+        for (int v = 0; v < VX; ++v)
 #pragma unroll
-            for (int h = 0; h < 8; ++h) {
-                const float xv = bf((bf16_t)(h & 1 ? u4[h >> 1] >> 16 : u4[h >> 1] & 0xffff));
-                const bf16_t* urow = us + (o * CI + c8 * 8 + h) * CO;
+            for (int c = 0; c < CI / 8; ++c) xq[v][c] = reinterpret_cast<const uint4*>(in + (p + v) * CI)[c];
+        const int x = (int)(p % W2);  // the VX voxels lie in one row (W2 a multiple of VX)
+        long long r = p / W2;
+        const int y = (int)(r % H2);
+        r /= H2;  // r = s * D2 + z
+        for (int og = 0; og < OG; ++og) {
+            const int o = o0 + og;
+            const long long vox = ((2 * r + (o >> 2)) * H + 2 * y + ((o >> 1) & 1)) * W + 2 * x + (o & 1);
 #pragma unroll
-                for (int co = 0; co < CO; ++co) acc[co] = fmaf(xv, bf(urow[co]), acc[co]);
+            for (int h = 0; h < CO / 16; ++h) {
+                float2 acc[VX][8];
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                    const float2 bb = make_float2(__ldg(b + h * 16 + 2 * c), __ldg(b + h * 16 + 2 * c + 1));
+#pragma unroll
+                    for (int v = 0; v < VX; ++v) acc[v][c] = bb;
+                }
+                const float* ub = us + og * CI * CO + h * 16;
+#pragma unroll
+                for (int c8 = 0; c8 < CI / 8; ++c8) {
+                    float xv[VX][8];
+#pragma unroll
+                    for (int v = 0; v < VX; ++v) unpack8(xq[v][c8], xv[v]);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) {
+                        const float4* u4 = reinterpret_cast<const float4*>(ub + (c8 * 8 + e) * CO);
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) {
+                            const float4 w = u4[c];
+#pragma unroll
+                            for (int v = 0; v < VX; ++v) {
+                                const float2 x2 = make_float2(xv[v][e], xv[v][e]);
+                                acc[v][2 * c] = __ffma2_rn(x2, make_float2(w.x, w.y), acc[v][2 * c]);
+                                acc[v][2 * c + 1] = __ffma2_rn(x2, make_float2(w.z, w.w), acc[v][2 * c + 1]);
+                            }
+                        }
+                    }
+                }
+#pragma unroll
+                for (int v = 0; v < VX; ++v) {
+                    uint4* dst = reinterpret_cast<uint4*>(out + (vox + 2 * v) * op + ooff + h * 16);
+                    dst[0] = make_uint4(pack_bf(acc[v][0].x, acc[v][0].y), pack_bf(acc[v][1].x, acc[v][1].y),
+                                        pack_bf(acc[v][2].x, acc[v][2].y), pack_bf(acc[v][3].x, acc[v][3].y));
+                    dst[1] = make_uint4(pack_bf(acc[v][4].x, acc[v][4].y), pack_bf(acc[v][5].x, acc[v][5].y),
+                                        pack_bf(acc[v][6].x, acc[v][6].y), pack_bf(acc[v][7].x, acc[v][7].y));
+                }
             }
-        }
-        uint4* dst = reinterpret_cast<uint4*>(out + v * op + ooff);
-#pragma unroll
-        for (int n8 = 0; n8 < CO / 8; ++n8) {
-            uint4 pk;
-            pk.x = (uint32_t)to_bf(acc[n8 * 8 + 0]) | ((uint32_t)to_bf(acc[n8 * 8 + 1]) << 16);
-            pk.y = (uint32_t)to_bf(acc[n8 * 8 + 2]) | ((uint32_t)to_bf(acc[n8 * 8 + 3]) << 16);
-            pk.z = (uint32_t)to_bf(acc[n8 * 8 + 4]) | ((uint32_t)to_bf(acc[n8 * 8 + 5]) << 16);
-            pk.w = (uint32_t)to_bf(acc[n8 * 8 + 6]) | ((uint32_t)to_bf(acc[n8 * 8 + 7]) << 16);
-            dst[n8] = pk;
         }
     }
 }
 
 // Data gradient of the transposed convolution, masked by the ReLU of its input:
-//   g_in[p][ci] = (sum_{o, co} g_out[child(p, o)][co] U[o][ci][co]) * (in[p][ci] > 0)
-template <int CI, int CO>
+//   g_in[p][ci] = (sum_{o, co} g_out[child(p, o)][co] U[o][ci][co]) * (in[p][ci] > 0),
+// the sum in the order of o, co. One coarse voxel and CB input channels (blockIdx.y) per
+// thread; the filter sits in shared memory as floats, [o][co][ci of the block].
+template <int CI, int CO, int CB>
 __global__ void __launch_bounds__(128) upconv_bwd_kernel(const bf16_t* __restrict__ gout, int gp, int goff,
                                                          const bf16_t* __restrict__ U, const bf16_t* __restrict__ in,
                                                          int D2, int H2, int W2, int nsamp, bf16_t* __restrict__ gin)
 {
-    __shared__ bf16_t us[8 * CI * CO];
-    for (int q = threadIdx.x; q < 8 * CI * CO; q += blockDim.x) us[q] = U[q];
+    extern __shared__ __align__(16) float us[];  // [8][CO][CB]
+    const int c0 = blockIdx.y * CB;
+    for (int q = threadIdx.x; q < 8 * CO * CB; q += blockDim.x) {
+        const int ci = q % CB, co = q / CB % CO, o = q / (CB * CO);
+        us[q] = bf(U[(o * CI + c0 + ci) * CO + co]);
+    }
     __syncthreads();
-    const int D = 2 * D2, H = 2 * H2, W = 2 * W2;
+    const int H = 2 * H2, W = 2 * W2;
     const long long total = (long long)nsamp * D2 * H2 * W2;
     for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < total; p += (long long)gridDim.x * blockDim.x) {
         const int x = (int)(p % W2);
         long long r = p / W2;
         const int y = (int)(r % H2);
         r /= H2;
-        const int z = (int)(r % D2);
-        const int s = (int)(r / D2);
-        float acc[CI];
+        float2 acc[CB / 2];
 #pragma unroll
-        for (int ci = 0; ci < CI; ++ci) acc[ci] = 0.f;
+        for (int c = 0; c < CB / 2; ++c) acc[c] = make_float2(0.f, 0.f);
         for (int o = 0; o < 8; ++o) {
-            const long long v = (((long long)s * D + 2 * z + (o >> 2)) * H + 2 * y + ((o >> 1) & 1)) * W + 2 * x + (o & 1);
-            const bf16_t* gr = gout + v * gp + goff;
-            for (int co = 0; co < CO; ++co) {
-                const float gv = bf(gr[co]);
+            const long long v = ((2 * r + (o >> 2)) * H + 2 * y + ((o >> 1) & 1)) * W + 2 * x + (o & 1);
+            const uint4* gr = reinterpret_cast<const uint4*>(gout + v * gp + goff);
 #pragma unroll
-                for (int ci = 0; ci < CI; ++ci) acc[ci] = fmaf(gv, bf(us[(o * CI + ci) * CO + co]), acc[ci]);
+            for (int c8 = 0; c8 < CO / 8; ++c8) {
+                float gv[8];
+                unpack8(gr[c8], gv);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    const float4* u4 = reinterpret_cast<const float4*>(us + (o * CO + c8 * 8 + e) * CB);
+                    const float2 g2 = make_float2(gv[e], gv[e]);
+#pragma unroll
+                    for (int c = 0; c < CB / 4; ++c) {
+                        const float4 w = u4[c];
+                        acc[2 * c] = __ffma2_rn(g2, make_float2(w.x, w.y), acc[2 * c]);
+                        acc[2 * c + 1] = __ffma2_rn(g2, make_float2(w.z, w.w), acc[2 * c + 1]);
+                    }
+                }
             }
         }
+        const uint4* ip = reinterpret_cast<const uint4*>(in + p * CI + c0);
+        uint4* dst = reinterpret_cast<uint4*>(gin + p * CI + c0);
 #pragma unroll
-        for (int ci = 0; ci < CI; ++ci) {
-            const float m = bf(in[p * CI + ci]) > 0.f ? 1.f : 0.f;
-            gin[p * CI + ci] = to_bf(acc[ci] * m);
+        for (int c8 = 0; c8 < CB / 8; ++c8) {
+            float iv[8], ov[8];
+            unpack8(ip[c8], iv);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const float a = e & 1 ? acc[c8 * 4 + e / 2].y : acc[c8 * 4 + e / 2].x;
+                ov[e] = a * (iv[e] > 0.f ? 1.f : 0.f);
+            }
+            dst[c8] = pack8(ov);
         }
     }
 }
 
 // Weight and bias gradient of the transposed convolution:
-//   dU[o][ci][co] += sum_p in[p][ci] g_out[child(p, o)][co],  db[co] += sum g_out[.][co].
-// Each block folds a range of p in registers (one (o, ci, co) set per thread) and adds
-// its partial sums once.
+//   dU[o][ci][co] += sum_p in[p][ci] g_out[child(p, o)][co],  db[co] += sum g_out[.][co],
+// as products of M = 16 input channels, N = 8 output channels and K = 16 coarse voxels on
+// mma.sync with FP32 accumulators in registers; warp o takes child o. A block stages 64
+// coarse voxels (4 row segments of 16) and their 512 children at a time, two stages ahead of
+// each other, in rows padded by 16 bytes (ldmatrix reads 8 rows on distinct banks), and adds
+// its sums once. (One scalar product per thread and voxel took 550 us for 32 -> 16 channels at
+// 128^3.)
+template <int CI, int CO>
+struct UpWgrad {
+    static constexpr int TP = 64, RI = 2 * CI + 16, RG = 2 * CO + 16;      // voxels, row bytes
+    static constexpr int stage = TP * RI + 8 * TP * RG;                     // bytes
+};
 template <int CI, int CO>
 __global__ void __launch_bounds__(256) upconv_wgrad_kernel(const bf16_t* __restrict__ in,
                                                            const bf16_t* __restrict__ gout, int gp, int goff,
                                                            int D2, int H2, int W2, int nsamp, float* dU, float* db)
 {
-    constexpr int NW = 8 * CI * CO;
-    constexpr int PER = (NW + 255) / 256;
-    constexpr int TP = 32;  // positions staged at once
-    __shared__ float xs[TP][CI];
-    __shared__ float gs[TP][8][CO];
-    float acc[PER];
+    typedef UpWgrad<CI, CO> G;
+    constexpr int TP = G::TP, RI = G::RI, RG = G::RG;
+    extern __shared__ __align__(16) unsigned char sm[];
+    const int tid = threadIdx.x, lane = tid & 31, o = tid >> 5;
+    const int H = 2 * H2, W = 2 * W2;
+    const long long total = (long long)nsamp * D2 * H2 * W2;  // a multiple of 16
+    const long long tiles = (total + TP - 1) / TP;
+    // stage s: in[TP][CI], then children [8][TP][CO]
+    auto load = [&](long long tile, int s) {
+        unsigned char* bi = sm + s * G::stage;
+        unsigned char* bg = bi + TP * RI;
+        for (int q = tid; q < TP * (CI / 8); q += 256) {
+            const int v = q / (CI / 8), c = q % (CI / 8);
+            const long long p = tile * TP + v;
+            tc::cp_async16_zfill(bi + v * RI + c * 16, p < total ? in + p * CI + 8 * c : in, p < total);
+        }
+        for (int q = tid; q < 8 * TP * (CO / 8); q += 256) {
+            const int c = q % (CO / 8), f = q / (CO / 8);
+            const int ox = f & 1, v = (f >> 1) % TP, zy = f / (2 * TP);  // children of a row side by side
+            const long long p = tile * TP + v;
+            const int x = (int)(p % W2);
+            long long r = p / W2;
+            const int y = (int)(r % H2);
+            r /= H2;
+            const long long vox = ((2 * r + (zy >> 1)) * H + 2 * y + (zy & 1)) * W + 2 * x + ox;
+            tc::cp_async16_zfill(bg + ((zy * 2 + ox) * TP + v) * RG + c * 16,
+                                 p < total ? gout + vox * gp + goff + 8 * c : gout, p < total);
+        }
+        tc::cp_async_commit();
+    };
+    float acc[CI / 16][CO / 8][4], bs[CO / 8];
 #pragma unroll
-    for (int u = 0; u < PER; ++u) acc[u] = 0.f;
-    float bacc = 0.f;
-    const int D = 2 * D2, H = 2 * H2, W = 2 * W2;
-    const long long total = (long long)nsamp * D2 * H2 * W2;
-    for (long long p0 = (long long)blockIdx.x * TP; p0 < total; p0 += (long long)gridDim.x * TP) {
-        __syncthreads();
-        for (int q = threadIdx.x; q < TP * CI; q += blockDim.x) {
-            const long long p = p0 + q / CI;
-            xs[q / CI][q % CI] = p < total ? bf(in[p * CI + q % CI]) : 0.f;
-        }
-        for (int q = threadIdx.x; q < TP * 8 * CO; q += blockDim.x) {
-            const int pi = q / (8 * CO), o = (q / CO) % 8, co = q % CO;
-            const long long p = p0 + pi;
-            float gv = 0.f;
-            if (p < total) {
-                const int x = (int)(p % W2);
-                long long r = p / W2;
-                const int y = (int)(r % H2);
-                r /= H2;
-                const int z = (int)(r % D2);
-                const int s = (int)(r / D2);
-                const long long v = (((long long)s * D + 2 * z + (o >> 2)) * H + 2 * y + ((o >> 1) & 1)) * W + 2 * x + (o & 1);
-                gv = bf(gout[v * gp + goff + co]);
-            }
-            gs[pi][o][co] = gv;
-        }
-        __syncthreads();
+    for (int n = 0; n < CO / 8; ++n) {
+        bs[n] = 0.f;
 #pragma unroll
-        for (int u = 0; u < PER; ++u) {
-            const int w = threadIdx.x + u * 256;
-            if (w < NW) {
-                const int o = w / (CI * CO), ci = (w / CO) % CI, co = w % CO;
-                float sacc = 0.f;
-                for (int pi = 0; pi < TP; ++pi) sacc = fmaf(xs[pi][ci], gs[pi][o][co], sacc);
-                acc[u] += sacc;
-            }
-        }
-        if (threadIdx.x < CO)
-            for (int pi = 0; pi < TP; ++pi)
-                for (int o = 0; o < 8; ++o) bacc += gs[pi][o][threadIdx.x];
+        for (int m = 0; m < CI / 16; ++m)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[m][n][e] = 0.f;
     }
+    const int av = (lane & 7) + ((lane >> 4) << 3), ac = (lane >> 3) & 1;
+    const int bv = (lane & 7) + (((lane >> 3) & 1) << 3), bc = lane >> 4;
+    long long tile = blockIdx.x;
+    if (tile < tiles) load(tile, 0);
+    for (int s = 0; tile < tiles; tile += gridDim.x, s ^= 1) {
+        if (tile + gridDim.x < tiles) {
+            load(tile + gridDim.x, s ^ 1);
+            tc::cp_async_wait<1>();
+        } else {
+            tc::cp_async_wait<0>();
+        }
+        __syncthreads();
+        const uint32_t bi = tc::smem_u32(sm + s * G::stage), bg = bi + TP * RI + (uint32_t)(o * TP * RG);
 #pragma unroll
-    for (int u = 0; u < PER; ++u) {
-        const int w = threadIdx.x + u * 256;
-        if (w < NW) atomicAdd(dU + w, acc[u]);
+        for (int k0 = 0; k0 < TP; k0 += 16) {
+            uint32_t af[CI / 16][4];
+#pragma unroll
+            for (int m = 0; m < CI / 16; ++m)
+                ldmatrix_x4_trans(bi + (uint32_t)((k0 + av) * RI + (2 * m + ac) * 16), af[m]);
+#pragma unroll
+            for (int n = 0; n < CO / 16; ++n) {
+                uint32_t gf[4];
+                ldmatrix_x4_trans(bg + (uint32_t)((k0 + bv) * RG + (2 * n + bc) * 16), gf);
+#pragma unroll
+                for (int m = 0; m < CI / 16; ++m) {
+                    mma_16816(acc[m][2 * n], af[m], gf[0], gf[1]);
+                    mma_16816(acc[m][2 * n + 1], af[m], gf[2], gf[3]);
+                }
+                // this lane's share of the bias sums: channel lane / 4 of each 8, 4 voxels
+#pragma unroll
+                for (int h = 0; h < 4; ++h)
+                    bs[2 * n + (h >> 1)] += __uint_as_float(gf[h] << 16) + __uint_as_float(gf[h] & 0xffff0000u);
+            }
+        }
+        __syncthreads();
     }
-    if (threadIdx.x < CO) atomicAdd(db + threadIdx.x, bacc);
+    const int g = lane >> 2, t4 = lane & 3;
+#pragma unroll
+    for (int m = 0; m < CI / 16; ++m)
+#pragma unroll
+        for (int n = 0; n < CO / 8; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int ci = m * 16 + g + (e >> 1) * 8, co = n * 8 + 2 * t4 + (e & 1);
+                atomicAdd(dU + (o * CI + ci) * CO + co, acc[m][n][e]);
+            }
+#pragma unroll
+    for (int n = 0; n < CO / 8; ++n) {
+        bs[n] += __shfl_xor_sync(0xffffffffu, bs[n], 1);
+        bs[n] += __shfl_xor_sync(0xffffffffu, bs[n], 2);
+        if (t4 == 0) atomicAdd(db + n * 8 + g, bs[n]);
+    }
 }
 
 // 1x1 output layer, loss and its gradient in one pass:
 //   y = b + sum_c w[c] d[v][c];  diff = y - target (on the cells with weight != 0);
 //   loss += diff^2 * wt; dy = 2 diff wt / count;  g_d[v][c] = dy w[c] (d[v][c] > 0);
 //   dw[c] += dy d[v][c], db += dy.
-// target == NULL: forward only (y written, nothing else).
+// target == NULL: forward only (y written, nothing else). The sums are folded by shuffles and
+// one add per block (a shared atomic per thread and channel took 650 of 668 us at 128^3).
 template <int C>
 __global__ void __launch_bounds__(256) out_layer_kernel(const bf16_t* __restrict__ d, const float* __restrict__ w,
                                                         const float* __restrict__ b, long long n, float* y,
@@ -889,18 +1051,12 @@ __global__ void __launch_bounds__(256) out_layer_kernel(const bf16_t* __restrict
                                                         const float* __restrict__ wt, float inv_count,
                                                         bf16_t* __restrict__ gd, float* dw, float* db, double* loss)
 {
-    __shared__ float sw[C];
-    __shared__ float sg[C + 1];
-    __shared__ double sl;
-    if (threadIdx.x < C) {
-        sw[threadIdx.x] = w[threadIdx.x];
-        sg[threadIdx.x] = 0.f;
-    }
-    if (threadIdx.x == 0) {
-        sg[C] = 0.f;
-        sl = 0.0;
-    }
-    __syncthreads();
+    __shared__ float sg[8][C + 1];
+    __shared__ double sl[8];
+    float wv_[C];
+#pragma unroll
+    for (int c = 0; c < C; ++c) wv_[c] = __ldg(w + c);
+    const float bias = __ldg(b);
     float gl[C];
 #pragma unroll
     for (int c = 0; c < C; ++c) gl[c] = 0.f;
@@ -911,14 +1067,14 @@ __global__ void __launch_bounds__(256) out_layer_kernel(const bf16_t* __restrict
         const uint4* dp = reinterpret_cast<const uint4*>(d + v * C);
 #pragma unroll
         for (int c8 = 0; c8 < C / 8; ++c8) {
-            const uint4 q = dp[c8];
-            const uint32_t u4[4] = {q.x, q.y, q.z, q.w};
+            float t[8];
+            unpack8(dp[c8], t);
 #pragma unroll
-            for (int h = 0; h < 8; ++h) dv[c8 * 8 + h] = bf((bf16_t)(h & 1 ? u4[h >> 1] >> 16 : u4[h >> 1] & 0xffff));
+            for (int h = 0; h < 8; ++h) dv[c8 * 8 + h] = t[h];
         }
-        float yv = b[0];
+        float yv = bias;
 #pragma unroll
-        for (int c = 0; c < C; ++c) yv = fmaf(sw[c], dv[c], yv);
+        for (int c = 0; c < C; ++c) yv = fmaf(wv_[c], dv[c], yv);
         if (y) y[v] = yv;
         if (!target) continue;
         const float wv = wt ? wt[v] : 1.f;
@@ -926,33 +1082,46 @@ __global__ void __launch_bounds__(256) out_layer_kernel(const bf16_t* __restrict
         ls += (double)diff * diff;
         const float dy = 2.f * diff * wv * inv_count;
         gb += dy;
-        bf16_t go[C];
-#pragma unroll
-        for (int c = 0; c < C; ++c) {
-            gl[c] = fmaf(dy, dv[c], gl[c]);
-            go[c] = to_bf(dv[c] > 0.f ? dy * sw[c] : 0.f);
-        }
         uint4* gp = reinterpret_cast<uint4*>(gd + v * C);
 #pragma unroll
         for (int c8 = 0; c8 < C / 8; ++c8) {
-            uint4 q;
-            q.x = (uint32_t)go[c8 * 8 + 0] | ((uint32_t)go[c8 * 8 + 1] << 16);
-            q.y = (uint32_t)go[c8 * 8 + 2] | ((uint32_t)go[c8 * 8 + 3] << 16);
-            q.z = (uint32_t)go[c8 * 8 + 4] | ((uint32_t)go[c8 * 8 + 5] << 16);
-            q.w = (uint32_t)go[c8 * 8 + 6] | ((uint32_t)go[c8 * 8 + 7] << 16);
-            gp[c8] = q;
+            float go[8];
+#pragma unroll
+            for (int h = 0; h < 8; ++h) {
+                const int c = c8 * 8 + h;
+                gl[c] = fmaf(dy, dv[c], gl[c]);
+                go[h] = dv[c] > 0.f ? dy * wv_[c] : 0.f;
+            }
+            gp[c8] = pack8(go);
         }
     }
     if (!target) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-    for (int c = 0; c < C; ++c) atomicAdd(&sg[c], gl[c]);
-    atomicAdd(&sg[C], gb);
-    atomicAdd(&sl, ls);
+    for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+        for (int c = 0; c < C; ++c) gl[c] += __shfl_xor_sync(0xffffffffu, gl[c], o);
+        gb += __shfl_xor_sync(0xffffffffu, gb, o);
+        ls += __shfl_xor_sync(0xffffffffu, ls, o);
+    }
+    if (lane == 0) {
+#pragma unroll
+        for (int c = 0; c < C; ++c) sg[warp][c] = gl[c];
+        sg[warp][C] = gb;
+        sl[warp] = ls;
+    }
     __syncthreads();
-    if (threadIdx.x < C) atomicAdd(dw + threadIdx.x, sg[threadIdx.x]);
-    if (threadIdx.x == 0) {
-        atomicAdd(db, sg[C]);
-        atomicAdd(loss, sl);
+    if (threadIdx.x <= C) {
+        float t = 0.f;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) t += sg[q][threadIdx.x];
+        atomicAdd(threadIdx.x < C ? dw + threadIdx.x : db, t);
+    }
+    if (threadIdx.x == 32) {
+        double t = 0;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) t += sl[q];
+        atomicAdd(loss, t);
     }
 }
 
@@ -977,28 +1146,39 @@ __global__ void adam_kernel(float* __restrict__ p, const float* __restrict__ g, 
 //     (CIN = layer Cin)
 //   data gradient (transpose = 1): the flipped, transposed filter, CIN = layer Cout,
 //     outputs = layer Cin: W[kc*8 + e][nb*NOUT + n][26 - (9 dz + t)]
-__global__ void pack_filter_kernel(const float* __restrict__ W, int cout, int cin, int nout, int transpose,
-                                   bf16_t* __restrict__ out)
+struct PackJob {
+    const float* W;
+    bf16_t* out;
+    int cout, cin, nout, transpose;
+};
+struct PackJobs {
+    PackJob job[20];
+};
+__device__ __forceinline__ void pack_filter(const PackJob& j, long long first, long long step)
 {
-    const int kcin = transpose ? cout : cin;   // K of the GEMM
-    const int nall = transpose ? cin : cout;   // N of the GEMM
-    const int nblocks = nall / nout;
-    const long long total = (long long)nblocks * 27 * kcin * nout;
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
+    const int kcin = j.transpose ? j.cout : j.cin;   // K of the GEMM
+    const int nall = j.transpose ? j.cin : j.cout;   // N of the GEMM
+    const long long total = 27ll * kcin * nall;
+    for (long long e = first; e < total; e += step) {
         const int el = (int)(e % 8);
         long long r = e / 8;
-        const int n = (int)(r % nout);
-        r /= nout;
+        const int n = (int)(r % j.nout);
+        r /= j.nout;
         const int dz = 2 - (int)(r % 3);
         r /= 3;
         const int kc = (int)(r % (kcin / 8));
         r /= kcin / 8;
         const int t = 9 * dz + (int)(r % 9);
         const int nb = (int)(r / 9);
-        const int k = kc * 8 + el, nn = nb * nout + n;
-        const float w = transpose ? W[((size_t)k * cin + nn) * 27 + (26 - t)] : W[((size_t)nn * cin + k) * 27 + t];
-        out[e] = to_bf(w);
+        const int k = kc * 8 + el, nn = nb * j.nout + n;
+        const float w = j.transpose ? j.W[((size_t)k * j.cin + nn) * 27 + (26 - t)] : j.W[((size_t)nn * j.cin + k) * 27 + t];
+        j.out[e] = to_bf(w);
     }
+}
+// one filter per blockIdx.y
+__global__ void pack_filter_kernel(const __grid_constant__ PackJobs jobs)
+{
+    pack_filter(jobs.job[blockIdx.y], blockIdx.x * (long long)blockDim.x + threadIdx.x, (long long)gridDim.x * blockDim.x);
 }
 
 __global__ void to_bf16_kernel(const float* __restrict__ src, bf16_t* __restrict__ dst, long long n)
