@@ -99,6 +99,7 @@ struct im3d_ctx {
     int resume_esize = 0;
     im3d_rsfe_checkpoint resume_from{};
     long long residual_checks = 0;  // rb_check calls, for the statistics
+    void* conv_ws = nullptr;        // im3d_ctx_conv_workspace
 };
 
 namespace {
@@ -2848,6 +2849,7 @@ int enter(im3d_ctx* ctx)
 cudaStream_t im3d_ctx_stream(im3d_ctx* ctx) { return ctx->stream; }
 int im3d_ctx_device(im3d_ctx* ctx) { return ctx->device; }
 std::string& im3d_ctx_error_ref(im3d_ctx* ctx) { return ctx->err; }
+void*& im3d_ctx_conv_workspace(im3d_ctx* ctx) { return ctx->conv_ws; }
 
 // ====================================================================== C ABI
 #endif
@@ -2902,6 +2904,7 @@ int im3d_ctx_destroy(im3d_ctx* ctx)
     cudaSetDevice(ctx->device);
     for (auto& kv : ctx->bufs)
         if (kv.second.p) cudaFree(kv.second.p);
+    if (ctx->conv_ws) cudaFree(ctx->conv_ws);
     if (ctx->ctrl_d) cudaFree(ctx->ctrl_d);
     if (ctx->ctrl_h) cudaFreeHost(ctx->ctrl_h);
     for (auto& e : ctx->ev)

@@ -12,6 +12,9 @@
 cudaStream_t im3d_ctx_stream(im3d_ctx* ctx);
 int im3d_ctx_device(im3d_ctx* ctx);
 std::string& im3d_ctx_error_ref(im3d_ctx* ctx);
+// Device workspace of im3d_conv3d_bf16 (its packed filter and error flag), allocated by its
+// first call on the context and freed with it; not part of the context's memory budget.
+void*& im3d_ctx_conv_workspace(im3d_ctx* ctx);
 
 namespace im3d {
 namespace unet {

@@ -874,39 +874,36 @@ int im3d_conv3d_bf16(im3d_ctx* ctx, const uint16_t* x, int c_pitch, int c_off, i
         err = "conv3d: x, w, bias and out must be device memory";
         return IM3D_ERR_INVALID_ARG;
     }
-    UN_CUDA(cudaSetDevice(im3d_ctx_device(ctx)));
+    const int dev = im3d_ctx_device(ctx);
+    UN_CUDA(cudaSetDevice(dev));
     cudaStream_t st = im3d_ctx_stream(ctx);
-    cudaDeviceProp prop;
-    UN_CUDA(cudaGetDeviceProperties(&prop, im3d_ctx_device(ctx)));
-    g_num_sms = prop.multiProcessorCount;
+    UN_CUDA(cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev));
+    // the context keeps the packed filter and the error flag (an allocation, a release and a
+    // query of every device property per call took 3 ms, the convolution 50 us)
+    void*& ws = im3d_ctx_conv_workspace(ctx);
+    if (!ws) UN_CUDA(cudaMalloc(&ws, 256 + (size_t)27 * 64 * 64 * 2));
+    int* errf = static_cast<int*>(ws);
+    bf16_t* wpk = reinterpret_cast<bf16_t*>(static_cast<char*>(ws) + 256);
+    // a caller's tensors may still be on their way on the default stream, which the context's
+    // own stream does not wait for
+    UN_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
+    UN_CUDA(cudaMemsetAsync(errf, 0, sizeof(int), st));
     const int nout = nout_for(cout);
-    bf16_t* wpk = nullptr;
-    int* errf = nullptr;
-    UN_CUDA(cudaMalloc(&wpk, (size_t)27 * cin * cout * 2));
-    if (cudaMalloc(&errf, sizeof(int)) != cudaSuccess) {
-        cudaFree(wpk);
-        err = "cudaMalloc failed";
-        return IM3D_ERR_OOM;
-    }
-    cudaMemsetAsync(errf, 0, sizeof(int), st);
     PackJobs jobs;
     jobs.job[0] = PackJob{w, wpk, cout, cin, nout, 0};
     pack_filter_kernel<<<flat_blocks(27LL * cin * cout), 256, 0, st>>>(jobs);
-    int s = launch_status(err, "pack_filter");
+    UN_TRY(launch_status(err, "pack_filter"));
     const View v{reinterpret_cast<const bf16_t*>(x), c_pitch, nx, ny, nz, nsamp};
-    if (s == IM3D_OK)
-        s = conv_any<CONV_BIAS_F32>(st, cin, nout, v, c_off, wpk, cout / nout, bias, out, cout, 0, nullptr, 0, 0,
-                                    errf, err);
+    UN_TRY(conv_any<CONV_BIAS_F32>(st, cin, nout, v, c_off, wpk, cout / nout, bias, out, cout, 0, nullptr, 0, 0, errf,
+                                   err));
     int h = 0;
-    if (s == IM3D_OK && cudaMemcpyAsync(&h, errf, sizeof(int), cudaMemcpyDeviceToHost, st) == cudaSuccess &&
-        cudaStreamSynchronize(st) == cudaSuccess && h) {
+    UN_CUDA(cudaMemcpyAsync(&h, errf, sizeof(int), cudaMemcpyDeviceToHost, st));
+    UN_CUDA(cudaStreamSynchronize(st));
+    if (h) {
         err = "conv3d: a wait gave up";
-        s = IM3D_ERR_CUDA;
+        return IM3D_ERR_CUDA;
     }
-    cudaStreamSynchronize(st);
-    cudaFree(wpk);
-    cudaFree(errf);
-    return s;
+    return IM3D_OK;
 }
 
 }  // extern "C"
