@@ -1149,33 +1149,40 @@ int cc_run(im3d_ctx* ctx, const T* img, T* res, const Dims& d, const T* init, in
         IM3D_TRY(sync(ctx));
         negative = v < pivot;  // a dark seed: the component of the negative image (:1740-1745)
     }
-    unsigned char* m0 = nullptr;
-    unsigned char* m1 = nullptr;
-    IM3D_TRY(tbuf<unsigned char>(ctx, "cc_mask0", (size_t)n, &m0));
-    IM3D_TRY(tbuf<unsigned char>(ctx, "cc_mask1", (size_t)n, &m1));
-    cc_init_kernel<T><<<flat_grid(n), 256, 0, ctx->stream>>>(img, init, m0, n, pivot, negative, seed);
+    CcDims c;
+    c.plane_rule = d.nz != 1;
+    c.na = d.nz == 1 ? 1 : d.nx;
+    c.nb = d.nz == 1 ? d.nx : d.ny;
+    c.nk = d.nz == 1 ? d.ny : d.nz;
+    c.words = (c.nk + 31) / 32;
+    const long long words = (long long)c.na * c.nb * c.words;
+    unsigned *white = nullptr, *comp = nullptr;
+    IM3D_TRY(tbuf<unsigned>(ctx, "cc_white", (size_t)words, &white));
+    IM3D_TRY(tbuf<unsigned>(ctx, "cc_comp", (size_t)words, &comp));
+    const int fgrid = flat_grid(words * 8);  // a warp per 4 words
+    cc_init_kernel<T><<<fgrid, 256, 0, ctx->stream>>>(img, init, white, comp, c, pivot, negative, seed);
     IM3D_TRY(check_launch(ctx, "cc_init"));
-    const dim3 grid((d.nz + kCcK - 1) / kCcK, (d.ny + kCcJ - 1) / kCcJ, (d.nx + kCcI - 1) / kCcI);
-    const dim3 blk(kCcK, kCcJ);
+    const dim3 grid((c.words + kCcW - 1) / kCcW, (c.nb + kCcB - 1) / kCcB, (c.na + kCcA - 1) / kCcA);
+    const dim3 blk(kCcW * kCcB * kCcA);
     unsigned long long* flag = ctx->ctrl_d->umax + 2;
     long long np = 0;
     for (;;) {
         IM3D_CUDA(ctx, cudaMemsetAsync(flag, 0, sizeof(unsigned long long), ctx->stream));
-        for (int r = 0; r < 4; ++r) {
+        constexpr int R = 4;  // passes per read of the flag, whose bit r tells that pass r grew
+        for (int r = 0; r < R; ++r) {
             const int pf = prof_begin(ctx, "cc_grow");
-            if (full) cc_grow_kernel<true><<<grid, blk, 0, ctx->stream>>>(m0, m1, d, flag);
-            else cc_grow_kernel<false><<<grid, blk, 0, ctx->stream>>>(m0, m1, d, flag);
+            if (full) cc_grow_kernel<true><<<grid, blk, 0, ctx->stream>>>(white, comp, c, flag, 1ull << r);
+            else cc_grow_kernel<false><<<grid, blk, 0, ctx->stream>>>(white, comp, c, flag, 1ull << r);
             prof_end(ctx, pf);
             IM3D_TRY(check_launch(ctx, "cc_grow"));
-            std::swap(m0, m1);
             ++np;
         }
         IM3D_TRY(read_ctrl(ctx));
-        if (ctx->ctrl_h->umax[2] == 0) break;
+        if ((ctx->ctrl_h->umax[2] >> (R - 1) & 1) == 0) break;
         // every pass that does not end the loop adds a cell
         if (np > n + 8) return fail(ctx, IM3D_ERR_CUDA, "connected_component: no fixed point");
     }
-    cc_output_kernel<T><<<flat_grid(n), 256, 0, ctx->stream>>>(m0, img, res, n, binary, mn, pivot);
+    cc_output_kernel<T><<<fgrid, 256, 0, ctx->stream>>>(comp, img, res, c, binary, mn, pivot);
     IM3D_TRY(check_launch(ctx, "cc_output"));
     if (passes) *passes = (int)(np < 0x7fffffff ? np : 0x7fffffff);
     return IM3D_OK;
