@@ -80,6 +80,8 @@ struct im3d_ctx {
     int batch_mode = IM3D_BATCH_AUTO;
     int tile_loads = 1;  // the FP32 Heaviside pass moves its rows with TMA where it can
     int num_sms = 148;
+    signed char cluster_ok[8] = {};  // rb_cluster_kernel per type and rule: 0 not asked, 1 can run, -1 cannot
+    size_t smem_optin = 0;           // shared memory a block may ask for
     int lex_key[4] = {0, 0, 0, 0};  // tile counts and sweeps of the lexicographic task list held in "lex_tasks"
     int ifit_chunks = 0;  // i chunks of the marching fit stage (0: cost model)
     size_t mem_limit = 0;  // device bytes the context may hold in buffers (0: no limit)
@@ -970,6 +972,86 @@ int rb_sweep(im3d_ctx* ctx, T* U, const T* B, const Dims& d, const GsCoef<T>& c,
     return IM3D_OK;
 }
 
+// Whether rb_cluster_kernel can run with `smem` bytes per block: the device can hold such a
+// cluster (asked once per context, type and boundary rule).
+template <typename T, int BC, bool P2>
+bool rb_cluster_kernel_ready(im3d_ctx* ctx, size_t smem)
+{
+    auto kern = rb_cluster_kernel<T, BC, P2>;
+    signed char& known = ctx->cluster_ok[(sizeof(T) == 8) * 4 + BC * 2 + P2];
+    if (known == 0) {
+        known = -1;
+        int optin = 0;
+        if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device) == cudaSuccess &&
+            cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, optin) == cudaSuccess) {
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(kRbCluster);
+            cfg.blockDim = dim3(kRbClThreads);
+            cfg.dynamicSmemBytes = (size_t)optin;
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeClusterDimension;
+            at[0].val.clusterDim.x = kRbCluster;
+            at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+            cfg.attrs = at;
+            cfg.numAttrs = 1;
+            int clusters = 0;
+            if (cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) == cudaSuccess && clusters > 0) {
+                known = 1;
+                ctx->smem_optin = (size_t)optin;
+            }
+        }
+        cudaGetLastError();
+    }
+    return known > 0 && smem <= ctx->smem_optin;
+}
+
+template <typename T, int BC, bool P2>
+int rb_cluster_launch(im3d_ctx* ctx, T* U, const T* B, const Dims& d, const GsCoef<T>& c, int sweeps)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kRbCluster);
+    cfg.blockDim = dim3(kRbClThreads);
+    cfg.dynamicSmemBytes = rb_cluster_smem<T>(d);
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = kRbCluster;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    const int pf = prof_begin(ctx, "rb_cluster");
+    IM3D_CUDA(ctx, cudaLaunchKernelEx(&cfg, rb_cluster_kernel<T, BC, P2>, U, B, d, c, sweeps));
+    prof_end(ctx, pf);
+    return check_launch(ctx, "rb_cluster");
+}
+
+// `sweeps` sweeps of the residual solve on b_eff. first: see rb_sweep.
+template <typename T>
+int rb_sweeps(im3d_ctx* ctx, T* U, const T* B, const Dims& d, const GsCoef<T>& c, double omega, int sweeps, int first)
+{
+    // up to 2304 vector groups per block and colour: 64^3 FP32 (1984) takes 1.64 us per
+    // half-sweep, 66^3 (2880) 2.55, a launch per half-sweep 2.44
+    const size_t smem = rb_cluster_smem<T>(d);
+    const int lo = c.neu ? 0 : 1;
+    const long long groups =
+        (long long)((d.nx + kRbCluster - 1) / kRbCluster) * (d.ny - 2 * lo) * (d.hz() / V16<T>::W);
+    if (omega == 1.0 && !(c.neu && c.bc != T(0)) && groups <= 2304 && smem <= 227 * 1024) {
+        const bool p2 = sizeof(T) == 8 && (c.pow2 & 7) == 7;
+        if (c.neu) {
+            if (p2 ? rb_cluster_kernel_ready<T, RB_NEU0, true>(ctx, smem) : rb_cluster_kernel_ready<T, RB_NEU0, false>(ctx, smem))
+                return p2 ? rb_cluster_launch<T, RB_NEU0, true>(ctx, U, B, d, c, sweeps)
+                          : rb_cluster_launch<T, RB_NEU0, false>(ctx, U, B, d, c, sweeps);
+        } else {
+            if (p2 ? rb_cluster_kernel_ready<T, RB_DIR, true>(ctx, smem) : rb_cluster_kernel_ready<T, RB_DIR, false>(ctx, smem))
+                return p2 ? rb_cluster_launch<T, RB_DIR, true>(ctx, U, B, d, c, sweeps)
+                          : rb_cluster_launch<T, RB_DIR, false>(ctx, U, B, d, c, sweeps);
+        }
+    }
+    for (int s = 0; s < sweeps; ++s) IM3D_TRY(rb_sweep(ctx, U, B, d, c, 0, omega, first && s == 0));
+    return IM3D_OK;
+}
+
 // Per-block partial sums of a reduction launch (nvals values per block).
 int part_buf(im3d_ctx* ctx, dim3 grid, int nvals, double** out)
 {
@@ -1067,8 +1149,9 @@ int rb_solve(im3d_ctx* ctx, T* U, const T* B, const Dims& d, const GsCoef<T>& c,
     *conv = false;
     *rel = -1;
     while (s < max_sweeps) {
-        IM3D_TRY(rb_sweep(ctx, U, B, d, c, 0, omega, s == 0));
-        ++s;
+        const int k = std::max(1, std::min(next, max_sweeps) - s);
+        IM3D_TRY(rb_sweeps(ctx, U, B, d, c, omega, k, s == 0));
+        s += k;
         if (s >= next || s == max_sweeps) {
             double r = 0;
             IM3D_TRY(rb_check<T>(ctx, U, B, d, c, &beff2, &r));
