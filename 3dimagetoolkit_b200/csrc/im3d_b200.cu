@@ -446,8 +446,16 @@ template <typename T, int N, class Ld, class St>
 int pass_k(im3d_ctx* ctx, Ld ld, St st, const Dims& d, const T* w, int nh,
            const char* name = "conv_k")
 {
+    // register windows for the supports of sigma 1 .. 4 at unit and 1.5 spacing; other
+    // supports run the loop over taps in shared memory (us at 171x203x117: 13 taps, four
+    // fields 62 -> 41, two 58 -> 35)
     if (nh == 19) return pass_k_win<T, N, 9>(ctx, ld, st, d, w, name);
     if (nh == 25) return pass_k_win<T, N, 12>(ctx, ld, st, d, w, name);
+    if (nh == 13) return pass_k_win<T, N, 6>(ctx, ld, st, d, w, name);
+    if (nh == 17) return pass_k_win<T, N, 8>(ctx, ld, st, d, w, name);
+    if (nh == 9) return pass_k_win<T, N, 4>(ctx, ld, st, d, w, name);
+    if constexpr (N == 1)
+        if (nh == 7) return pass_k_win<T, N, 3>(ctx, ld, st, d, w, name);
     const int S = nh / 2;
     size_t smem = (size_t)RK * (TK + 2 * S) * sizeof(Vec<T, N>) + nh * sizeof(T) + 16;
     auto kern = conv_k_kernel<T, N, TK, RK, Ld, St>;
@@ -586,6 +594,9 @@ int pass_s(im3d_ctx* ctx, Ld ld, St st, const Dims& d, const T* w, int nh,
 {
     if (nh == 19) return pass_s_win<T, N, AXIS, 9>(ctx, ld, st, d, w, name);
     if (nh == 25) return pass_s_win<T, N, AXIS, 12>(ctx, ld, st, d, w, name);
+    if (nh == 13) return pass_s_win<T, N, AXIS, 6>(ctx, ld, st, d, w, name);
+    if constexpr (N == 1)
+        if (nh == 7) return pass_s_win<T, N, AXIS, 3>(ctx, ld, st, d, w, name);
     constexpr int TA = TileA<T>::v;
     const int S = nh / 2;
     size_t smem = (size_t)(TA + 2 * S) * TW * sizeof(Vec<T, N>) + nh * sizeof(T) + 16;
@@ -696,9 +707,12 @@ int pass_i_fit(im3d_ctx* ctx, const Vec<T, 4>* in, Vec<T, 2>* out, T* f1, T* f2,
     if constexpr (sizeof(T) == 4) {
         if (nh == 19) return pass_i_fit_march<9>(ctx, in, out, f1, f2, d, hw, l1, l2);
         if (nh == 25) return pass_i_fit_march<12>(ctx, in, out, f1, f2, d, hw, l1, l2);
+        if (nh == 13) return pass_i_fit_march<6>(ctx, in, out, f1, f2, d, hw, l1, l2);
     }
     if (nh == 19) return pass_i_fit_win<T, 9>(ctx, in, out, f1, f2, d, w, l1, l2);
     if (nh == 25) return pass_i_fit_win<T, 12>(ctx, in, out, f1, f2, d, w, l1, l2);
+    if constexpr (sizeof(T) == 8)
+        if (nh == 13) return pass_i_fit_win<T, 6>(ctx, in, out, f1, f2, d, w, l1, l2);
     constexpr int TA = TileA<T>::v;
     const int S = nh / 2;
     size_t smem = (size_t)(TA + 4 * S) * TW * sizeof(Vec<T, 4>) +

@@ -882,8 +882,9 @@ __device__ __forceinline__ void conv_i_fit_march_body(const uint3 blockIdx, cons
                     const bool inside = m >= 0 && m < d.nx;
                     float pv = 0.f, qv = 0.f;
                     if (col && (inside || d.cyc)) {
-                        const float f1 = __fdividef(a0[0].x, a0[0].y);
-                        const float f2 = __fdividef(a1[0].x, a1[0].y);
+                        // (13 taps keep the division of the kernel they used to run on)
+                        const float f1 = S == 6 ? a0[0].x / a0[0].y : __fdividef(a0[0].x, a0[0].y);
+                        const float f2 = S == 6 ? a1[0].x / a1[0].y : __fdividef(a1[0].x, a1[0].y);
                         pv = f1 * l1 - f2 * l2;
                         qv = (f1 * f1) * l1 - (f2 * f2) * l2;
                         if (f1_out && inside && m >= i0 && m < i1) {
