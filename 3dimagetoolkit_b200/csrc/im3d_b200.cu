@@ -869,7 +869,7 @@ int check_flags(im3d_ctx* ctx)
 
 constexpr int kNI = 8;  // planes per thread of the scalar column-marching kernels
 constexpr int kNV = 2;  // planes per thread of the vectorised kernels (measured best on B200)
-constexpr int kNVres = 2;  // planes per thread of the residual check
+constexpr int kNVres = 4;  // most planes per thread of the residual check
 const dim3 kBlkVec(32, 4, 1);
 
 // half-sweep and residual grid: the (vector group, row) pairs of a plane flattened over
@@ -880,6 +880,15 @@ dim3 grid_rb_flat(const Dims& d, dim3 blk, int zmul = 1, int ni = kNV)
     const long long pairs = (long long)(d.hz() / V16<T>::W) * d.ny;
     const long long per = (long long)blk.x * blk.y;
     return dim3((unsigned)((pairs + per - 1) / per), 1, ((d.nx + ni - 1) / ni) * zmul);
+}
+
+// planes per thread of the residual check: 4 on large grids, 2 where 4 leave fewer than 16
+// blocks per SM (us with 2 and 4: 171x203x117 27 / 31, 256^3 50 / 47.5, 512x512x320 227 / 202)
+template <typename T>
+int res_planes(const Dims& d)
+{
+    const dim3 g = grid_rb_flat<T>(d, kBlkVec, 2, kNVres);
+    return (long long)g.x * g.z >= 16 * 148 ? kNVres : 2;
 }
 
 // natural-layout vectorised kernels: (vector group, row) pairs flattened over x blocks
@@ -1123,16 +1132,21 @@ template <typename T>
 int rb_check(im3d_ctx* ctx, const T* U, const T* B, const Dims& d, const GsCoef<T>& c,
              double* beff2, double* rel)
 {
-    const dim3 grid = grid_rb_flat<T>(d, kBlkVec, 2, kNVres);
+    const int ni = res_planes<T>(d);
+    const dim3 grid = grid_rb_flat<T>(d, kBlkVec, 2, ni);
     const int nvals = *beff2 < 0 ? 2 : 1;
     double* part = nullptr;
     IM3D_TRY(part_buf(ctx, grid, nvals, &part));
     ctx->residual_checks++;
     const int pf = prof_begin(ctx, "rb_residual");
-    if (fits_int32(d))
-        rb_residual_vec_kernel<T, kNVres, int><<<grid, kBlkVec, 0, ctx->stream>>>(U, B, d, c, part, nvals == 2 ? 1 : 0);
-    else
-        rb_residual_vec_kernel<T, kNVres><<<grid, kBlkVec, 0, ctx->stream>>>(U, B, d, c, part, nvals == 2 ? 1 : 0);
+    const int wb = nvals == 2 ? 1 : 0;
+    if (fits_int32(d)) {
+        if (c.neu) rb_residual_vec_kernel<T, kNVres, true, int><<<grid, kBlkVec, 0, ctx->stream>>>(U, B, d, c, part, wb, ni);
+        else rb_residual_vec_kernel<T, kNVres, false, int><<<grid, kBlkVec, 0, ctx->stream>>>(U, B, d, c, part, wb, ni);
+    } else {
+        if (c.neu) rb_residual_vec_kernel<T, kNVres, true, long long><<<grid, kBlkVec, 0, ctx->stream>>>(U, B, d, c, part, wb, ni);
+        else rb_residual_vec_kernel<T, kNVres, false, long long><<<grid, kBlkVec, 0, ctx->stream>>>(U, B, d, c, part, wb, ni);
+    }
     prof_end(ctx, pf);
     IM3D_TRY(check_launch(ctx, "rb_residual"));
     IM3D_TRY(finalize(ctx, part, grid, nvals, SUM_RES2));
@@ -2457,7 +2471,7 @@ int worklist_group(im3d_ctx* ctx, const std::vector<int>& ids, const im3d_volume
                                  dsc.nx, dsc.ny, dsc.nz, dsc.hx, dsc.hy, dsc.hz, p, nullptr, nullptr,
                                  nullptr, nullptr, nullptr);
         const Dims& d = V[q].d;
-        const dim3 gr = grid_rb_flat<T>(d, kBlkVec, 2, kNVres);
+        const dim3 gr = grid_rb_flat<T>(d, kBlkVec, 2, res_planes<T>(d));
         const bool vec = d.nz % V16<T>::W == 0;
         const dim3 gc = vec ? grid_vec<T>(d, kBlkVec) : grid_col(d, kBlkVol);
         if (st == IM3D_OK)
@@ -2539,8 +2553,9 @@ int worklist_group(im3d_ctx* ctx, const std::vector<int>& ids, const im3d_volume
             jrd[c].h.push_back({RbD{v.upk, v.bpk, d, v.coef, c, c}, gpk});
             jrn[c].h.push_back({RbN{v.upk, v.bpk, d, v.coef, c, c}, gpk});
         }
-        const dim3 gr = grid_rb_flat<T>(d, kBlkVec, 2, kNVres);
-        jres.h.push_back({Res{v.upk, v.bpk, d, v.coef, part_res[q]}, gr});
+        const int ni = res_planes<T>(d);
+        const dim3 gr = grid_rb_flat<T>(d, kBlkVec, 2, ni);
+        jres.h.push_back({Res{v.upk, v.bpk, d, v.coef, part_res[q], ni}, gr});
         fin_res[q] = FinalizeJob{part_res[q], (long long)gr.x * gr.y * gr.z, ctrl[q].sum};
         vecrow[q] = d.nz % V16<T>::W == 0;
         const dim3 gv = grid_vec<T>(d, kBlkVec), gcol = grid_col(d, kBlkVol), gvol = grid_vol(d, kBlkVol);
@@ -2687,7 +2702,7 @@ int worklist_group(im3d_ctx* ctx, const std::vector<int>& ids, const im3d_volume
                         flags.push_back(C[q].beff2 < 0 ? 1 : 0);
                     }
                 }
-                IM3D_TRY((wl_launch<Res, 256, 4>(sc, jres, due, flags.data(), kBlkVec, 0, "rb_residual")));
+                IM3D_TRY((wl_launch<Res, 128, 6>(sc, jres, due, flags.data(), kBlkVec, 0, "rb_residual")));
                 IM3D_TRY(wl_finalize(sc, fin_res_d, due, flags.data(), 1, SUM_RES2));
                 IM3D_CUDA(sc, cudaMemcpyAsync(ctx->wl_ctrl_h + q0, ctrl + q0, (q1 - q0) * sizeof(Ctrl),
                                               cudaMemcpyDeviceToHost, sc->stream));

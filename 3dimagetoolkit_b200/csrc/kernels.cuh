@@ -1367,36 +1367,6 @@ __global__ void dir_faces_kernel(T* r, Dims d, T bc)
         r[d.idx(i, j, k)] = bc;
 }
 
-// FP64 residual of one unknown of (1/dt - Lap) u = b_eff:
-//   r = sum of neighbour terms + b_eff - diag * u,  diag = 1/dt + sum_a c_a/h_a^2
-// with c_a = 2 inside and 1 on a Neumann face (the same rows the sweep solves).
-template <typename T, class R>
-__device__ __forceinline__ double gs_residual_fp64(const GsCoef<T>& c, const Dims& d, int i,
-                                                   int j, int k, double b, double u, R r)
-{
-    if (!c.neu) {
-        const double sx = r(1, 0, 0) + r(-1, 0, 0);
-        const double sy = r(0, 1, 0) + r(0, -1, 0);
-        const double sz = r(0, 0, 1) + r(0, 0, -1);
-        return sx * c.ihx2d + sy * c.ihy2d + sz * c.ihz2d + b - c.diagd * u;
-    }
-    const int cx = i == 0 ? 0 : (i == d.nx - 1 ? 2 : 1);
-    const int cy = j == 0 ? 0 : (j == d.ny - 1 ? 2 : 1);
-    const int cz = k == 0 ? 0 : (k == d.nz - 1 ? 2 : 1);
-    const int nb = (cx != 1) + (cy != 1) + (cz != 1);
-    const double bcn = c.bcnd[nb];
-    const double tx = cx == 1 ? r(1, 0, 0) + r(-1, 0, 0)
-                              : (cx == 0 ? r(1, 0, 0) - bcn * c.hx : r(-1, 0, 0) + bcn * c.hx);
-    const double ty = cy == 1 ? r(0, 1, 0) + r(0, -1, 0)
-                              : (cy == 0 ? r(0, 1, 0) - bcn * c.hy : r(0, -1, 0) + bcn * c.hy);
-    const double tz = cz == 1 ? r(0, 0, 1) + r(0, 0, -1)
-                              : (cz == 0 ? r(0, 0, 1) - bcn * c.hz : r(0, 0, -1) + bcn * c.hz);
-    const double diag = 1.0 / c.dt + (cx == 1 ? 2.0 : 1.0) * c.ihx2d + (cy == 1 ? 2.0 : 1.0) * c.ihy2d +
-                        (cz == 1 ? 2.0 : 1.0) * c.ihz2d;
-    return tx * c.ihx2d + ty * c.ihy2d + tz * c.ihz2d + b - diag * u;
-}
-
-
 // The (vector group g, row j) pairs of a block of planes, flattened over the grid's x
 // blocks, so that no lane idles when a row's `groups` are not a multiple of blockDim.x
 // (40 groups at nz = 320 left 24 of every 64 lanes idle). A power-of-two number of
@@ -1920,92 +1890,130 @@ __global__ void __launch_bounds__(kRbClThreads, 1) rb_cluster_kernel(T* __restri
             reinterpret_cast<VV*>(U + col * npk + (long long)i0 * cells)[q] = reinterpret_cast<const VV*>(su[col])[q + vecs];
 }
 
-// Vectorised FP64 residual, same walk as rb_half_vec_kernel; blockIdx.z covers
-// (plane block, colour).
-template <typename T, int NI, typename IX = long long>
-__device__ __forceinline__ void rb_residual_vec_body(const uint3 blockIdx, const dim3 gridDim, const T* __restrict__ U, const T* __restrict__ B, Dims d, GsCoef<T> c, double* part, int want_beff)
+// FP64 residual of (1/dt - Lap) u = b_eff over the unknowns, and sum b_eff^2 when want_beff;
+// blockIdx.z covers (plane block, colour). The walk of rb_march_kernel: a thread takes a group
+// of W packed cells over ni <= NI planes of i, every cell by the interior formula
+//   r = sum of neighbour terms + b_eff - diag * u,  diag = 1/dt + sum_a c_a / h_a^2,
+// with c_a = 2 inside; on a Neumann face the missing neighbour is the ghost value of
+// rb_group and c_a = 1, and cells that are no unknowns (Dirichlet faces, padding) count 0.
+// What bounds it: conversions to FP64 (about 5 per cell; a value is converted once and kept
+// for the planes that read it) and the reads. us against per-cell face tests with a generic
+// boundary path (88 instructions per cell): 256^3 66 -> 49, 512x512x320 300 -> 214, 171x203x117
+// Neumann 38 -> 30 (6 blocks of 128 threads per SM; unlimited and 8 measured slower).
+template <typename T, int NI, bool NEU, typename IX = long long>
+__device__ __forceinline__ void rb_residual_vec_body(const uint3 blockIdx, const dim3 gridDim, const T* __restrict__ U, const T* __restrict__ B, const Dims& d, const GsCoef<T>& c, double* part, int want_beff, int ni)
 {
     typedef V16<T> VT;
     typedef typename VT::type VV;
     constexpr int W = VT::W;
+    constexpr int lo = NEU ? 0 : 1;
     int g, j;
-    flat_pair(blockIdx, (unsigned)(d.hz() / W), g, j);
-    const int color = blockIdx.z & 1;
-    const int i0 = (blockIdx.z >> 1) * NI;
     const int hz = d.hz();
+    flat_pair(blockIdx, (unsigned)(hz / W), g, j);
+    const int color = blockIdx.z & 1;
+    const int ib = (int)(blockIdx.z >> 1) * ni;
+    const int i0 = ib < lo ? lo : ib, i1 = min(ib + ni, d.nx - lo);
     const int m0 = g * W;
     double acc = 0, accb = 0;
-    if (m0 < hz && j < d.ny) {
+    if (j >= lo && j < d.ny - lo && i0 < i1) {
         const IX plane = (IX)d.ny * hz;
         const IX npk = plane * d.nx;
-        const T* own = U + (color ? npk : 0);
-        const T* oth = U + (color ? 0 : npk);
-        const T* bb = B + (color ? npk : 0);
-        const bool jint = j >= 1 && j <= d.ny - 2;
-        const int lo = c.neu ? 0 : 1;
         const IX q0 = ((IX)i0 * d.ny + j) * hz + m0;
-        VV o[NI + 2];
+        const T* po = U + (color ? 0 : npk) + q0;
+        const T* pu = U + (color ? npk : 0) + q0;
+        const T* pb = B + (color ? npk : 0) + q0;
+        const int cy = j == 0 ? 0 : (j == d.ny - 1 ? 2 : 1);
+        const bool has_ym = !NEU || cy != 0, has_yp = !NEU || cy != 2;
+        int par = (i0 + j + color) & 1;
+        VV ymn = VV{}, ypn = VV{}, bn, un;
+        T en = T(0);
+        auto side = [&](const T* p, int pr) {
+            if (has_ym) ymn = *reinterpret_cast<const VV*>(p - hz);
+            if (has_yp) ypn = *reinterpret_cast<const VV*>(p + hz);
+            const bool e_ok = pr ? m0 + W < hz : m0 >= 1;
+            en = e_ok ? p[pr ? W : -1] : T(0);
+        };
+        auto to_d = [](const VV& v, double (&o)[W]) {
 #pragma unroll
-        for (int t = 0; t < NI + 2; ++t) {
-            const int i = i0 - 1 + t;
-            if (i >= 0 && i < d.nx) o[t] = *reinterpret_cast<const VV*>(oth + q0 + (IX)(t - 1) * plane);
-            else o[t] = VV{};
+            for (int cc = 0; cc < W; ++cc) o[cc] = (double)VT::get(v, cc);
+        };
+        double xm[W], xc[W], xp[W];
+        {
+            VV v = VV{};
+            if (!NEU || i0 >= 1) v = *reinterpret_cast<const VV*>(po - plane);
+            to_d(v, xm);
+            to_d(*reinterpret_cast<const VV*>(po), xc);
         }
+        side(po, par);
+        bn = *reinterpret_cast<const VV*>(pb);
+        un = *reinterpret_cast<const VV*>(pu);
 #pragma unroll
         for (int t = 0; t < NI; ++t) {
             const int i = i0 + t;
-            if (i >= d.nx) break;
-            const IX q = q0 + (IX)t * plane;
-            const int par = (i + j + color) & 1;
-            const bool rowint = jint && i >= 1 && i <= d.nx - 2;
-            const VV bv = *reinterpret_cast<const VV*>(bb + q);
-            const VV uv = *reinterpret_cast<const VV*>(own + q);
-            if (rowint) {
-                const VV ym = *reinterpret_cast<const VV*>(oth + q - hz);
-                const VV yp = *reinterpret_cast<const VV*>(oth + q + hz);
-                const IX qe = par ? q + W : q - 1;
-                const bool e_ok = par ? (m0 + W < hz) : (m0 >= 1);
-                const double extra = e_ok ? (double)oth[qe] : 0.0;
+            if (i >= i1) break;
+            const VV ym = ymn, yp = ypn, bv = bn, uv = un;
+            const double extra = (double)en;
+            VV xv = VV{};
+            if (!NEU || i + 1 < d.nx) xv = *reinterpret_cast<const VV*>(po + plane);
+            if (t + 1 < NI && i + 1 < i1) {
+                side(po + plane, par ^ 1);
+                pb += plane;
+                pu += plane;
+                bn = *reinterpret_cast<const VV*>(pb);
+                un = *reinterpret_cast<const VV*>(pu);
+            }
+            to_d(xv, xp);
+            const int last = ((d.nz - 1 - par) >> 1) - m0;    // the last cell with k < nz
+            const bool last_k = ((d.nz - 1 - par) & 1) == 0;  // ... and whether its k is nz - 1
+            const int cx = NEU ? (i == 0 ? 0 : (i == d.nx - 1 ? 2 : 1)) : 1;
 #pragma unroll
-                for (int cc = 0; cc < W; ++cc) {
-                    const int k = 2 * (m0 + cc) + par;
-                    if (!(k >= 1 && k <= d.nz - 2)) continue;
-                    const double ctr = (double)VT::get(o[t + 1], cc);
-                    const double kn = par ? (cc + 1 < W ? (double)VT::get(o[t + 1], cc + 1) : extra)
-                                          : (cc >= 1 ? (double)VT::get(o[t + 1], cc - 1) : extra);
-                    const double b = (double)VT::get(bv, cc);
-                    const double r = ((double)VT::get(o[t], cc) + (double)VT::get(o[t + 2], cc)) * c.ihx2d +
-                                     ((double)VT::get(ym, cc) + (double)VT::get(yp, cc)) * c.ihy2d +
-                                     (ctr + kn) * c.ihz2d + b - c.diagd * (double)VT::get(uv, cc);
-                    acc += r * r;
-                    accb += b * b;
+            for (int cc = 0; cc < W; ++cc) {
+                const bool at0 = cc == 0 && par == 0 && m0 == 0, at1 = last_k && cc == last;
+                double sx = xm[cc] + xp[cc];
+                double sy = (double)VT::get(ym, cc) + (double)VT::get(yp, cc);
+                double zn = par ? (cc + 1 < W ? xc[cc + 1] : extra) : (cc >= 1 ? xc[cc - 1] : extra);
+                double zc = xc[cc];
+                double diag = c.diagd;
+                if (NEU) {
+                    // a missing neighbour was read as 0 (past the row: replaced here)
+                    if (at1) {
+                        if (par) zn = 0;
+                        else zc = 0;
+                    }
+                    if (at0 || at1 || cx != 1 || cy != 1) {
+                        const double bcn = c.bcnd[(cx != 1) + (cy != 1) + (at0 || at1)];
+                        if (cx != 1) sx += cx == 0 ? -(bcn * c.hx) : bcn * c.hx;
+                        if (cy != 1) sy += cy == 0 ? -(bcn * c.hy) : bcn * c.hy;
+                        if (at0) zn += -(bcn * c.hz);
+                        if (at1) zn += bcn * c.hz;
+                        diag = 1.0 / c.dt + (cx == 1 ? 2.0 : 1.0) * c.ihx2d + (cy == 1 ? 2.0 : 1.0) * c.ihy2d +
+                               (at0 || at1 ? 1.0 : 2.0) * c.ihz2d;
+                    }
                 }
+                const double b = (double)VT::get(bv, cc);
+                double r = sx * c.ihx2d + sy * c.ihy2d + (zc + zn) * c.ihz2d + b - diag * (double)VT::get(uv, cc);
+                const bool unknown = cc <= last && (NEU || !(at0 || at1));
+                r = unknown ? r : 0.0;
+                acc += r * r;
+                if (want_beff) accb += unknown ? b * b : 0.0;
             }
 #pragma unroll
             for (int cc = 0; cc < W; ++cc) {
-                const int k = 2 * (m0 + cc) + par;
-                if (k >= d.nz) continue;
-                if (rowint && k >= 1 && k <= d.nz - 2) continue;
-                if (!(i >= lo && j >= lo && k >= lo && i < d.nx - lo && j < d.ny - lo && k < d.nz - lo))
-                    continue;
-                auto rd = [&](int oi, int oj, int ok) {
-                    return (double)oth[d.pidx(i + oi, j + oj, k + ok)];
-                };
-                const double b = (double)VT::get(bv, cc);
-                const double r = gs_residual_fp64<T>(c, d, i, j, k, b, (double)VT::get(uv, cc), rd);
-                acc += r * r;
-                accb += b * b;
+                xm[cc] = xc[cc];
+                xc[cc] = xp[cc];
             }
+            po += plane;
+            par ^= 1;
         }
     }
     if (want_beff) block_sum2_store(acc, accb, part, block_linear_id(blockIdx, gridDim), grid_blocks(gridDim));
     else block_sum_store(acc, part, block_linear_id(blockIdx, gridDim));
 }
 
-template <typename T, int NI, typename IX = long long>
-__global__ void __launch_bounds__(256, 4) rb_residual_vec_kernel(const T* __restrict__ U, const T* __restrict__ B, Dims d, GsCoef<T> c, double* part, int want_beff)
+template <typename T, int NI, bool NEU, typename IX>
+__global__ void __launch_bounds__(128, 6) rb_residual_vec_kernel(const T* __restrict__ U, const T* __restrict__ B, Dims d, GsCoef<T> c, double* part, int want_beff, int ni)
 {
-    rb_residual_vec_body<T, NI, IX>(blockIdx, gridDim, U, B, d, c, part, want_beff);
+    rb_residual_vec_body<T, NI, NEU, IX>(blockIdx, gridDim, U, B, d, c, part, want_beff, ni);
 }
 
 

@@ -143,9 +143,11 @@ struct RbResidualJob {
     Dims d;
     GsCoef<T> c;
     double* part;
+    int ni;
     __device__ __forceinline__ void operator()(uint3 b, dim3 g, int flag) const
     {
-        rb_residual_vec_body<T, NI>(b, g, U, B, d, c, part, flag);
+        if (c.neu) rb_residual_vec_body<T, NI, true>(b, g, U, B, d, c, part, flag, ni);
+        else rb_residual_vec_body<T, NI, false>(b, g, U, B, d, c, part, flag, ni);
     }
 };
 
