@@ -781,6 +781,22 @@ GsCoef<T> make_coef(double hx, double hy, double hz, double dt, double bc, int n
     return c;
 }
 
+template <typename T>
+HStep<T> make_hstep(double hx, double hy, double hz)
+{
+    HStep<T> s;
+    s.pow2 = 0;
+    const double h[3] = {hx, hy, hz};
+    for (int a = 0; a < 3; ++a) {
+        int e = 0;
+        s.h[a] = (T)h[a];
+        s.two[a] = (T)(2. * h[a]);
+        s.inv[a] = (T)(1. / (2. * h[a]));
+        if (std::frexp(2. * h[a], &e) == 0.5 && e > -1000 && e < 1000) s.pow2 |= 1 << a;
+    }
+    return s;
+}
+
 // Lexicographic sweeps, reference order, natural layout, in place (lex_tile_kernel). The
 // task list depends on the tile counts and the number of sweeps only; the context keeps the
 // last one. A wait that gave up raises ctrl flag 1.
@@ -905,8 +921,8 @@ dim3 grid_col(const Dims& d, dim3 blk, int ni = kNI)
     return dim3((d.nz + blk.x - 1) / blk.x, (d.ny + blk.y - 1) / blk.y, (d.nx + ni - 1) / ni);
 }
 
-// planes per thread of the column Bregman kernel (it holds every load of its planes)
-constexpr int kNIbr = 2;
+// planes per thread of the column Bregman and div kernels (they hold every load of their planes)
+constexpr int kNIbr = 2, kNIdv = 2;
 
 // Launch as a programmatic dependent of the previous kernel on the stream: the kernel
 // must begin with griddepcontrol.wait (rb_half_vec_kernel does), which holds it until
@@ -1600,7 +1616,7 @@ int rsfe_prepare(im3d_ctx* ctx, VolState<T>& v, const T* myim_user, const T* ini
             src = blurred;
         }
         edge_kernel<T><<<grid_vol(d, kBlkVol), kBlkVol, 0, ctx->stream>>>(
-            src, g, d, hx, hy, hz, (T)p->beta, (T)p->lamda, (T)p->nu);
+            src, g, d, make_hstep<T>(hx, hy, hz), (T)p->beta, (T)p->lamda, (T)p->nu);
         IM3D_TRY(check_launch(ctx, "edge"));
     }
 
@@ -1699,6 +1715,7 @@ int rsfe_apply(im3d_ctx* ctx, const T* myim_user, const T* init_user, int nx, in
     const T center = vs.center;
     const T inv_eps = vs.inv_eps;
     const double hhh = vs.hhh;
+    const HStep<T> hs = make_hstep<T>(hx, hy, hz);
     const int t0 = vs.t0;
     double tollerance = vs.tollerance;
     int init_variables = vs.init_variables;
@@ -1891,18 +1908,18 @@ int rsfe_apply(im3d_ctx* ctx, const T* myim_user, const T* init_user, int nx, in
             const int pf = prof_begin(ctx, "bregman");
             if (vec)
                 bregman_vec_kernel<T, kNV><<<grid_vec<T>(d, kBlkVec), kBlkVec, 0, ctx->stream>>>(
-                    phi_new, b3, dmb, g, d, hx, hy, hz);
+                    phi_new, b3, dmb, g, d, hs);
             else
                 bregman_kernel<T, kNIbr><<<grid_col(d, kBlkVol, kNIbr), kBlkVol, 0, ctx->stream>>>(
-                    phi_new, b3, dmb, g, d, hx, hy, hz);
+                    phi_new, b3, dmb, g, d, hs);
             prof_end(ctx, pf);
             IM3D_TRY(check_launch(ctx, "bregman"));
             const int pf2 = prof_begin(ctx, "div");
             if (vec)
                 div_vec_kernel<T, kNV><<<grid_vec<T>(d, kBlkVec), kBlkVec, 0, ctx->stream>>>(
-                    dmb, divdb, d, hx, hy, hz);
+                    dmb, divdb, d, hs);
             else
-                div_kernel<T><<<grid_vol(d, kBlkVol), kBlkVol, 0, ctx->stream>>>(dmb, divdb, d, hx, hy, hz);
+                div_kernel<T, kNIdv><<<grid_col(d, kBlkVol, kNIdv), kBlkVol, 0, ctx->stream>>>(dmb, divdb, d, hs);
             prof_end(ctx, pf2);
             IM3D_TRY(check_launch(ctx, "div"));
         }
@@ -2004,7 +2021,7 @@ int grad_op(im3d_ctx* ctx, const T* in_user, T* out_user, int nx, int ny, int nz
     T* out = nullptr;
     IM3D_TRY(dev_in<T>(ctx, in_user, d.n(), "in_a", &in));
     IM3D_TRY(dev_out<T>(ctx, out_user, 3 * d.n(), "out_a", &out));
-    grad_kernel<T><<<grid_vol(d, kBlkVol), kBlkVol, 0, ctx->stream>>>(in, out, d, hx, hy, hz);
+    grad_kernel<T><<<grid_vol(d, kBlkVol), kBlkVol, 0, ctx->stream>>>(in, out, d, make_hstep<T>(hx, hy, hz));
     IM3D_TRY(check_launch(ctx, "grad"));
     IM3D_TRY(out_finish<T>(ctx, out_user, out, 3 * d.n()));
     return sync(ctx);
@@ -2021,7 +2038,7 @@ int div_op(im3d_ctx* ctx, const T* in_user, T* out_user, int nx, int ny, int nz,
     T* out = nullptr;
     IM3D_TRY(dev_in<T>(ctx, in_user, 3 * d.n(), "in_a", &in));
     IM3D_TRY(dev_out<T>(ctx, out_user, d.n(), "out_a", &out));
-    div_kernel<T><<<grid_vol(d, kBlkVol), kBlkVol, 0, ctx->stream>>>(in, out, d, hx, hy, hz);
+    div_kernel<T, kNIdv><<<grid_col(d, kBlkVol, kNIdv), kBlkVol, 0, ctx->stream>>>(in, out, d, make_hstep<T>(hx, hy, hz));
     IM3D_TRY(check_launch(ctx, "div"));
     IM3D_TRY(out_finish<T>(ctx, out_user, out, d.n()));
     return sync(ctx);
@@ -2498,7 +2515,7 @@ int worklist_group(im3d_ctx* ctx, const std::vector<int>& ids, const im3d_volume
     using BrV = BregmanJob<T, kNV, true>;
     using BrS = BregmanJob<T, kNIbr, false>;
     using DvV = DivJob<T, kNV, true>;
-    using DvS = DivJob<T, 0, false>;
+    using DvS = DivJob<T, kNIdv, false>;
     JobTable<KHeav> jk;
     JobTable<SJ4> js4;
     JobTable<SJ2> js2;
@@ -2520,7 +2537,7 @@ int worklist_group(im3d_ctx* ctx, const std::vector<int>& ids, const im3d_volume
     for (int q = 0; q < nv; ++q) {
         const VolState<T>& v = V[q];
         const Dims& d = v.d;
-        const double hx = vols[ids[q]].hx, hy = vols[ids[q]].hy, hz = vols[ids[q]].hz;
+        const HStep<T> hs = make_hstep<T>(vols[ids[q]].hx, vols[ids[q]].hy, vols[ids[q]].hz);
         jk.h.push_back({KHeav{LdHeaviside<T>{v.phi, v.u0, d, v.center, v.inv_eps}, StVec<T, 4>{v.W1, d}, d,
                               v.tp.w[2]}, k_win_grid<T, 4>(d)});
         js4.h.push_back({SJ4{LdVec<T, 4>{v.W1, d}, StVec<T, 4>{v.W2, d}, d, v.tp.w[1]}, s_win_grid<T, 1>(d)});
@@ -2558,15 +2575,15 @@ int worklist_group(im3d_ctx* ctx, const std::vector<int>& ids, const im3d_volume
         jres.h.push_back({Res{v.upk, v.bpk, d, v.coef, part_res[q], ni}, gr});
         fin_res[q] = FinalizeJob{part_res[q], (long long)gr.x * gr.y * gr.z, ctrl[q].sum};
         vecrow[q] = d.nz % V16<T>::W == 0;
-        const dim3 gv = grid_vec<T>(d, kBlkVec), gcol = grid_col(d, kBlkVol), gvol = grid_vol(d, kBlkVol);
+        const dim3 gv = grid_vec<T>(d, kBlkVec), gcol = grid_col(d, kBlkVol);
         jclv.h.push_back({ClV{v.upk, v.phi, nullptr, d, v.a0, v.b0, part_cl[q]}, gv});
         jcls.h.push_back({ClS{v.upk, v.phi, nullptr, d, v.a0, v.b0, part_cl[q]}, gcol});
         const dim3 gcl = vecrow[q] ? gv : gcol;
         fin_cl[q] = FinalizeJob{part_cl[q], (long long)gcl.x * gcl.y * gcl.z, ctrl[q].sum};
-        jbrv.h.push_back({BrV{v.phi, v.b3, v.dmb, v.g, d, hx, hy, hz}, gv});
-        jbrs.h.push_back({BrS{v.phi, v.b3, v.dmb, v.g, d, hx, hy, hz}, grid_col(d, kBlkVol, kNIbr)});
-        jdvv.h.push_back({DvV{v.dmb, v.divdb, d, hx, hy, hz}, gv});
-        jdvs.h.push_back({DvS{v.dmb, v.divdb, d, hx, hy, hz}, gvol});
+        jbrv.h.push_back({BrV{v.phi, v.b3, v.dmb, v.g, d, hs}, gv});
+        jbrs.h.push_back({BrS{v.phi, v.b3, v.dmb, v.g, d, hs}, grid_col(d, kBlkVol, kNIbr)});
+        jdvv.h.push_back({DvV{v.dmb, v.divdb, d, hs}, gv});
+        jdvs.h.push_back({DvS{v.dmb, v.divdb, d, hs}, grid_col(d, kBlkVol, kNIdv)});
     }
     IM3D_TRY(upload_jobs(ctx, "wl_k_heaviside", jk));
     IM3D_TRY(upload_jobs(ctx, "wl_s_j4", js4));

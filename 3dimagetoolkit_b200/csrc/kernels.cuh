@@ -975,35 +975,37 @@ __global__ void __launch_bounds__(TW* TY) conv_i_fit_kernel(const Vec<T, 4>* __r
 }
 
 // ------------------------------------------------------------------ stencils
-// x / (2h) of the difference stencils: FP64 divides, with the reference's operations;
-// FP32 multiplies by the reciprocal, which gives the same value when 2h is a power of
-// two (unit spacing) and is within 1 ulp of it otherwise, at a fraction of a
-// division's instructions.
+// Spacings of the difference stencils, filled on the host (2 h and 1 / (2 h) in T: computed
+// per thread in double they were most of the column kernels' instructions).
 template <typename T>
-__device__ __forceinline__ T over_two_h(T x, T two_h, T inv_two_h)
+struct HStep {
+    T h[3], two[3], inv[3];
+    int pow2;  // bit a set: 2 h of axis a is a power of two
+};
+
+// x / (2h) of the difference stencils: FP64 divides, with the reference's operations (where 2h
+// is a power of two the product with its reciprocal is the same number); FP32 multiplies by
+// the reciprocal, which gives the same value when 2h is a power of two (unit spacing) and is
+// within 1 ulp of it otherwise, at a fraction of a division's instructions.
+template <int AXIS, typename T>
+__device__ __forceinline__ T over_two_h(T x, const HStep<T>& hs)
 {
-    if constexpr (sizeof(T) == 4) return x * inv_two_h;
-    else return x / two_h;
+    if constexpr (sizeof(T) == 4) return x * hs.inv[AXIS];
+    else return (hs.pow2 >> AXIS & 1) ? x * hs.inv[AXIS] : x / hs.two[AXIS];
 }
 
 // One component of image3d::grad at a point with position pos on an axis of length
 // len (image3d_imp.hxx:762-838): central inside, one-sided second order on faces.
-template <typename T>
-__device__ __forceinline__ T grad_term(const T* f, long long p, long long stride, int pos,
-                                       int len, double h)
+template <int AXIS, typename T>
+__device__ __forceinline__ T grad_term(const T* f, long long p, long long stride, int pos, int len, const HStep<T>& hs)
 {
-    // FP32 multiplies by 1/(2h) as the vectorised kernels do (over_two_h); FP64 divides
-    const T two_h = T(2. * h), inv_two_h = T(1. / (2. * h));
-    if (pos == 0)
-        return over_two_h(T(4) * f[p + stride] - T(3) * f[p] - f[p + 2 * stride], two_h, inv_two_h);
-    if (pos == len - 1)
-        return over_two_h(T(3) * f[p] - T(4) * f[p - stride] + f[p - 2 * stride], two_h, inv_two_h);
-    return over_two_h(f[p + stride] - f[p - stride], two_h, inv_two_h);
+    if (pos == 0) return over_two_h<AXIS>(T(4) * f[p + stride] - T(3) * f[p] - f[p + 2 * stride], hs);
+    if (pos == len - 1) return over_two_h<AXIS>(T(3) * f[p] - T(4) * f[p - stride] + f[p - 2 * stride], hs);
+    return over_two_h<AXIS>(f[p + stride] - f[p - stride], hs);
 }
 
 template <typename T>
-__global__ void grad_kernel(const T* __restrict__ f, T* __restrict__ g, Dims d, double hx,
-                            double hy, double hz)
+__global__ void grad_kernel(const T* __restrict__ f, T* __restrict__ g, Dims d, HStep<T> hs)
 {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
@@ -1011,9 +1013,9 @@ __global__ void grad_kernel(const T* __restrict__ f, T* __restrict__ g, Dims d, 
     if (k >= d.nz || j >= d.ny) return;
     const long long p = d.idx(i, j, k);
     const long long n = d.n();
-    g[p] = grad_term(f, p, (long long)d.ny * d.nz, i, d.nx, hx);
-    g[n + p] = grad_term(f, p, (long long)d.nz, j, d.ny, hy);
-    g[2 * n + p] = grad_term(f, p, 1, k, d.nz, hz);
+    g[p] = grad_term<0>(f, p, (long long)d.ny * d.nz, i, d.nx, hs);
+    g[n + p] = grad_term<1>(f, p, (long long)d.nz, j, d.ny, hs);
+    g[2 * n + p] = grad_term<2>(f, p, 1, k, d.nz, hs);
 }
 
 // im3d::div at one point (image3d_imp.hxx:1060-1380) with the reference's two
@@ -1022,7 +1024,7 @@ __global__ void grad_kernel(const T* __restrict__ f, T* __restrict__ g, Dims d, 
 // z term reads Z-2 twice (:1203-1213).
 template <typename T>
 __device__ __forceinline__ T div_point(const T* f0, const T* f1, const T* f2, const Dims& d,
-                                       int i, int j, int k, double hx, double hy, double hz)
+                                       int i, int j, int k, HStep<T> hs)
 {
     const long long p = d.idx(i, j, k);
     const long long sx = (long long)d.ny * d.nz, sy = d.nz;
@@ -1031,48 +1033,93 @@ __device__ __forceinline__ T div_point(const T* f0, const T* f1, const T* f2, co
     const int cz = k == 0 ? 0 : (k == d.nz - 1 ? 2 : 1);
     T tx, tz;
     if (cx == 2 && cy == 1 && cz == 1)
-        tx = (T(3) * f0[p] - T(4) * f0[p - sx] + f0[p - 2 * sx]) / T(2.) * T(hx);
+        tx = (T(3) * f0[p] - T(4) * f0[p - sx] + f0[p - 2 * sx]) / T(2.) * hs.h[0];
     else
-        tx = grad_term(f0, p, sx, i, d.nx, hx);
-    const T ty = grad_term(f1, p, sy, j, d.ny, hy);
+        tx = grad_term<0>(f0, p, sx, i, d.nx, hs);
+    const T ty = grad_term<1>(f1, p, sy, j, d.ny, hs);
     if (cx == 1 && cy == 0 && cz == 2)
-        tz = (T(3) * f2[p] - T(4) * f2[p - 1] + f2[p - 1]) / T(2. * hz);
+        tz = (T(3) * f2[p] - T(4) * f2[p - 1] + f2[p - 1]) / hs.two[2];
     else
-        tz = grad_term(f2, p, 1, k, d.nz, hz);
+        tz = grad_term<2>(f2, p, 1, k, d.nz, hs);
     return tx + ty + tz;
 }
 
-template <typename T>
-__device__ __forceinline__ void div_body(const uint3 blockIdx, const dim3 gridDim, const T* __restrict__ v, T* __restrict__ out, Dims d, double hx, double hy, double hz)
+// div_point for every cell, any nz: a thread owns the (j, k) column of NI planes, consecutive
+// lanes consecutive k. Rows inside i and j take central x and y terms and a z term whose
+// one-sided forms on the faces k = 0 and k = nz - 1 replace it by selects (the third point is
+// read beside the neighbours); other rows take div_point. Every read of the NI planes comes
+// before the first store. One cell per thread by div_point alone with the spacings divided per
+// thread took 40 us at 171x203x117, the columns 33 us, and with HStep 31 us (FP32).
+template <typename T, int NI>
+__device__ __forceinline__ void div_body(const uint3 blockIdx, const dim3 gridDim, const T* __restrict__ v, T* __restrict__ out, Dims d, HStep<T> hs)
 {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int i = blockIdx.z;
+    const int i0 = blockIdx.z * NI;
     if (k >= d.nz || j >= d.ny) return;
-    const long long n = d.n();
-    out[d.idx(i, j, k)] = div_point(v, v + n, v + 2 * n, d, i, j, k, hx, hy, hz);
+    const int cnt = min(NI, d.nx - i0);
+    const long long n = d.n(), plane = (long long)d.ny * d.nz, sy = d.nz;
+    const T *f0 = v, *f1 = v + n, *f2 = v + 2 * n;
+    const long long p0 = d.idx(i0, j, k);
+    const bool jint = j >= 1 && j <= d.ny - 2;
+    // the two z neighbours, or on a face the two points inward: a = k + 1 (k - 1 at the high
+    // face), b = k - 1 (k + 2 at the low face, k - 2 at the high one)
+    const int za = k == d.nz - 1 ? -1 : 1, zb = k == 0 ? 2 : (k == d.nz - 1 ? -2 : -1);
+    T x[NI + 2], ym[NI], yp[NI], z0[NI], z1[NI], zc[NI];
+#pragma unroll
+    for (int t = 0; t < NI + 2; ++t) {
+        const int i = i0 - 1 + t;
+        x[t] = (t <= cnt + 1 && i >= 0 && i < d.nx) ? f0[p0 + (t - 1) * plane] : T(0);
+    }
+#pragma unroll
+    for (int t = 0; t < NI; ++t) {
+        ym[t] = yp[t] = z0[t] = z1[t] = zc[t] = T(0);
+        if (t >= cnt || !jint) continue;
+        const long long p = p0 + t * plane;
+        ym[t] = f1[p - sy];
+        yp[t] = f1[p + sy];
+        zc[t] = f2[p];
+        z0[t] = f2[p + za];
+        z1[t] = f2[p + zb];
+    }
+#pragma unroll
+    for (int t = 0; t < NI; ++t) {
+        if (t >= cnt) break;
+        const int i = i0 + t;
+        T r;
+        if (jint && i >= 1 && i <= d.nx - 2) {
+            const T tx = over_two_h<0>(x[t + 2] - x[t], hs);
+            const T ty = over_two_h<1>(yp[t] - ym[t], hs);
+            const T mid = over_two_h<2>(z0[t] - z1[t], hs);
+            const T lo = over_two_h<2>(T(4) * z0[t] - T(3) * zc[t] - z1[t], hs);
+            const T hi = over_two_h<2>(T(3) * zc[t] - T(4) * z0[t] + z1[t], hs);
+            r = tx + ty + (k == 0 ? lo : (k == d.nz - 1 ? hi : mid));
+        } else {
+            r = div_point(f0, f1, f2, d, i, j, k, hs);
+        }
+        out[p0 + t * plane] = r;
+    }
 }
 
-template <typename T>
-__global__ void div_kernel(const T* __restrict__ v, T* __restrict__ out, Dims d, double hx, double hy, double hz)
+template <typename T, int NI>
+__global__ void __launch_bounds__(256) div_kernel(const T* __restrict__ v, T* __restrict__ out, Dims d, HStep<T> hs)
 {
-    div_body<T>(blockIdx, gridDim, v, out, d, hx, hy, hz);
+    div_body<T, NI>(blockIdx, gridDim, v, out, d, hs);
 }
 
 // Edge detector, GRAD branch (rsfe_splitbregman_imp.hxx:220-232, 308-313):
 // g = nu / (lamda (1 + beta |grad f|^2)), evaluated in the reference's order.
 template <typename T>
-__global__ void edge_kernel(const T* __restrict__ f, T* __restrict__ g, Dims d, double hx,
-                            double hy, double hz, T beta, T lamda, T nu)
+__global__ void edge_kernel(const T* __restrict__ f, T* __restrict__ g, Dims d, HStep<T> hs, T beta, T lamda, T nu)
 {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     const int i = blockIdx.z;
     if (k >= d.nz || j >= d.ny) return;
     const long long p = d.idx(i, j, k);
-    const T g0 = grad_term(f, p, (long long)d.ny * d.nz, i, d.nx, hx);
-    const T g1 = grad_term(f, p, (long long)d.nz, j, d.ny, hy);
-    const T g2 = grad_term(f, p, 1, k, d.nz, hz);
+    const T g0 = grad_term<0>(f, p, (long long)d.ny * d.nz, i, d.nx, hs);
+    const T g1 = grad_term<1>(f, p, (long long)d.nz, j, d.ny, hs);
+    const T g2 = grad_term<2>(f, p, 1, k, d.nz, hs);
     T a = g0 * g0;
     a += g1 * g1;
     a += g2 * g2;
@@ -2075,7 +2122,7 @@ __global__ void __launch_bounds__(256) clamp_tol_kernel(const T* __restrict__ u,
 // Thread per (k, j) column marching over NI planes with phi(i-1), phi(i), phi(i+1)
 // in registers; j and k neighbours come through L1.
 template <typename T, int NI>
-__device__ __forceinline__ void bregman_body(const uint3 blockIdx, const dim3 gridDim, const T* __restrict__ phi, T* __restrict__ b3, T* __restrict__ dmb, const T* __restrict__ g, Dims d, double hx, double hy, double hz)
+__device__ __forceinline__ void bregman_body(const uint3 blockIdx, const dim3 gridDim, const T* __restrict__ phi, T* __restrict__ b3, T* __restrict__ dmb, const T* __restrict__ g, Dims d, HStep<T> hs)
 {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
@@ -2086,8 +2133,6 @@ __device__ __forceinline__ void bregman_body(const uint3 blockIdx, const dim3 gr
     const long long n = d.n();
     const long long sy = d.nz;
     const long long p0 = d.idx(i0, j, k);
-    const T two_hx = T(2. * hx), two_hy = T(2. * hy), two_hz = T(2. * hz);
-    const T ihx = T(1. / (2. * hx)), ihy = T(1. / (2. * hy)), ihz = T(1. / (2. * hz));
     // Every load of the NI planes is issued before the first store (the stores to b3
     // and dmb would otherwise hold the next plane's loads back): phi along i for planes
     // i0-1 .. i0+NI (and the second one-sided point on an i face), the j and k
@@ -2135,16 +2180,16 @@ __device__ __forceinline__ void bregman_body(const uint3 blockIdx, const dim3 gr
         const long long p = p0 + (long long)t * plane;
         const T fm = fi[t], f0 = fi[t + 1], fp = fi[t + 2];
         T gr[3];
-        if (i == 0) gr[0] = over_two_h(T(4) * fp - T(3) * f0 - fi2[t], two_hx, ihx);
-        else if (i == d.nx - 1) gr[0] = over_two_h(T(3) * f0 - T(4) * fm + fi2[t], two_hx, ihx);
-        else gr[0] = over_two_h(fp - fm, two_hx, ihx);
+        if (i == 0) gr[0] = over_two_h<0>(T(4) * fp - T(3) * f0 - fi2[t], hs);
+        else if (i == d.nx - 1) gr[0] = over_two_h<0>(T(3) * f0 - T(4) * fm + fi2[t], hs);
+        else gr[0] = over_two_h<0>(fp - fm, hs);
         // j == 0: fjp = phi(j+1), fjm = phi(j+2); j == ny-1: fjm = phi(j-1), fjp = phi(j-2)
-        if (j == 0) gr[1] = over_two_h(T(4) * fjp[t] - T(3) * f0 - fjm[t], two_hy, ihy);
-        else if (j == d.ny - 1) gr[1] = over_two_h(T(3) * f0 - T(4) * fjm[t] + fjp[t], two_hy, ihy);
-        else gr[1] = over_two_h(fjp[t] - fjm[t], two_hy, ihy);
-        if (k == 0) gr[2] = over_two_h(T(4) * fkp[t] - T(3) * f0 - fkm[t], two_hz, ihz);
-        else if (k == d.nz - 1) gr[2] = over_two_h(T(3) * f0 - T(4) * fkm[t] + fkp[t], two_hz, ihz);
-        else gr[2] = over_two_h(fkp[t] - fkm[t], two_hz, ihz);
+        if (j == 0) gr[1] = over_two_h<1>(T(4) * fjp[t] - T(3) * f0 - fjm[t], hs);
+        else if (j == d.ny - 1) gr[1] = over_two_h<1>(T(3) * f0 - T(4) * fjm[t] + fjp[t], hs);
+        else gr[1] = over_two_h<1>(fjp[t] - fjm[t], hs);
+        if (k == 0) gr[2] = over_two_h<2>(T(4) * fkp[t] - T(3) * f0 - fkm[t], hs);
+        else if (k == d.nz - 1) gr[2] = over_two_h<2>(T(3) * f0 - T(4) * fkm[t] + fkp[t], hs);
+        else gr[2] = over_two_h<2>(fkp[t] - fkm[t], hs);
         const T gg = gv[t];
 #pragma unroll
         for (int cmp = 0; cmp < 3; ++cmp) {
@@ -2161,9 +2206,9 @@ __device__ __forceinline__ void bregman_body(const uint3 blockIdx, const dim3 gr
 }
 
 template <typename T, int NI>
-__global__ void __launch_bounds__(256) bregman_kernel(const T* __restrict__ phi, T* __restrict__ b3, T* __restrict__ dmb, const T* __restrict__ g, Dims d, double hx, double hy, double hz)
+__global__ void __launch_bounds__(256) bregman_kernel(const T* __restrict__ phi, T* __restrict__ b3, T* __restrict__ dmb, const T* __restrict__ g, Dims d, HStep<T> hs)
 {
-    bregman_body<T, NI>(blockIdx, gridDim, phi, b3, dmb, g, d, hx, hy, hz);
+    bregman_body<T, NI>(blockIdx, gridDim, phi, b3, dmb, g, d, hs);
 }
 
 // ---- vectorised natural-layout kernels (nz a multiple of W = 16/sizeof(T)) ----
@@ -2245,7 +2290,7 @@ __global__ void __launch_bounds__(256) clamp_tol_vec_kernel(const T* __restrict_
 // Split-Bregman update (see bregman_kernel), vectorised along k; rows on an i or j face
 // of the volume take the scalar one-sided stencils.
 template <typename T, int NI>
-__device__ __forceinline__ void bregman_vec_body(const uint3 blockIdx, const dim3 gridDim, const T* __restrict__ phi, T* __restrict__ b3, T* __restrict__ dmb, const T* __restrict__ g3, Dims d, double hx, double hy, double hz)
+__device__ __forceinline__ void bregman_vec_body(const uint3 blockIdx, const dim3 gridDim, const T* __restrict__ phi, T* __restrict__ b3, T* __restrict__ dmb, const T* __restrict__ g3, Dims d, HStep<T> hs)
 {
     typedef V16<T> VT;
     typedef typename VT::type VV;
@@ -2258,8 +2303,6 @@ __device__ __forceinline__ void bregman_vec_body(const uint3 blockIdx, const dim
     const long long plane = (long long)d.ny * d.nz;
     const long long sy = d.nz;
     const long long n = d.n();
-    const T two_hx = T(2. * hx), two_hy = T(2. * hy), two_hz = T(2. * hz);
-    const T ihx = T(1. / (2. * hx)), ihy = T(1. / (2. * hy)), ihz = T(1. / (2. * hz));
     const bool jint = j >= 1 && j <= d.ny - 2;
     const long long p0 = d.idx(i0, j, kb);
     VV f[NI + 2];
@@ -2317,23 +2360,23 @@ __device__ __forceinline__ void bregman_vec_body(const uint3 blockIdx, const dim
                 // i and j inside: central x and y terms; the z term is central or, on
                 // the faces k = 0 and k = nz-1, grad_term's one-sided difference,
                 // evaluated with the same operations without a branch
-                gr[0] = over_two_h(VT::get(f[t + 2], cc) - VT::get(f[t], cc), two_hx, ihx);
-                gr[1] = over_two_h(VT::get(yp, cc) - VT::get(ym, cc), two_hy, ihy);
-                T tz = over_two_h(zz[cc + 2] - zz[cc], two_hz, ihz);
+                gr[0] = over_two_h<0>(VT::get(f[t + 2], cc) - VT::get(f[t], cc), hs);
+                gr[1] = over_two_h<1>(VT::get(yp, cc) - VT::get(ym, cc), hs);
+                T tz = over_two_h<2>(zz[cc + 2] - zz[cc], hs);
                 if (cc == 0) {
-                    const T lo = over_two_h(T(4) * zz[cc + 2] - T(3) * zz[cc + 1] - zz[cc + 3], two_hz, ihz);
+                    const T lo = over_two_h<2>(T(4) * zz[cc + 2] - T(3) * zz[cc + 1] - zz[cc + 3], hs);
                     tz = k == 0 ? lo : tz;
                 }
                 if (cc == W - 1) {
-                    const T hi = over_two_h(T(3) * zz[cc + 1] - T(4) * zz[cc] + zz[cc - 1], two_hz, ihz);
+                    const T hi = over_two_h<2>(T(3) * zz[cc + 1] - T(4) * zz[cc] + zz[cc - 1], hs);
                     tz = k == d.nz - 1 ? hi : tz;
                 }
                 gr[2] = tz;
             } else {
                 const long long pc = p + cc;
-                gr[0] = grad_term(phi, pc, plane, i, d.nx, hx);
-                gr[1] = grad_term(phi, pc, sy, j, d.ny, hy);
-                gr[2] = grad_term(phi, pc, 1, k, d.nz, hz);
+                gr[0] = grad_term<0>(phi, pc, plane, i, d.nx, hs);
+                gr[1] = grad_term<1>(phi, pc, sy, j, d.ny, hs);
+                gr[2] = grad_term<2>(phi, pc, 1, k, d.nz, hs);
             }
             const T gv = VT::get(gg, cc);
 #pragma unroll
@@ -2357,15 +2400,15 @@ __device__ __forceinline__ void bregman_vec_body(const uint3 blockIdx, const dim
 }
 
 template <typename T, int NI>
-__global__ void __launch_bounds__(256) bregman_vec_kernel(const T* __restrict__ phi, T* __restrict__ b3, T* __restrict__ dmb, const T* __restrict__ g3, Dims d, double hx, double hy, double hz)
+__global__ void __launch_bounds__(256) bregman_vec_kernel(const T* __restrict__ phi, T* __restrict__ b3, T* __restrict__ dmb, const T* __restrict__ g3, Dims d, HStep<T> hs)
 {
-    bregman_vec_body<T, NI>(blockIdx, gridDim, phi, b3, dmb, g3, d, hx, hy, hz);
+    bregman_vec_body<T, NI>(blockIdx, gridDim, phi, b3, dmb, g3, d, hs);
 }
 
 // im3d::div vectorised along k (see div_point); rows on an i or j face of the volume
 // take the scalar rule with the reference's quirks.
 template <typename T, int NI>
-__device__ __forceinline__ void div_vec_body(const uint3 blockIdx, const dim3 gridDim, const T* __restrict__ v, T* __restrict__ out, Dims d, double hx, double hy, double hz)
+__device__ __forceinline__ void div_vec_body(const uint3 blockIdx, const dim3 gridDim, const T* __restrict__ v, T* __restrict__ out, Dims d, HStep<T> hs)
 {
     typedef V16<T> VT;
     typedef typename VT::type VV;
@@ -2381,8 +2424,6 @@ __device__ __forceinline__ void div_vec_body(const uint3 blockIdx, const dim3 gr
     const T* f0 = v;
     const T* f1 = v + n;
     const T* f2 = v + 2 * n;
-    const T two_hx = T(2. * hx), two_hy = T(2. * hy), two_hz = T(2. * hz);
-    const T ihx = T(1. / (2. * hx)), ihy = T(1. / (2. * hy)), ihz = T(1. / (2. * hz));
     const bool jint = j >= 1 && j <= d.ny - 2;
     const long long p0 = d.idx(i0, j, kb);
     VV x[NI + 2];
@@ -2415,31 +2456,31 @@ __device__ __forceinline__ void div_vec_body(const uint3 blockIdx, const dim3 gr
 #pragma unroll
             for (int cc = 0; cc < W; ++cc) {
                 const int k = kb + cc;
-                const T tx = over_two_h(VT::get(x[t + 2], cc) - VT::get(x[t], cc), two_hx, ihx);
-                const T ty = over_two_h(VT::get(yp, cc) - VT::get(ym, cc), two_hy, ihy);
-                T tz = over_two_h(zz[cc + 2] - zz[cc], two_hz, ihz);
+                const T tx = over_two_h<0>(VT::get(x[t + 2], cc) - VT::get(x[t], cc), hs);
+                const T ty = over_two_h<1>(VT::get(yp, cc) - VT::get(ym, cc), hs);
+                T tz = over_two_h<2>(zz[cc + 2] - zz[cc], hs);
                 if (cc == 0) {
-                    const T lo = over_two_h(T(4) * zz[cc + 2] - T(3) * zz[cc + 1] - zz[cc + 3], two_hz, ihz);
+                    const T lo = over_two_h<2>(T(4) * zz[cc + 2] - T(3) * zz[cc + 1] - zz[cc + 3], hs);
                     tz = k == 0 ? lo : tz;
                 }
                 if (cc == W - 1) {
-                    const T hi = over_two_h(T(3) * zz[cc + 1] - T(4) * zz[cc] + zz[cc - 1], two_hz, ihz);
+                    const T hi = over_two_h<2>(T(3) * zz[cc + 1] - T(4) * zz[cc] + zz[cc - 1], hs);
                     tz = k == d.nz - 1 ? hi : tz;
                 }
                 VT::set(o, cc, tx + ty + tz);
             }
         } else {
 #pragma unroll
-            for (int cc = 0; cc < W; ++cc) VT::set(o, cc, div_point(f0, f1, f2, d, i, j, kb + cc, hx, hy, hz));
+            for (int cc = 0; cc < W; ++cc) VT::set(o, cc, div_point(f0, f1, f2, d, i, j, kb + cc, hs));
         }
         *reinterpret_cast<VV*>(out + p) = o;
     }
 }
 
 template <typename T, int NI>
-__global__ void __launch_bounds__(256) div_vec_kernel(const T* __restrict__ v, T* __restrict__ out, Dims d, double hx, double hy, double hz)
+__global__ void __launch_bounds__(256) div_vec_kernel(const T* __restrict__ v, T* __restrict__ out, Dims d, HStep<T> hs)
 {
-    div_vec_body<T, NI>(blockIdx, gridDim, v, out, d, hx, hy, hz);
+    div_vec_body<T, NI>(blockIdx, gridDim, v, out, d, hs);
 }
 
 // sum (a - b)^2 and sum b^2 over n elements (relative change of a sweep)

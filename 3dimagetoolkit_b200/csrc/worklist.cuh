@@ -173,11 +173,11 @@ struct BregmanJob {
     T* dmb;
     const T* g3;
     Dims d;
-    double hx, hy, hz;
+    HStep<T> hs;
     __device__ __forceinline__ void operator()(uint3 b, dim3 g, int) const
     {
-        if constexpr (VEC) bregman_vec_body<T, NI>(b, g, phi, b3, dmb, g3, d, hx, hy, hz);
-        else bregman_body<T, NI>(b, g, phi, b3, dmb, g3, d, hx, hy, hz);
+        if constexpr (VEC) bregman_vec_body<T, NI>(b, g, phi, b3, dmb, g3, d, hs);
+        else bregman_body<T, NI>(b, g, phi, b3, dmb, g3, d, hs);
     }
 };
 
@@ -186,11 +186,11 @@ struct DivJob {
     const T* v;
     T* out;
     Dims d;
-    double hx, hy, hz;
+    HStep<T> hs;
     __device__ __forceinline__ void operator()(uint3 b, dim3 g, int) const
     {
-        if constexpr (VEC) div_vec_body<T, NI>(b, g, v, out, d, hx, hy, hz);
-        else div_body<T>(b, g, v, out, d, hx, hy, hz);
+        if constexpr (VEC) div_vec_body<T, NI>(b, g, v, out, d, hs);
+        else div_body<T, NI>(b, g, v, out, d, hs);
     }
 };
 
