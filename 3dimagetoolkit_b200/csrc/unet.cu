@@ -231,19 +231,23 @@ template <int CO, int CI>
 int wgrad_launch(cudaStream_t st, const View& x, int xcoff, int cin, const View& dz, int zcoff, int cout, float* dw,
                  int* errf, std::string& err)
 {
-    const int TW = x.W <= 128 ? x.W : 128;
-    if (x.W % 16 != 0 || x.W % TW != 0) {
+    const int TWm = x.W <= 128 ? x.W : 128;
+    if (x.W % 16 != 0 || x.W % TWm != 0) {
         err = "weight gradient: W must be a multiple of 16, and of 128 above 128";
         return IM3D_ERR_UNSUPPORTED;
     }
     const int nblocks = (cout / CO) * (cin / CI);
     const int ctas = std::max(1, g_num_sms / nblocks);
-    for (int TH : {4, 2, 1}) {
-        if (TH > x.H && TH > 1) continue;
+    // four rows first, then the width: a plane of X carries two more rows and columns than its tile
+    for (int t = 0; t < 6; ++t) {
+        const int TH = 4 >> (t / 2), TW = t % 2 ? TWm / 2 : TWm;
+        if ((TH > x.H && TH > 1) || TW % 16 != 0) continue;
         WgradArgs a;
-        a.xbytes = align_up((TH + 2) * (TW + 2) * 2 * CI, 1024);
+        a.xbytes = align_up((TH + 2) * (TW + 8) * 2 * CI, 1024);
         a.zbytes = align_up(TH * TW * 2 * CO, 1024);
-        const int smem = 1024 + kWgXStages * a.xbytes + kWgZStages * a.zbytes + 16 * (kWgXStages + kWgZStages);
+        const int rings = kWgXStages * a.xbytes + kWgZStages * a.zbytes;
+        // the rings hold the sums of the block at the end
+        const int smem = 1024 + std::max(rings + 16 * (kWgXStages + kWgZStages), CO * CI * 27 * 4);
         if (smem > 226 * 1024) continue;
         a.D = x.D;
         a.H = x.H;
@@ -252,10 +256,7 @@ int wgrad_launch(cudaStream_t st, const View& x, int xcoff, int cin, const View&
         a.TW = TW;
         a.tiles_w = x.W / TW;
         a.tiles_h = (x.H + TH - 1) / TH;
-        const long long cols = (long long)x.nsamp * a.tiles_w * a.tiles_h;
-        a.zc = plan_zc(x.D, cols, ctas);
-        a.nzc = (x.D + a.zc - 1) / a.zc;
-        a.units = cols * a.nzc;
+        a.planes = (long long)x.nsamp * a.tiles_w * a.tiles_h * x.D;
         a.zcoff = zcoff;
         a.xcoff = xcoff;
         a.cin = cin;
@@ -263,11 +264,11 @@ int wgrad_launch(cudaStream_t st, const View& x, int xcoff, int cin, const View&
         a.dw = dw;
         a.err = errf;
         CUtensorMap xm, zm;
-        UN_TRY(make_map(x, CI, TW + 2, TH + 2, &xm, err));
+        UN_TRY(make_map(x, CI, TW + 8, TH + 2, &xm, err));
         UN_TRY(make_map(dz, CO, TW, TH, &zm, err));
         auto kern = wgrad_mma_kernel<CO, CI>;
         UN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        const long long gx = std::min<long long>(ctas, a.units);
+        const long long gx = std::min<long long>(ctas, a.planes);
         kern<<<dim3((unsigned)gx, (unsigned)nblocks), kWgThreads, smem, st>>>(xm, zm, a);
         return launch_status(err, "wgrad_mma_kernel");
     }

@@ -418,7 +418,7 @@ __global__ void __launch_bounds__(kMarchThreads, 1) conv3_march_kernel(const __g
 }
 
 // ---------------------------------------------------------------- weight gradient
-constexpr int kWgWarps = 9;                      // multiplying warps: one per (dz, dy)
+constexpr int kWgWarps = 12;                     // multiplying warps: 4 per dz
 constexpr int kWgThreads = 32 * (kWgWarps + 1);  // and one that loads
 constexpr int kWgXStages = 5, kWgZStages = 3;      // planes of X and of dZ in shared memory
 
@@ -426,8 +426,7 @@ struct WgradArgs {
     int D, H, W;      // volume of one sample
     int TH, TW;       // tile rows and columns (TW divides W, TW <= 128, a multiple of 16)
     int tiles_w, tiles_h;
-    int zc, nzc;      // planes of a unit, units along z
-    long long units;  // nsamp * nzc * tiles_h * tiles_w
+    long long planes;  // nsamp * tiles_h * tiles_w * D, split evenly over the blocks
     int xbytes, zbytes;  // a staged plane of X (halo included) and of dZ, multiples of 1024
     int zcoff, xcoff;    // first channel of dZ and of X in their tensors
     int cin;             // input channels of the layer
@@ -460,24 +459,57 @@ __device__ __forceinline__ uint32_t swizzled(int r, int c)
     return (uint32_t)(r * ROW + ((ROW == 32 ? c ^ ((r >> 2) & 1) : c ^ ((r >> 1) & 3)) << 4));
 }
 
+// One step of a warp of wgrad_mma_kernel: 16 voxels of each of R rows of dZ against the R + 2
+// rows of X around them, for the nine (dy, dx) taps. zp, xp: addresses of this lane's ldmatrix
+// rows in the first row of dZ and of X (for each dx); zpitch, xpitch: bytes to the next row.
+template <int R>
+__device__ __forceinline__ void wgrad_rows(float (&acc)[3][3][2][4], uint32_t zp, const uint32_t (&xp)[3], uint32_t zpitch,
+                                           uint32_t xpitch)
+{
+    uint32_t zf[R][4];
+#pragma unroll
+    for (int h = 0; h < R + 2; ++h) {
+        uint32_t xf[3][4];
+        if (h < R) ldmatrix_x4_trans(zp + h * zpitch, zf[h < R ? h : 0]);
+#pragma unroll
+        for (int t = 0; t < 3; ++t) ldmatrix_x4_trans(xp[t] + h * xpitch, xf[t]);
+#pragma unroll
+        for (int dy = 2; dy >= 0; --dy) {
+            if (h - dy < 0 || h - dy >= R) continue;
+#pragma unroll
+            for (int t = 0; t < 3; ++t)
+#pragma unroll
+                for (int n = 0; n < 2; ++n)
+                    mma_16816(acc[dy][t][n], zf[h - dy < 0 || h - dy >= R ? 0 : h - dy], xf[t][2 * n], xf[t][2 * n + 1]);
+        }
+    }
+}
+
 // dW[co][ci][tap] = sum over voxels of dZ[v][co] X[v + tap][ci], for CO output and CI input
-// channels (blockIdx.y). A CTA marches along z through units of TH x TW columns: X planes and
-// dZ planes stream through rings in shared memory (TMA), each X plane serving three output
-// planes. Warp (dz, dy) keeps the accumulators of its three dx taps in registers over all its
-// units and adds them to the gradient once.
+// channels (blockIdx.y). The planes of all tiles are split evenly over the blocks; a block
+// marches along z: X planes and dZ planes stream through rings in shared memory (TMA), each X
+// plane serving three output planes. A warp holds the sums of 16 x 16 channels for the nine
+// (dy, dx) taps of one dz in registers, over all its planes; the four warps of a dz (one per
+// scheduler, so that the tensor pipes are loaded alike) take the blocks of 16 x 16 channels and,
+// where these are fewer than four, shares of the voxels. The block's sums are joined in shared
+// memory and added to the gradient once, 16 bytes per atomic.
 // The products run on mma.sync (M = 16 output channels, N = 8 input channels, K = 16 voxels):
 // both operands are read transposed from channels-last rows by ldmatrix, and M = 16 fits 16
 // and 32 channels exactly, where tcgen05's smallest M (64) multiplies three quarters or half
 // of it for nothing and needs one MMA per tap of 16 or 32 columns.
-// What bounds it: the TMA's rows of 32 or 64 bytes (twice the multiplying warps measured the
-// same). us against the tcgen05 form (M = 64, N = CI, load and multiply in turn): 16 x 16 at
-// 128^3 929 -> 131, 16 x 32 at 128^3 about 950 -> 227, 32 x 32 at 64^3 about 420 -> 79.
+// What bounds it: the tensor pipe, about 8 cycles per mma.sync of a scheduler, 50 to 75 % of
+// the time; staging alone takes 48 of 90 us. us against one warp per (dz, dy), which left one
+// scheduler with half more to do than the others, read each X fragment three times from shared
+// memory and ran whole columns per block on 128 of 148 SMs: 16 x 16 at 128^3 130 -> 90,
+// 16 x 32 at 128^3 227 -> 157, 32 x 32 at 64^3 80 -> 48, 32 x 16 at 64^3 51 -> 32 (the tcgen05
+// form, M = 64, N = CI, load and multiply in turn: 929, 950, 420).
 template <int CO, int CI>
 __global__ void __launch_bounds__(kWgThreads, 1) wgrad_mma_kernel(const __grid_constant__ CUtensorMap xmap,
                                                                   const __grid_constant__ CUtensorMap zmap,
                                                                   const __grid_constant__ WgradArgs a)
 {
     constexpr int RX = 2 * CI, RZ = 2 * CO;  // bytes of a row (one voxel)
+    constexpr int MB = CO / 16, NB = CI / 16, KQ = 4 / (MB * NB);
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -502,15 +534,22 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_mma_kernel(const __grid_c
     }
     __syncthreads();
     const int cob = blockIdx.y / a.ciblocks, cib = blockIdx.y % a.ciblocks;
-    const int P = a.TW + 2;
-    auto unit = [&](long long u, int& w0, int& h0, int& z0, int& zn, int& s) {
-        w0 = (int)(u % a.tiles_w) * a.TW;
-        u /= a.tiles_w;
-        h0 = (int)(u % a.tiles_h) * a.TH;
-        u /= a.tiles_h;
-        z0 = (int)(u % a.nzc) * a.zc;
-        s = (int)(u / a.nzc);
-        zn = min(a.zc, a.D - z0);
+    const int P = a.TW + 8;  // voxels of a staged row of X: a multiple of 8 keeps the swizzle's phase
+    // multiplying warp: filter plane dz, block (mb, nb) of 16 x 16 channels, share kq of the voxels
+    const int dz = warp / 4, mb = warp % 4 % MB, nb = warp % 4 / MB % NB, kq = warp % 4 / (MB * NB);
+    float acc[3][3][2][4];  // [dy][dx][8 input channels]
+#pragma unroll
+    for (int e = 0; e < 72; ++e) (&acc[0][0][0][0])[e] = 0.f;
+    // this block's planes, and the column (tile) and planes of it that start at plane p
+    const long long p0 = a.planes * blockIdx.x / gridDim.x, p1 = a.planes * (blockIdx.x + 1) / gridDim.x;
+    auto unit = [&](long long p, int& w0, int& h0, int& z0, int& zn, int& s) {
+        long long c = p / a.D;
+        z0 = (int)(p - c * a.D);
+        zn = (int)min((long long)(a.D - z0), p1 - p);
+        w0 = (int)(c % a.tiles_w) * a.TW;
+        c /= a.tiles_w;
+        h0 = (int)(c % a.tiles_h) * a.TH;
+        s = (int)(c / a.tiles_h);
     };
     if (warp == kWgWarps) {
         if (lane == 0) {
@@ -518,9 +557,10 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_mma_kernel(const __grid_c
             int sx = 0, sz = 0, nx = 0, nzl = 0;  // next stages, loads issued (up to the stages)
             uint32_t phx = 1, phz = 1;            // parity of a free stage: the first pass finds them free
             bool ok = true;
-            for (long long u = blockIdx.x; u < a.units && ok; u += gridDim.x) {
-                int w0, h0, z0, zn, s;
-                unit(u, w0, h0, z0, zn, s);
+            int zn;
+            for (long long p = p0; p < p1 && ok; p += zn) {
+                int w0, h0, z0, s;
+                unit(p, w0, h0, z0, zn, s);
                 // X planes z0 - 1 .. z0 + zn; the dZ plane z goes out with the X plane z + 1
                 for (int z = z0 - 1; z <= z0 + zn && ok; ++z) {
                     ok = tc::mbar_wait(emptyx + sx, phx) && !s_fail;
@@ -552,28 +592,26 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_mma_kernel(const __grid_c
             }
         }
     } else {
-        const int dz = warp / 3, dy = warp - 3 * dz;
-        float acc[3][CO / 16][CI / 8][4];
-#pragma unroll
-        for (int t = 0; t < 3; ++t)
-#pragma unroll
-            for (int m = 0; m < CO / 16; ++m)
-#pragma unroll
-                for (int n = 0; n < CI / 8; ++n)
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) acc[t][m][n][e] = 0.f;
         // ldmatrix rows of this lane: A (voxel, chunk of 8 output channels), B (voxel, chunk of
         // 8 input channels) of the fragment order of mma.m16n8k16
-        const int av = (lane & 7) + ((lane >> 4) << 3), ac = (lane >> 3) & 1;
-        const int bv = (lane & 7) + (((lane >> 3) & 1) << 3), bc = lane >> 4;
+        const int av = (lane & 7) + ((lane >> 4) << 3), ac = 2 * mb + ((lane >> 3) & 1);
+        const int bv = (lane & 7) + (((lane >> 3) & 1) << 3), bc = 2 * nb + (lane >> 4);
+        // this warp's part of a plane: columns of 16 voxels kc0, kc0 + kstep .., `rows` rows from r0
+        const int ksteps = a.TW / 16, rparts = ksteps >= KQ ? 1 : KQ / ksteps, kparts = KQ / rparts;
+        const int kc0 = kq % kparts, rp = kq / kparts;
+        const int r0 = rp * a.TH / rparts, rows = rp < rparts ? (rp + 1) * a.TH / rparts - r0 : 0;
+        const uint32_t zpitch = a.TW * RZ, xpitch = P * RX, zo = swizzled<RZ>(av, ac) + r0 * zpitch;
+        const uint32_t xo[3] = {swizzled<RX>(bv, bc) + r0 * xpitch, swizzled<RX>(bv + 1, bc) + r0 * xpitch,
+                                swizzled<RX>(bv + 2, bc) + r0 * xpitch};
         int sx = 0, sz = 0;  // stages of X plane z - 1 and of dZ plane z
         uint32_t wx = 0, wz = 0;  // parities of the next X stage to wait for and of dZ
         int nwx = 0;              // next X stage to wait for
         const uint32_t xs0 = tc::smem_u32(xs), zs0 = tc::smem_u32(zs);
         bool ok = true;
-        for (long long u = blockIdx.x; u < a.units && ok; u += gridDim.x) {
-            int w0, h0, z0, zn, s;
-            unit(u, w0, h0, z0, zn, s);
+        int zn;
+        for (long long p = p0; p < p1 && ok; p += zn) {
+            int w0, h0, z0, s;
+            unit(p, w0, h0, z0, zn, s);
             for (int z = z0; z < z0 + zn; ++z) {
                 for (int q = z == z0 ? 0 : 2; q < 3 && ok; ++q) {
                     ok = tc::mbar_wait(fullx + nwx, wx) && !s_fail;
@@ -586,28 +624,13 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_mma_kernel(const __grid_c
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 const int sp = sx + dz < kWgXStages ? sx + dz : sx + dz - kWgXStages;
-                const uint32_t xp = xs0 + (uint32_t)(sp * a.xbytes), zp = zs0 + (uint32_t)(sz * a.zbytes);
-                for (int r = 0; r < a.TH; ++r) {
-                    const int zrow = r * a.TW, xrow = (r + dy) * P;
-#pragma unroll 2
-                    for (int k0 = 0; k0 < a.TW; k0 += 16) {
-                        uint32_t af[CO / 16][4];
-#pragma unroll
-                        for (int m = 0; m < CO / 16; ++m)
-                            ldmatrix_x4_trans(zp + swizzled<RZ>(zrow + k0 + av, 2 * m + ac), af[m]);
-#pragma unroll
-                        for (int t = 0; t < 3; ++t)
-#pragma unroll
-                            for (int n = 0; n < CI / 16; ++n) {
-                                uint32_t bf_[4];
-                                ldmatrix_x4_trans(xp + swizzled<RX>(xrow + k0 + t + bv, 2 * n + bc), bf_);
-#pragma unroll
-                                for (int m = 0; m < CO / 16; ++m) {
-                                    mma_16816(acc[t][m][2 * n], af[m], bf_[0], bf_[1]);
-                                    mma_16816(acc[t][m][2 * n + 1], af[m], bf_[2], bf_[3]);
-                                }
-                            }
-                    }
+                const uint32_t xp = xs0 + (uint32_t)(sp * a.xbytes), zp = zs0 + (uint32_t)(sz * a.zbytes) + zo;
+                for (int kc = kc0; kc < ksteps; kc += kparts) {
+                    const uint32_t zk = zp + kc * (16 * RZ), xb = xp + kc * (16 * RX);
+                    const uint32_t xk[3] = {xb + xo[0], xb + xo[1], xb + xo[2]};
+                    if (rows == 4) wgrad_rows<4>(acc, zk, xk, zpitch, xpitch);
+                    else if (rows == 2) wgrad_rows<2>(acc, zk, xk, zpitch, xpitch);
+                    else if (rows == 1) wgrad_rows<1>(acc, zk, xk, zpitch, xpitch);
                 }
                 __syncwarp();
                 // X plane z - 1 (and at the unit's end z and z + 1) and dZ plane z are free
@@ -622,25 +645,38 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_mma_kernel(const __grid_c
                 }
             }
         }
-        if (!ok) {
-            s_fail = 1;
-        } else {
-            const int g = lane >> 2, t4 = lane & 3;
-#pragma unroll
-            for (int t = 0; t < 3; ++t)
-#pragma unroll
-                for (int m = 0; m < CO / 16; ++m)
-#pragma unroll
-                    for (int n = 0; n < CI / 8; ++n)
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            const int co = cob * CO + m * 16 + g + (e >> 1) * 8;
-                            const int ci = cib * CI + n * 8 + 2 * t4 + (e & 1);
-                            atomicAdd(a.dw + ((size_t)co * a.cin + ci) * 27 + dz * 9 + dy * 3 + t, acc[t][m][n][e]);
-                        }
-        }
+        if (!ok) s_fail = 1;
     }
     __syncthreads();
+    // every load has landed and been read: the rings hold the sums, [co][ci][tap], the KQ warps
+    // of a block of 16 x 16 channels one after another
+    if (!s_fail) {
+        float* sum = reinterpret_cast<float*>(smem);
+        const int g = lane >> 2, t4 = lane & 3;
+        for (int q = 0; q < KQ; ++q) {
+            if (warp < kWgWarps && kq == q) {
+#pragma unroll
+                for (int dy = 0; dy < 3; ++dy)
+#pragma unroll
+                    for (int t = 0; t < 3; ++t)
+#pragma unroll
+                        for (int n = 0; n < 2; ++n)
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) {
+                                const int co = mb * 16 + g + (e >> 1) * 8, ci = nb * 16 + n * 8 + 2 * t4 + (e & 1);
+                                float* o = sum + (co * CI + ci) * 27 + dz * 9 + dy * 3 + t;
+                                *o = q == 0 ? acc[dy][t][n][e] : *o + acc[dy][t][n][e];
+                            }
+            }
+            __syncthreads();
+        }
+        // (rows of CI x 27 floats start on 16 bytes: the filters' offsets are multiples of 16)
+        for (int e = 4 * tid; e < CO * CI * 27; e += 4 * kWgThreads) {
+            const int co = e / (CI * 27), rest = e - co * (CI * 27);
+            atomicAdd(reinterpret_cast<float4*>(a.dw + ((size_t)(cob * CO + co) * a.cin + cib * CI) * 27 + rest),
+                      *reinterpret_cast<const float4*>(sum + e));
+        }
+    }
     if (s_fail && tid == 0) atomicExch(a.err, 2);
 }
 
