@@ -925,7 +925,7 @@ dim3 grid_col(const Dims& d, dim3 blk, int ni = kNI)
 constexpr int kNIbr = 2, kNIdv = 2;
 
 // Launch as a programmatic dependent of the previous kernel on the stream: the kernel
-// wait with griddepcontrol.wait before it reads what that kernel wrote, which holds it until
+// must wait with griddepcontrol.wait before it reads what that kernel wrote, which holds it until
 // the previous grid's writes are visible.
 template <typename... KArgs, typename... Args>
 int launch_dependent(im3d_ctx* ctx, void (*kern)(KArgs...), dim3 grid, dim3 blk, Args... args)
