@@ -4,7 +4,7 @@ levels. The gradient of two samples is the mean of their own gradients: every ac
 data gradient is the same BF16 number up to the factor 2 of the mean, and the weight gradients
 add the same products in other units and blocks. The FP32 accumulators may truncate at each of
 up to a few hundred additions per block (2^-24 each): 2e-5 relative per parameter tensor. The
-single-sample gradients are held to the CPU checker in test_gpu_unet.py."""
+single-sample gradients are held to the network on the CPU in test_gpu_unet.py."""
 import numpy as np
 import pytest
 
