@@ -85,9 +85,9 @@ struct View {
     int D, H, W, nsamp;
 };
 
-// Tensor map of a view for boxes of `chans` channels x bw x bh of one plane. Boxes of 8
-// channels are not swizzled, those of 16 and 32 with the swizzle of their 32 or 64 bytes.
-int make_map(const View& v, int chans, int bw, int bh, CUtensorMap* map, std::string& err)
+// Tensor map of a view for boxes of `chans` channels x bw x bh x depth. Boxes of 8 channels
+// are not swizzled, those of 16, 32 and 64 with the swizzle of their 32, 64 or 128 bytes.
+int make_map(const View& v, int chans, int bw, int bh, int depth, CUtensorMap* map, std::string& err)
 {
     auto fn = encode_fn();
     if (!fn) {
@@ -99,12 +99,14 @@ int make_map(const View& v, int chans, int bw, int bh, CUtensorMap* map, std::st
                           (cuuint64_t)v.nsamp};
     cuuint64_t strides[4] = {v.pitch * es, v.pitch * es * v.W, v.pitch * es * v.W * v.H,
                              v.pitch * es * v.W * v.H * v.D};
-    cuuint32_t box[5] = {(cuuint32_t)chans, (cuuint32_t)bw, (cuuint32_t)bh, 1, 1};
+    cuuint32_t box[5] = {(cuuint32_t)chans, (cuuint32_t)bw, (cuuint32_t)bh, (cuuint32_t)depth, 1};
     cuuint32_t estr[5] = {1, 1, 1, 1, 1};
     const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<bf16_t*>(v.p), dims, strides, box, estr,
                           CU_TENSOR_MAP_INTERLEAVE_NONE,
-                          chans == 8 ? CU_TENSOR_MAP_SWIZZLE_NONE
-                                     : (chans == 16 ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_64B),
+                          chans == 8    ? CU_TENSOR_MAP_SWIZZLE_NONE
+                          : chans == 16 ? CU_TENSOR_MAP_SWIZZLE_32B
+                          : chans == 32 ? CU_TENSOR_MAP_SWIZZLE_64B
+                                        : CU_TENSOR_MAP_SWIZZLE_128B,
                           CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) {
         err = "cuTensorMapEncodeTiled failed (" + std::to_string((int)r) + ")";
@@ -186,7 +188,7 @@ int conv_launch(cudaStream_t st, const View& x, int in_coff, const bf16_t* wpk, 
         return IM3D_ERR_UNSUPPORTED;
     }
     CUtensorMap map;
-    UN_TRY(make_map(x, 8, a.g.TW + 2, a.g.TH + 2, &map, err));
+    UN_TRY(make_map(x, 8, a.g.TW + 2, a.g.TH + 2, 1, &map, err));
     auto kern = conv3_march_kernel<CIN, NOUT, MODE>;
     UN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     a.wpk = wpk;
@@ -227,63 +229,74 @@ int conv_any(cudaStream_t st, int cin, int nout, const View& x, int in_coff, con
 // Output-channel block width for a layer.
 int nout_for(int cout) { return cout < 32 ? 16 : 32; }
 
-template <int CO, int CI>
-int wgrad_launch(cudaStream_t st, const View& x, int xcoff, int cin, const View& dz, int zcoff, int cout, float* dw,
-                 int* errf, std::string& err)
+// Tiles and blocks of the weight gradient's chains (wgrad_mma_kernel), which fix the order of
+// its sums. They follow the first form of this kernel, on tcgen05: tile rows TH of 8, 4, 2 or 1,
+// the most whose 8-channel regions of one plane of dZ and three of X fitted 220 KB (the 64-row A
+// operand reading 8 regions), and one chain per SM for each group of taps that its 512
+// accumulator columns held (27, 16 and 8 taps at 16, 32 and 64 input channels, the same number
+// of groups as blocks of 16 input channels here).
+bool wgrad_plan(int cin, int cout, int H, int TW, int* TH, int* chains)
 {
-    const int TWm = x.W <= 128 ? x.W : 128;
-    if (x.W % 16 != 0 || x.W % TWm != 0) {
+    const int P = TW + 2;
+    for (int th : {8, 4, 2, 1}) {
+        if (th > H && th > 1) continue;
+        const int rz = align_up((th + 2) * P * 16, 1024), rx = align_up(3 * (th + 2) * P * 16, 1024);
+        const int over = (8 - cout / 8) * rz - (cin / 8) * rx;
+        if ((cout / 8) * rz + (cin / 8) * rx + kGuardBytes + 64 + 1024 + std::max(over, 0) > 220 * 1024) continue;
+        *TH = th;
+        *chains = (g_num_sms + cin / 16 - 1) / (cin / 16);
+        return true;
+    }
+    return false;
+}
+
+template <int CO>
+int wgrad_launch(cudaStream_t st, const View& x, int xcoff, int cin, const View& dz, int zcoff, float* dw, int* errf,
+                 std::string& err)
+{
+    WgradArgs a;
+    a.TW = x.W <= 128 ? x.W : 128;
+    if (x.W % 16 != 0 || x.W % a.TW != 0) {
         err = "weight gradient: W must be a multiple of 16, and of 128 above 128";
         return IM3D_ERR_UNSUPPORTED;
     }
-    const int nblocks = (cout / CO) * (cin / CI);
-    const int ctas = std::max(1, g_num_sms / nblocks);
-    // four rows first, then the width: a plane of X carries two more rows and columns than its tile
-    for (int t = 0; t < 6; ++t) {
-        const int TH = 4 >> (t / 2), TW = t % 2 ? TWm / 2 : TWm;
-        if ((TH > x.H && TH > 1) || TW % 16 != 0) continue;
-        WgradArgs a;
-        a.xbytes = align_up((TH + 2) * (TW + 8) * 2 * CI, 1024);
-        a.zbytes = align_up(TH * TW * 2 * CO, 1024);
-        const int rings = kWgXStages * a.xbytes + kWgZStages * a.zbytes;
-        // the rings hold the sums of the block at the end
-        const int smem = 1024 + std::max(rings + 16 * (kWgXStages + kWgZStages), CO * CI * 27 * 4);
-        if (smem > 226 * 1024) continue;
-        a.D = x.D;
-        a.H = x.H;
-        a.W = x.W;
-        a.TH = TH;
-        a.TW = TW;
-        a.tiles_w = x.W / TW;
-        a.tiles_h = (x.H + TH - 1) / TH;
-        a.planes = (long long)x.nsamp * a.tiles_w * a.tiles_h * x.D;
-        a.zcoff = zcoff;
-        a.xcoff = xcoff;
-        a.cin = cin;
-        a.ciblocks = cin / CI;
-        a.dw = dw;
-        a.err = errf;
-        CUtensorMap xm, zm;
-        UN_TRY(make_map(x, CI, TW + 8, TH + 2, &xm, err));
-        UN_TRY(make_map(dz, CO, TW, TH, &zm, err));
-        auto kern = wgrad_mma_kernel<CO, CI>;
-        UN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        const long long gx = std::min<long long>(ctas, a.planes);
-        kern<<<dim3((unsigned)gx, (unsigned)nblocks), kWgThreads, smem, st>>>(xm, zm, a);
-        return launch_status(err, "wgrad_mma_kernel");
+    int chains = 0;
+    if (!wgrad_plan(cin, CO, x.H, a.TW, &a.TH, &chains)) {
+        err = "weight gradient: no tiling fits shared memory";
+        return IM3D_ERR_UNSUPPORTED;
     }
-    err = "weight gradient: no tiling fits shared memory";
-    return IM3D_ERR_UNSUPPORTED;
+    a.D = x.D;
+    a.H = x.H;
+    a.W = x.W;
+    a.tiles_w = x.W / a.TW;
+    a.tiles_h = (x.H + a.TH - 1) / a.TH;
+    a.ntiles = (long long)x.nsamp * x.D * a.tiles_h * a.tiles_w;
+    a.xbytes = 3 * (a.TW + 8) * 32;  // a multiple of 256, the repeat of its swizzle
+    a.zbytes = a.TW * 2 * CO;        // ... of 512 and more
+    a.zcoff = zcoff;
+    a.xcoff = xcoff;
+    a.cin = cin;
+    a.dw = dw;
+    a.err = errf;
+    const int rings = kWgXRows * a.xbytes + kWgZRows * a.zbytes + 16 * (kWgXRows + kWgZRows);
+    // the rings hold the sums of the block at the end
+    const int smem = 1024 + std::max(rings, CO * 16 * 27 * 4);
+    CUtensorMap xm, zm;
+    UN_TRY(make_map(x, 16, a.TW + 8, 1, 3, &xm, err));
+    UN_TRY(make_map(dz, CO, a.TW, 1, 1, &zm, err));
+    auto kern = wgrad_mma_kernel<CO>;
+    UN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    const long long gx = std::min<long long>(chains, a.ntiles);
+    kern<<<dim3((unsigned)gx, (unsigned)(cin / 16)), kWgThreads, smem, st>>>(xm, zm, a);
+    return launch_status(err, "wgrad_mma_kernel");
 }
 
-// Blocks of 16 or 32 output and input channels.
 int wgrad_any(cudaStream_t st, int cin, const View& x, int xcoff, const View& dz, int zcoff, int cout, float* dw,
               int* errf, std::string& err)
 {
-    if (cin == 16 && cout == 16) return wgrad_launch<16, 16>(st, x, xcoff, cin, dz, zcoff, cout, dw, errf, err);
-    if (cin == 16) return wgrad_launch<32, 16>(st, x, xcoff, cin, dz, zcoff, cout, dw, errf, err);
-    if (cout == 16) return wgrad_launch<16, 32>(st, x, xcoff, cin, dz, zcoff, cout, dw, errf, err);
-    return wgrad_launch<32, 32>(st, x, xcoff, cin, dz, zcoff, cout, dw, errf, err);
+    if (cout == 16) return wgrad_launch<16>(st, x, xcoff, cin, dz, zcoff, dw, errf, err);
+    if (cout == 32) return wgrad_launch<32>(st, x, xcoff, cin, dz, zcoff, dw, errf, err);
+    return wgrad_launch<64>(st, x, xcoff, cin, dz, zcoff, dw, errf, err);
 }
 
 int flat_blocks(long long n, int per = 256)

@@ -18,8 +18,9 @@
 // padded tile, N = the output channels of the launch (16 or 32) of the three output planes
 // that the input plane feeds, K = 16 input channels per instruction; the FP32 accumulators
 // live in TMEM and are drained by 4 warps (bias + ReLU or the ReLU mask of the data
-// gradient, BF16 store). The weight gradient (wgrad_mma_kernel) marches the same way with its
-// accumulators in registers (mma.sync: its M, the output channels, is 16 or 32).
+// gradient, BF16 store). The weight gradient (wgrad_mma_kernel) streams rows of the
+// activations and of the output's gradient, with its accumulators in registers (mma.sync: its M
+// fits 16 and 32 output channels).
 // Pooling, the 2x2x2 transposed convolutions, the 1x1 output layer, the loss and Adam
 // are small SIMT kernels.
 #pragma once
@@ -418,20 +419,19 @@ __global__ void __launch_bounds__(kMarchThreads, 1) conv3_march_kernel(const __g
 }
 
 // ---------------------------------------------------------------- weight gradient
-constexpr int kWgWarps = 12;                     // multiplying warps: 4 per dz
+constexpr int kWgWarps = 12;                     // multiplying warps
 constexpr int kWgThreads = 32 * (kWgWarps + 1);  // and one that loads
-constexpr int kWgXStages = 5, kWgZStages = 3;      // planes of X and of dZ in shared memory
+constexpr int kWgXRows = 8, kWgZRows = 5;        // rows of X (of three planes) and of dZ in shared memory
 
 struct WgradArgs {
-    int D, H, W;      // volume of one sample
-    int TH, TW;       // tile rows and columns (TW divides W, TW <= 128, a multiple of 16)
+    int D, H, W;       // volume of one sample
+    int TH, TW;        // tile rows and columns (TW divides W, TW <= 128, a multiple of 16)
     int tiles_w, tiles_h;
-    long long planes;  // nsamp * tiles_h * tiles_w * D, split evenly over the blocks
-    int xbytes, zbytes;  // a staged plane of X (halo included) and of dZ, multiples of 1024
+    long long ntiles;  // nsamp * D * tiles_h * tiles_w
+    int xbytes, zbytes;  // a staged row of X (three planes, halo included) and of dZ
     int zcoff, xcoff;    // first channel of dZ and of X in their tensors
     int cin;             // input channels of the layer
-    int ciblocks;        // blocks of CI input channels (blockIdx.y = output block * ciblocks + input block)
-    float* dw;           // FP32 gradient [cout][cin][27] (the parameter layout), accumulated with atomics
+    float* dw;           // FP32 gradient [CO][cin][27] (the parameter layout), accumulated with atomics
     int* err;
 };
 
@@ -451,81 +451,78 @@ __device__ __forceinline__ void mma_16816(float (&d)[4], const uint32_t (&a)[4],
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// Byte offset of 16-byte chunk c of row r in a plane of rows of ROW bytes that the TMA wrote
-// with its ROW-byte swizzle (32: chunk bit 0 ^ address bit 7; 64: chunk bits ^ bits 7, 8).
+// Byte offset of 16-byte chunk c of row r in rows of ROW bytes that the TMA wrote with its
+// ROW-byte swizzle (32: chunk bit 0 ^ address bit 7; 64: chunk bits ^ bits 7, 8; 128: ^ bits 7 to 9).
 template <int ROW>
 __device__ __forceinline__ uint32_t swizzled(int r, int c)
 {
-    return (uint32_t)(r * ROW + ((ROW == 32 ? c ^ ((r >> 2) & 1) : c ^ ((r >> 1) & 3)) << 4));
+    return (uint32_t)(r * ROW + ((ROW == 32 ? c ^ ((r >> 2) & 1) : ROW == 64 ? c ^ ((r >> 1) & 3) : c ^ (r & 7)) << 4));
 }
 
-// One step of a warp of wgrad_mma_kernel: 16 voxels of each of R rows of dZ against the R + 2
-// rows of X around them, for the nine (dy, dx) taps. zp, xp: addresses of this lane's ldmatrix
-// rows in the first row of dZ and of X (for each dx); zpitch, xpitch: bytes to the next row.
-template <int R>
-__device__ __forceinline__ void wgrad_rows(float (&acc)[3][3][2][4], uint32_t zp, const uint32_t (&xp)[3], uint32_t zpitch,
-                                           uint32_t xpitch)
+// The sums of one row of dZ by a warp: NT taps of 16 * MB output channels against 16 input
+// channels, 16 voxels per step along the row. zp: this lane's ldmatrix row per block of 16
+// output channels; xp: per tap.
+template <int NT, int MB, int RZ>
+__device__ __forceinline__ void wgrad_row(float (&acc)[3][MB][2][4], const uint32_t (&zp)[MB], const uint32_t (&xp)[3], int ksteps)
 {
-    uint32_t zf[R][4];
+#pragma unroll(MB == 4 ? 1 : 2)
+    for (int kc = 0; kc < ksteps; ++kc) {
+        uint32_t zf[MB][4], xf[NT][4];
 #pragma unroll
-    for (int h = 0; h < R + 2; ++h) {
-        uint32_t xf[3][4];
-        if (h < R) ldmatrix_x4_trans(zp + h * zpitch, zf[h < R ? h : 0]);
+        for (int m = 0; m < MB; ++m) ldmatrix_x4_trans(zp[m] + kc * (16 * RZ), zf[m]);
 #pragma unroll
-        for (int t = 0; t < 3; ++t) ldmatrix_x4_trans(xp[t] + h * xpitch, xf[t]);
+        for (int t = 0; t < NT; ++t) ldmatrix_x4_trans(xp[t] + kc * (16 * 32), xf[t]);
 #pragma unroll
-        for (int dy = 2; dy >= 0; --dy) {
-            if (h - dy < 0 || h - dy >= R) continue;
+        for (int t = 0; t < NT; ++t)
 #pragma unroll
-            for (int t = 0; t < 3; ++t)
+            for (int m = 0; m < MB; ++m)
 #pragma unroll
-                for (int n = 0; n < 2; ++n)
-                    mma_16816(acc[dy][t][n], zf[h - dy < 0 || h - dy >= R ? 0 : h - dy], xf[t][2 * n], xf[t][2 * n + 1]);
-        }
+                for (int n = 0; n < 2; ++n) mma_16816(acc[t][m][n], zf[m], xf[t][2 * n], xf[t][2 * n + 1]);
     }
 }
 
-// dW[co][ci][tap] = sum over voxels of dZ[v][co] X[v + tap][ci], for CO output and CI input
-// channels (blockIdx.y). The planes of all tiles are split evenly over the blocks; a block
-// marches along z: X planes and dZ planes stream through rings in shared memory (TMA), each X
-// plane serving three output planes. A warp holds the sums of 16 x 16 channels for the nine
-// (dy, dx) taps of one dz in registers, over all its planes; the four warps of a dz (one per
-// scheduler, so that the tensor pipes are loaded alike) take the blocks of 16 x 16 channels and,
-// where these are fewer than four, shares of the voxels. The block's sums are joined in shared
-// memory and added to the gradient once, 16 bytes per atomic.
-// The products run on mma.sync (M = 16 output channels, N = 8 input channels, K = 16 voxels):
-// both operands are read transposed from channels-last rows by ldmatrix, and M = 16 fits 16
-// and 32 channels exactly, where tcgen05's smallest M (64) multiplies three quarters or half
-// of it for nothing and needs one MMA per tap of 16 or 32 columns.
-// What bounds it: the tensor pipe, about 8 cycles per mma.sync of a scheduler, 50 to 75 % of
-// the time; staging alone takes 48 of 90 us. us against one warp per (dz, dy), which left one
-// scheduler with half more to do than the others, read each X fragment three times from shared
-// memory and ran whole columns per block on 128 of 148 SMs: 16 x 16 at 128^3 130 -> 90,
-// 16 x 32 at 128^3 227 -> 157, 32 x 32 at 64^3 80 -> 48, 32 x 16 at 64^3 51 -> 32 (the tcgen05
-// form, M = 64, N = CI, load and multiply in turn: 929, 950, 420).
-template <int CO, int CI>
+// dW[co][ci][tap] = sum over voxels of dZ[v][co] X[v + tap][ci], for all CO output channels and
+// 16 input channels (blockIdx.y).
+// The order of the sums is part of the result: the tensor core's FP32 accumulator truncates, so
+// that another order moves the gradient by up to 6e-5 (2 x 128 x 128 x 256), and a training run
+// with it. Every (co, ci, tap) is one chain of multiplications of 16 voxels each: block
+// blockIdx.x takes the tiles blockIdx.x, blockIdx.x + gridDim.x, ... (columns, rows, planes,
+// samples, the first fastest) row by row, 16 voxels after 16 along a row, and the blocks' sums
+// are added to the gradient with one atomic each. The host's plan (wgrad_plan) fixes the
+// tiles and the number of blocks.
+// Rows stream through rings in shared memory (TMA): a row of X of the three planes around the
+// tile's, and a row of dZ. The 27 taps are spread over 12 warps, three to the first three, two to
+// the others (7, 7, 7 and 6 per scheduler), each with its sums in registers throughout.
+// The products run on mma.sync (M = 16 output channels, N = 8 input channels, K = 16 voxels),
+// which gives the bits of tcgen05.mma for the same chain: both operands are read transposed from
+// channels-last rows by ldmatrix, and M = 16 fits 16 and 32 channels exactly, where tcgen05's
+// smallest M (64) multiplies three quarters or half of it for nothing.
+// us (output x input channels): 16 x 16 at 128^3 124, 16 x 32 at 128^3 261, 32 x 32 at 64^3 60,
+// 32 x 16 at 64^3 37; the same chains on tcgen05, load and multiply in turn: 929, 950, 420 for
+// the first three. Consecutive tiles of a chain lie in other rows and planes, so X is read for each of
+// its three planes anew; chains marching along z (90, 157, 48, 32 us) are other sums.
+template <int CO>
 __global__ void __launch_bounds__(kWgThreads, 1) wgrad_mma_kernel(const __grid_constant__ CUtensorMap xmap,
                                                                   const __grid_constant__ CUtensorMap zmap,
                                                                   const __grid_constant__ WgradArgs a)
 {
-    constexpr int RX = 2 * CI, RZ = 2 * CO;  // bytes of a row (one voxel)
-    constexpr int MB = CO / 16, NB = CI / 16, KQ = 4 / (MB * NB);
+    constexpr int CI = 16, RX = 2 * CI, RZ = 2 * CO, MB = CO / 16;  // RX, RZ: bytes of a voxel
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    unsigned char* xs = smem;
-    unsigned char* zs = xs + kWgXStages * a.xbytes;
-    uint64_t* fullx = reinterpret_cast<uint64_t*>(zs + kWgZStages * a.zbytes);
-    uint64_t* emptyx = fullx + kWgXStages;
-    uint64_t* fullz = emptyx + kWgXStages;
-    uint64_t* emptyz = fullz + kWgZStages;
+    unsigned char* zs = smem;
+    unsigned char* xs = zs + kWgZRows * a.zbytes;
+    uint64_t* fullx = reinterpret_cast<uint64_t*>(xs + kWgXRows * a.xbytes);
+    uint64_t* emptyx = fullx + kWgXRows;
+    uint64_t* fullz = emptyx + kWgXRows;
+    uint64_t* emptyz = fullz + kWgZRows;
     __shared__ volatile int s_fail;
     if (tid == 0) {
-        for (int q = 0; q < kWgXStages; ++q) {
+        for (int q = 0; q < kWgXRows; ++q) {
             tc::mbar_init(fullx + q, 1);
             tc::mbar_init(emptyx + q, kWgWarps);
         }
-        for (int q = 0; q < kWgZStages; ++q) {
+        for (int q = 0; q < kWgZRows; ++q) {
             tc::mbar_init(fullz + q, 1);
             tc::mbar_init(emptyz + q, kWgWarps);
         }
@@ -533,52 +530,52 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_mma_kernel(const __grid_c
         s_fail = 0;
     }
     __syncthreads();
-    const int cob = blockIdx.y / a.ciblocks, cib = blockIdx.y % a.ciblocks;
+    const int cib = blockIdx.y;
     const int P = a.TW + 8;  // voxels of a staged row of X: a multiple of 8 keeps the swizzle's phase
-    // multiplying warp: filter plane dz, block (mb, nb) of 16 x 16 channels, share kq of the voxels
-    const int dz = warp / 4, mb = warp % 4 % MB, nb = warp % 4 / MB % NB, kq = warp % 4 / (MB * NB);
-    float acc[3][3][2][4];  // [dy][dx][8 input channels]
+    float acc[3][MB][2][4];  // [this warp's taps][16 output channels][8 input channels]
 #pragma unroll
-    for (int e = 0; e < 72; ++e) (&acc[0][0][0][0])[e] = 0.f;
-    // this block's planes, and the column (tile) and planes of it that start at plane p
-    const long long p0 = a.planes * blockIdx.x / gridDim.x, p1 = a.planes * (blockIdx.x + 1) / gridDim.x;
-    auto unit = [&](long long p, int& w0, int& h0, int& z0, int& zn, int& s) {
-        long long c = p / a.D;
-        z0 = (int)(p - c * a.D);
-        zn = (int)min((long long)(a.D - z0), p1 - p);
-        w0 = (int)(c % a.tiles_w) * a.TW;
-        c /= a.tiles_w;
-        h0 = (int)(c % a.tiles_h) * a.TH;
-        s = (int)(c / a.tiles_h);
+    for (int t = 0; t < 3; ++t)
+#pragma unroll
+        for (int m = 0; m < MB; ++m)
+#pragma unroll
+            for (int e = 0; e < 8; ++e) acc[t][m][e >> 2][e & 3] = 0.f;
+    // a tile's first column and row, its rows inside the volume, plane and sample
+    auto place = [&](long long r, int& w0, int& h0, int& rows, int& z, int& s) {
+        w0 = (int)(r % a.tiles_w) * a.TW;
+        r /= a.tiles_w;
+        h0 = (int)(r % a.tiles_h) * a.TH;
+        r /= a.tiles_h;
+        z = (int)(r % a.D);
+        s = (int)(r / a.D);
+        rows = min(a.TH, a.H - h0);
     };
     if (warp == kWgWarps) {
         if (lane == 0) {
-            const uint32_t xb = (uint32_t)((a.TH + 2) * P * RX), zb = (uint32_t)(a.TH * a.TW * RZ);
-            int sx = 0, sz = 0, nx = 0, nzl = 0;  // next stages, loads issued (up to the stages)
-            uint32_t phx = 1, phz = 1;            // parity of a free stage: the first pass finds them free
+            const uint32_t xb = (uint32_t)(3 * P * RX), zb = (uint32_t)(a.TW * RZ);
+            int sx = 0, sz = 0, nx = 0, nzl = 0;  // next slots, loads issued (up to the slots)
+            uint32_t phx = 1, phz = 1;            // parity of a free slot: the first pass finds them free
             bool ok = true;
-            int zn;
-            for (long long p = p0; p < p1 && ok; p += zn) {
-                int w0, h0, z0, s;
-                unit(p, w0, h0, z0, zn, s);
-                // X planes z0 - 1 .. z0 + zn; the dZ plane z goes out with the X plane z + 1
-                for (int z = z0 - 1; z <= z0 + zn && ok; ++z) {
+            for (long long tile = blockIdx.x; tile < a.ntiles && ok; tile += gridDim.x) {
+                int w0, h0, rows, z, s;
+                place(tile, w0, h0, rows, z, s);
+                // X rows h0 - 1 .. h0 + rows; the dZ row h goes out with the X row h + 1
+                for (int j = 0; j < rows + 2 && ok; ++j) {
                     ok = tc::mbar_wait(emptyx + sx, phx) && !s_fail;
                     if (!ok) break;
                     tc::mbar_arrive_expect_tx(fullx + sx, xb);
-                    tc::tma_load_5d(xs + sx * a.xbytes, &xmap, fullx + sx, a.xcoff + cib * CI, w0 - 1, h0 - 1, z, s);
-                    nx = min(nx + 1, kWgXStages);
-                    if (++sx == kWgXStages) {
+                    tc::tma_load_5d(xs + sx * a.xbytes, &xmap, fullx + sx, a.xcoff + cib * CI, w0 - 1, h0 - 1 + j, z - 1, s);
+                    nx = min(nx + 1, kWgXRows);
+                    if (++sx == kWgXRows) {
                         sx = 0;
                         phx ^= 1u;
                     }
-                    if (z <= z0) continue;
+                    if (j < 2) continue;
                     ok = tc::mbar_wait(emptyz + sz, phz) && !s_fail;
                     if (!ok) break;
                     tc::mbar_arrive_expect_tx(fullz + sz, zb);
-                    tc::tma_load_5d(zs + sz * a.zbytes, &zmap, fullz + sz, a.zcoff + cob * CO, w0, h0, z - 1, s);
-                    nzl = min(nzl + 1, kWgZStages);
-                    if (++sz == kWgZStages) {
+                    tc::tma_load_5d(zs + sz * a.zbytes, &zmap, fullz + sz, a.zcoff, w0, h0 + j - 2, z, s);
+                    nzl = min(nzl + 1, kWgZRows);
+                    if (++sz == kWgZRows) {
                         sz = 0;
                         phz ^= 1u;
                     }
@@ -594,28 +591,30 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_mma_kernel(const __grid_c
     } else {
         // ldmatrix rows of this lane: A (voxel, chunk of 8 output channels), B (voxel, chunk of
         // 8 input channels) of the fragment order of mma.m16n8k16
-        const int av = (lane & 7) + ((lane >> 4) << 3), ac = 2 * mb + ((lane >> 3) & 1);
-        const int bv = (lane & 7) + (((lane >> 3) & 1) << 3), bc = 2 * nb + (lane >> 4);
-        // this warp's part of a plane: columns of 16 voxels kc0, kc0 + kstep .., `rows` rows from r0
-        const int ksteps = a.TW / 16, rparts = ksteps >= KQ ? 1 : KQ / ksteps, kparts = KQ / rparts;
-        const int kc0 = kq % kparts, rp = kq / kparts;
-        const int r0 = rp * a.TH / rparts, rows = rp < rparts ? (rp + 1) * a.TH / rparts - r0 : 0;
-        const uint32_t zpitch = a.TW * RZ, xpitch = P * RX, zo = swizzled<RZ>(av, ac) + r0 * zpitch;
-        const uint32_t xo[3] = {swizzled<RX>(bv, bc) + r0 * xpitch, swizzled<RX>(bv + 1, bc) + r0 * xpitch,
-                                swizzled<RX>(bv + 2, bc) + r0 * xpitch};
-        int sx = 0, sz = 0;  // stages of X plane z - 1 and of dZ plane z
-        uint32_t wx = 0, wz = 0;  // parities of the next X stage to wait for and of dZ
-        int nwx = 0;              // next X stage to wait for
-        const uint32_t xs0 = tc::smem_u32(xs), zs0 = tc::smem_u32(zs);
+        const int av = (lane & 7) + ((lane >> 4) << 3), ac = (lane >> 3) & 1;
+        const int bv = (lane & 7) + (((lane >> 3) & 1) << 3), bc = lane >> 4;
+        uint32_t zo[MB], xo[3];
+        int dy[3];
+#pragma unroll
+        for (int m = 0; m < MB; ++m) zo[m] = tc::smem_u32(zs) + swizzled<RZ>(av, 2 * m + ac);
+#pragma unroll
+        for (int t = 0; t < 3; ++t) {
+            const int tap = min(warp + t * kWgWarps, 26);  // dz * 9 + dy * 3 + dx
+            dy[t] = tap / 3 % 3;
+            xo[t] = tc::smem_u32(xs) + (uint32_t)(tap / 9 * P * RX) + swizzled<RX>(bv + tap % 3, bc);
+        }
+        const int ksteps = a.TW / 16;
+        int sx = 0, sz = 0;       // slots of X row h - 1 and of dZ row h
+        uint32_t wx = 0, wz = 0;  // parities of the next X slot to wait for and of dZ
+        int nwx = 0;              // next X slot to wait for
         bool ok = true;
-        int zn;
-        for (long long p = p0; p < p1 && ok; p += zn) {
-            int w0, h0, z0, s;
-            unit(p, w0, h0, z0, zn, s);
-            for (int z = z0; z < z0 + zn; ++z) {
-                for (int q = z == z0 ? 0 : 2; q < 3 && ok; ++q) {
+        for (long long tile = blockIdx.x; tile < a.ntiles && ok; tile += gridDim.x) {
+            int w0, h0, rows, z, s;
+            place(tile, w0, h0, rows, z, s);
+            for (int r = 0; r < rows; ++r) {
+                for (int q = r == 0 ? 0 : 2; q < 3 && ok; ++q) {
                     ok = tc::mbar_wait(fullx + nwx, wx) && !s_fail;
-                    if (++nwx == kWgXStages) {
+                    if (++nwx == kWgXRows) {
                         nwx = 0;
                         wx ^= 1u;
                     }
@@ -623,23 +622,24 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_mma_kernel(const __grid_c
                 ok = ok && tc::mbar_wait(fullz + sz, wz) && !s_fail;
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
-                const int sp = sx + dz < kWgXStages ? sx + dz : sx + dz - kWgXStages;
-                const uint32_t xp = xs0 + (uint32_t)(sp * a.xbytes), zp = zs0 + (uint32_t)(sz * a.zbytes) + zo;
-                for (int kc = kc0; kc < ksteps; kc += kparts) {
-                    const uint32_t zk = zp + kc * (16 * RZ), xb = xp + kc * (16 * RX);
-                    const uint32_t xk[3] = {xb + xo[0], xb + xo[1], xb + xo[2]};
-                    if (rows == 4) wgrad_rows<4>(acc, zk, xk, zpitch, xpitch);
-                    else if (rows == 2) wgrad_rows<2>(acc, zk, xk, zpitch, xpitch);
-                    else if (rows == 1) wgrad_rows<1>(acc, zk, xk, zpitch, xpitch);
+                uint32_t zp[MB], xp[3];
+#pragma unroll
+                for (int m = 0; m < MB; ++m) zp[m] = zo[m] + (uint32_t)(sz * a.zbytes);
+#pragma unroll
+                for (int t = 0; t < 3; ++t) {
+                    const int q = sx + dy[t] < kWgXRows ? sx + dy[t] : sx + dy[t] - kWgXRows;
+                    xp[t] = xo[t] + (uint32_t)(q * a.xbytes);
                 }
+                if (warp < 27 - 2 * kWgWarps) wgrad_row<3, MB, RZ>(acc, zp, xp, ksteps);
+                else wgrad_row<2, MB, RZ>(acc, zp, xp, ksteps);
                 __syncwarp();
-                // X plane z - 1 (and at the unit's end z and z + 1) and dZ plane z are free
-                for (int q = 0; q < (z == z0 + zn - 1 ? 3 : 1); ++q) {
+                // X row h - 1 (and at the tile's end h and h + 1) and dZ row h are free
+                for (int q = 0; q < (r == rows - 1 ? 3 : 1); ++q) {
                     if (lane == 0) tc::mbar_arrive(emptyx + sx);
-                    if (++sx == kWgXStages) sx = 0;
+                    if (++sx == kWgXRows) sx = 0;
                 }
                 if (lane == 0) tc::mbar_arrive(emptyz + sz);
-                if (++sz == kWgZStages) {
+                if (++sz == kWgZRows) {
                     sz = 0;
                     wz ^= 1u;
                 }
@@ -648,32 +648,29 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_mma_kernel(const __grid_c
         if (!ok) s_fail = 1;
     }
     __syncthreads();
-    // every load has landed and been read: the rings hold the sums, [co][ci][tap], the KQ warps
-    // of a block of 16 x 16 channels one after another
+    // every load has landed and been read: the rings hold the block's sums, [co][ci][tap]
     if (!s_fail) {
         float* sum = reinterpret_cast<float*>(smem);
         const int g = lane >> 2, t4 = lane & 3;
-        for (int q = 0; q < KQ; ++q) {
-            if (warp < kWgWarps && kq == q) {
+        if (warp < kWgWarps) {
 #pragma unroll
-                for (int dy = 0; dy < 3; ++dy)
+            for (int t = 0; t < 3; ++t) {
+                const int tap = warp + t * kWgWarps;
+                if (tap > 26) continue;
 #pragma unroll
-                    for (int t = 0; t < 3; ++t)
+                for (int m = 0; m < MB; ++m)
 #pragma unroll
-                        for (int n = 0; n < 2; ++n)
-#pragma unroll
-                            for (int e = 0; e < 4; ++e) {
-                                const int co = mb * 16 + g + (e >> 1) * 8, ci = nb * 16 + n * 8 + 2 * t4 + (e & 1);
-                                float* o = sum + (co * CI + ci) * 27 + dz * 9 + dy * 3 + t;
-                                *o = q == 0 ? acc[dy][t][n][e] : *o + acc[dy][t][n][e];
-                            }
+                    for (int e = 0; e < 8; ++e) {
+                        const int co = m * 16 + g + ((e >> 1) & 1) * 8, ci = (e >> 2) * 8 + 2 * t4 + (e & 1);
+                        sum[(co * CI + ci) * 27 + tap] = acc[t][m][e >> 2][e & 3];
+                    }
             }
-            __syncthreads();
         }
+        __syncthreads();
         // (rows of CI x 27 floats start on 16 bytes: the filters' offsets are multiples of 16)
         for (int e = 4 * tid; e < CO * CI * 27; e += 4 * kWgThreads) {
             const int co = e / (CI * 27), rest = e - co * (CI * 27);
-            atomicAdd(reinterpret_cast<float4*>(a.dw + ((size_t)(cob * CO + co) * a.cin + cib * CI) * 27 + rest),
+            atomicAdd(reinterpret_cast<float4*>(a.dw + ((size_t)co * a.cin + cib * CI) * 27 + rest),
                       *reinterpret_cast<const float4*>(sum + e));
         }
     }
