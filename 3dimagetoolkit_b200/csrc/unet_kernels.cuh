@@ -963,11 +963,14 @@ __global__ void __launch_bounds__(128) upconv_bwd_kernel(const bf16_t* __restric
 // Weight and bias gradient of the transposed convolution:
 //   dU[o][ci][co] += sum_p in[p][ci] g_out[child(p, o)][co],  db[co] += sum g_out[.][co],
 // as products of M = 16 input channels, N = 8 output channels and K = 16 coarse voxels on
-// mma.sync with FP32 accumulators in registers; warp o takes child o. A block stages 64
-// coarse voxels (4 row segments of 16) and their 512 children at a time, two stages ahead of
-// each other, in rows padded by 16 bytes (ldmatrix reads 8 rows on distinct banks), and adds
-// its sums once. (One scalar product per thread and voxel took 550 us for 32 -> 16 channels at
-// 128^3.)
+// mma.sync; warp o takes child o. A block stages 64 coarse voxels (4 row segments of 16) and
+// their 512 children at a time, two stages ahead of each other, in rows padded by 16 bytes
+// (ldmatrix reads 8 rows on distinct banks), and adds its sums once. (One scalar product per
+// thread and voxel took 550 us for 32 -> 16 channels at 128^3, this 30.)
+// The tensor core's accumulator truncates, so it holds one stage only (4 multiplications); the
+// stages are joined by FP32 additions that round to nearest. Error of up1's gradient against
+// FP64 sums at 128^3 / 2 x 128 x 128 x 256: 2.6e-7 / 2.7e-7 (one accumulator over all
+// stages 2.4e-6 / 6.3e-6; scalar products 1.1e-6 / 1.0e-6).
 template <int CI, int CO>
 struct UpWgrad {
     static constexpr int TP = 64, RI = 2 * CI + 16, RG = 2 * CO + 16;      // voxels, row bytes
@@ -1030,26 +1033,45 @@ __global__ void __launch_bounds__(256) upconv_wgrad_kernel(const bf16_t* __restr
         }
         __syncthreads();
         const uint32_t bi = tc::smem_u32(sm + s * G::stage), bg = bi + TP * RI + (uint32_t)(o * TP * RG);
+        uint32_t gf[TP / 16][CO / 16][4];
 #pragma unroll
-        for (int k0 = 0; k0 < TP; k0 += 16) {
-            uint32_t af[CI / 16][4];
+        for (int n = 0; n < CO / 16; ++n) {
+            float b0 = 0.f, b1 = 0.f;  // this lane's share of the bias sums: channel lane / 4 of each 8
 #pragma unroll
-            for (int m = 0; m < CI / 16; ++m)
-                ldmatrix_x4_trans(bi + (uint32_t)((k0 + av) * RI + (2 * m + ac) * 16), af[m]);
-#pragma unroll
-            for (int n = 0; n < CO / 16; ++n) {
-                uint32_t gf[4];
-                ldmatrix_x4_trans(bg + (uint32_t)((k0 + bv) * RG + (2 * n + bc) * 16), gf);
-#pragma unroll
-                for (int m = 0; m < CI / 16; ++m) {
-                    mma_16816(acc[m][2 * n], af[m], gf[0], gf[1]);
-                    mma_16816(acc[m][2 * n + 1], af[m], gf[2], gf[3]);
-                }
-                // this lane's share of the bias sums: channel lane / 4 of each 8, 4 voxels
-#pragma unroll
-                for (int h = 0; h < 4; ++h)
-                    bs[2 * n + (h >> 1)] += __uint_as_float(gf[h] << 16) + __uint_as_float(gf[h] & 0xffff0000u);
+            for (int k = 0; k < TP / 16; ++k) {
+                uint32_t(&f)[4] = gf[k][n];
+                ldmatrix_x4_trans(bg + (uint32_t)((16 * k + bv) * RG + (2 * n + bc) * 16), f);
+                auto four = [](uint32_t u, uint32_t v) {
+                    return (__uint_as_float(u << 16) + __uint_as_float(u & 0xffff0000u)) +
+                           (__uint_as_float(v << 16) + __uint_as_float(v & 0xffff0000u));
+                };
+                b0 += four(f[0], f[1]);
+                b1 += four(f[2], f[3]);
             }
+            bs[2 * n] += b0;
+            bs[2 * n + 1] += b1;
+        }
+#pragma unroll
+        for (int m = 0; m < CI / 16; ++m) {
+            float part[CO / 8][4];
+#pragma unroll
+            for (int n = 0; n < CO / 8; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) part[n][e] = 0.f;
+#pragma unroll
+            for (int k = 0; k < TP / 16; ++k) {
+                uint32_t af[4];
+                ldmatrix_x4_trans(bi + (uint32_t)((16 * k + av) * RI + (2 * m + ac) * 16), af);
+#pragma unroll
+                for (int n = 0; n < CO / 16; ++n) {
+                    mma_16816(part[2 * n], af, gf[k][n][0], gf[k][n][1]);
+                    mma_16816(part[2 * n + 1], af, gf[k][n][2], gf[k][n][3]);
+                }
+            }
+#pragma unroll
+            for (int n = 0; n < CO / 8; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[m][n][e] += part[n][e];
         }
         __syncthreads();
     }
@@ -1063,11 +1085,20 @@ __global__ void __launch_bounds__(256) upconv_wgrad_kernel(const bf16_t* __restr
                 const int ci = m * 16 + g + (e >> 1) * 8, co = n * 8 + 2 * t4 + (e & 1);
                 atomicAdd(dU + (o * CI + ci) * CO + co, acc[m][n][e]);
             }
+    // the children's bias sums are joined in shared memory (every stage has been read)
+    float(*bsum)[CO] = reinterpret_cast<float(*)[CO]>(sm);
 #pragma unroll
     for (int n = 0; n < CO / 8; ++n) {
         bs[n] += __shfl_xor_sync(0xffffffffu, bs[n], 1);
         bs[n] += __shfl_xor_sync(0xffffffffu, bs[n], 2);
-        if (t4 == 0) atomicAdd(db + n * 8 + g, bs[n]);
+        if (t4 == 0) bsum[o][n * 8 + g] = bs[n];
+    }
+    __syncthreads();
+    if (tid < CO) {
+        float t = 0.f;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) t += bsum[c][tid];
+        atomicAdd(db + tid, t);
     }
 }
 
