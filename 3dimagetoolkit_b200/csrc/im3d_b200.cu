@@ -836,8 +836,11 @@ int lex_sweeps(im3d_ctx* ctx, T* r, const T* b, const Dims& d, const GsCoef<T>& 
         const int key[4] = {a.nti, a.ntj, a.ntk, ns};
         unsigned long long* tasks = nullptr;
         const size_t count = (size_t)nt * ns;
+        // the old list's buffer may be gone from here on, also when this call fails
+        const bool known = std::memcmp(key, ctx->lex_key, sizeof key) == 0;
+        if (!known) ctx->lex_key[0] = 0;
         IM3D_TRY(tbuf<unsigned long long>(ctx, "lex_tasks", count, &tasks));
-        if (std::memcmp(key, ctx->lex_key, sizeof key) != 0) {
+        if (!known) {
             // counting sort of (tile, sweep) by i + j + k + 2 sweep
             const int levels = a.nti + a.ntj + a.ntk - 2 + 2 * (ns - 1);
             std::vector<size_t> at(levels + 1, 0);
@@ -856,7 +859,6 @@ int lex_sweeps(im3d_ctx* ctx, T* r, const T* b, const Dims& d, const GsCoef<T>& 
                 if (pass == 0)
                     for (int l = 0; l < levels; ++l) at[l + 1] += at[l];
             }
-            ctx->lex_key[0] = 0;  // no list while the copy can fail
             IM3D_CUDA(ctx, cudaMemcpyAsync(tasks, list.data(), count * sizeof(unsigned long long),
                                            cudaMemcpyHostToDevice, ctx->stream));
             IM3D_TRY(sync(ctx));  // the list must outlive the copy

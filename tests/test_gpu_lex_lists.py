@@ -1,0 +1,47 @@
+"""GPU: the task list of the lexicographic sweeps (lex_tile_kernel), which the context keeps from
+call to call. Sweeps in FP64 are bit-exact against the oracle's sequential loops."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+
+
+def _case(shape, seed):
+    rng = np.random.default_rng(seed)
+    return rng.standard_normal(shape), rng.standard_normal(shape)
+
+
+def _sweep(c, u, b, sweeps, **kw):
+    """The sweeps on device arrays (the context then needs no buffers of its own for them)."""
+    du, db = torch.from_numpy(u.copy()).cuda(), torch.from_numpy(b).cuda()
+    torch.cuda.synchronize()
+    c.poisson_sweeps(du, db, sweeps=sweeps, **kw)
+    return du.cpu().numpy()
+
+
+def test_list_after_a_failed_allocation(pkg, O):
+    """A larger list that finds no device memory costs the context its old list: the next call of
+    the old size must write its list again (it took whatever the new buffer held)."""
+    u, b = _case((40, 37, 52), 3)
+    want = O.poisson_sweeps(u, b, dt=1.0, bc=0.0, bc_type=pkg.BC_DIR, sweeps=3, h=(1.0, 1.0, 1.0))
+    big = torch.zeros((258, 258, 258), device="cuda")
+    with pkg.Context(0) as c:
+        c.poisson_sweeps(big, big.clone(), sweeps=1)
+        first = _sweep(c, u, b, 3)
+        # 4096 tiles x 512 sweeps: a list of 16 MB, with 6 MB left on the device
+        rhs = big.clone()
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        free = torch.cuda.mem_get_info()[0]
+        hold = torch.empty(free - (6 << 20), dtype=torch.uint8, device="cuda")
+        try:
+            c.poisson_sweeps(big, rhs, sweeps=512)
+        except pkg.Im3dError as e:
+            assert e.status == 5  # out of memory
+        del hold
+        torch.cuda.empty_cache()
+        again = _sweep(c, u, b, 3)
+    assert np.array_equal(first, want)
+    assert np.array_equal(again, want)
