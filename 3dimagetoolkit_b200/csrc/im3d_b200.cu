@@ -13,6 +13,7 @@
 #include <chrono>
 #include <cstring>
 #include <mutex>
+#include <new>
 #include <string>
 #include <thread>
 #include <unordered_map>
@@ -36,6 +37,8 @@ using namespace im3d;
 #ifndef IM3D_UNIT
 #define IM3D_UNIT 0
 #endif
+
+constexpr const char* kLexLists = "lex_lists";  // buffer of the lexicographic sweeps' task list
 
 struct DevBuf {
     void* p = nullptr;
@@ -82,7 +85,7 @@ struct im3d_ctx {
     int num_sms = 148;
     signed char cluster_ok[8] = {};  // rb_cluster_kernel per type and rule: 0 not asked, 1 can run, -1 cannot
     size_t smem_optin = 0;           // shared memory a block may ask for
-    int lex_key[4] = {0, 0, 0, 0};  // tile counts and sweeps of the lexicographic task list held in "lex_tasks"
+    int lex_key[4] = {0, 0, 0, 0};  // tile counts and sweeps of the lexicographic task list held in kLexLists
     int ifit_chunks = 0;  // i chunks of the marching fit stage (0: cost model)
     size_t mem_limit = 0;  // device bytes the context may hold in buffers (0: no limit)
     size_t mem_held = 0;   // device bytes it holds in buffers now
@@ -206,14 +209,31 @@ void prof_resolve(im3d_ctx* ctx)
     if (all) ctx->pending.clear();
 }
 
-// Device buffer of at least `bytes` under `name`, reused across calls.
+// Gives up the task list of the lexicographic sweeps, which work without it (lex_sweeps);
+// false when none is held.
+bool release_lists(im3d_ctx* ctx)
+{
+    auto it = ctx->bufs.find(kLexLists);
+    if (it == ctx->bufs.end() || !it->second.p) return false;
+    cudaFree(it->second.p);
+    ctx->mem_held -= it->second.bytes;
+    it->second = DevBuf();
+    ctx->lex_key[0] = 0;
+    return true;
+}
+
+// Device buffer of at least `bytes` under `name`, reused across calls. Where the memory for it
+// is short, the task list of the lexicographic sweeps gives way first.
 int buf(im3d_ctx* ctx, const char* name, size_t bytes, void** out, bool zero = false)
 {
     DevBuf& b = ctx->bufs[name];
     if (b.bytes < bytes) {
         // the context's memory budget (IM3D_OPT_DEVICE_MEMORY_LIMIT) is checked before
-        // anything is freed or allocated
-        if (ctx->mem_limit && ctx->mem_held - b.bytes + bytes > ctx->mem_limit) {
+        // anything else is freed or allocated
+        auto over = [&]() { return ctx->mem_limit && ctx->mem_held - b.bytes + bytes > ctx->mem_limit; };
+        const bool lists = std::strcmp(name, kLexLists) == 0;
+        if (over() && !lists) release_lists(ctx);
+        if (over()) {
             ctx->err = std::string("device memory limit of the context (") +
                        std::to_string(ctx->mem_limit) + " bytes) reached: buffer " + name + " needs " +
                        std::to_string(bytes) + " bytes, " + std::to_string(ctx->mem_held - b.bytes) +
@@ -225,8 +245,13 @@ int buf(im3d_ctx* ctx, const char* name, size_t bytes, void** out, bool zero = f
         b.p = nullptr;
         b.bytes = 0;
         cudaError_t e = cudaMalloc(&b.p, bytes);
+        if (e != cudaSuccess && !lists && release_lists(ctx)) {
+            cudaGetLastError();
+            e = cudaMalloc(&b.p, bytes);
+        }
         if (e != cudaSuccess) {
             cudaGetLastError();
+            b.p = nullptr;
             ctx->err = std::string("cudaMalloc(") + name + ", " + std::to_string(bytes) +
                        " bytes): " + cudaGetErrorString(e);
             return IM3D_ERR_OOM;
@@ -797,9 +822,78 @@ HStep<T> make_hstep(double hx, double hy, double hz)
     return s;
 }
 
-// Lexicographic sweeps, reference order, natural layout, in place (lex_tile_kernel). The
-// task list depends on the tile counts and the number of sweeps only; the context keeps the
-// last one. A wait that gave up raises ctrl flag 1.
+// The task list and the tiles' counters of `ns` sweeps (lex_tile_kernel), in one buffer. The list
+// depends on the tile counts and the number of sweeps only; the context keeps the last one.
+int lex_lists(im3d_ctx* ctx, LexArgs& a, int ns)
+{
+    const int key[4] = {a.nti, a.ntj, a.ntk, ns};
+    const size_t nt = (size_t)a.nti * a.ntj * a.ntk, count = nt * ns;
+    // the old list's buffer may be gone from here on, also when this call fails
+    const bool known = std::memcmp(key, ctx->lex_key, sizeof key) == 0;
+    if (!known) ctx->lex_key[0] = 0;
+    unsigned long long* tasks = nullptr;
+    IM3D_TRY(tbuf<unsigned long long>(ctx, kLexLists, count + (nt + 2) / 2, &tasks));
+    a.tasks = tasks;
+    a.ntasks = (int)count;
+    a.next = reinterpret_cast<int*>(tasks + count);
+    a.done = a.next + 1;
+    if (known) return IM3D_OK;
+    // counting sort of (tile, sweep) by i + j + k + 2 sweep
+    const int levels = a.nti + a.ntj + a.ntk - 2 + 2 * (ns - 1);
+    std::vector<size_t> at;
+    std::vector<unsigned long long> list;
+    try {
+        at.assign(levels + 1, 0);
+        list.resize(count);
+    } catch (const std::bad_alloc&) {
+        return fail(ctx, IM3D_ERR_OOM, "no host memory for the lexicographic task list");
+    }
+    for (int pass = 0; pass < 2; ++pass) {
+        for (int s = 0; s < ns; ++s)
+            for (int i = 0; i < a.nti; ++i)
+                for (int j = 0; j < a.ntj; ++j)
+                    for (int k = 0; k < a.ntk; ++k) {
+                        const int l = i + j + k + 2 * s;
+                        if (pass == 0) ++at[l + 1];
+                        else
+                            list[at[l]++] = (unsigned long long)i | (unsigned long long)j << 16 |
+                                            (unsigned long long)k << 32 | (unsigned long long)s << 48;
+                    }
+        if (pass == 0)
+            for (int l = 0; l < levels; ++l) at[l + 1] += at[l];
+    }
+    IM3D_CUDA(ctx, cudaMemcpyAsync(tasks, list.data(), count * sizeof(unsigned long long), cudaMemcpyHostToDevice,
+                                   ctx->stream));
+    IM3D_TRY(sync(ctx));  // the list must outlive the copy
+    std::memcpy(ctx->lex_key, key, sizeof key);
+    return IM3D_OK;
+}
+
+// One lexicographic sweep without any memory, one launch per hyperplane (lex_plane_kernel).
+template <typename T>
+int lex_planes(im3d_ctx* ctx, T* r, const T* b, const Dims& d, const GsCoef<T>& c)
+{
+    const int lo = c.neu ? 0 : 1;
+    const int hix = d.nx - lo, hiy = d.ny - lo, hiz = d.nz - lo;
+    const dim3 blk(32, 4);
+    for (int s = 3 * lo; s <= (hix - 1) + (hiy - 1) + (hiz - 1); ++s) {
+        const int i0 = std::max(lo, s - (hiy - 1) - (hiz - 1));
+        const int i1 = std::min(hix - 1, s - 2 * lo);
+        if (i0 > i1) continue;
+        const int j0 = std::max(lo, s - i1 - (hiz - 1));
+        const int j1 = std::min(hiy - 1, s - i0 - lo);
+        if (j0 > j1) continue;
+        const dim3 grid((j1 - j0 + 1 + blk.x - 1) / blk.x, (i1 - i0 + 1 + blk.y - 1) / blk.y);
+        lex_plane_kernel<T><<<grid, blk, 0, ctx->stream>>>(r, b, d, c, s, lo, i0, j0);
+        IM3D_TRY(check_launch(ctx, "lex_plane"));
+    }
+    return IM3D_OK;
+}
+
+// Lexicographic sweeps, reference order, natural layout, in place: by tiles (lex_tile_kernel),
+// several sweeps per launch, or where the device or the context's memory limit has no room for
+// the task list one sweep per launch, or by hyperplanes (5 sweeps of 64^3 in FP64: 262 us by
+// tiles, 3804 by hyperplanes). A wait that gave up raises ctrl flag 1.
 template <typename T>
 int lex_sweeps(im3d_ctx* ctx, T* r, const T* b, const Dims& d, const GsCoef<T>& c, int sweeps)
 {
@@ -816,12 +910,8 @@ int lex_sweeps(im3d_ctx* ctx, T* r, const T* b, const Dims& d, const GsCoef<T>& 
     a.ntk = tiles(d.nz);
     const long long nt = (long long)a.nti * a.ntj * a.ntk;
     // sweeps of one launch: the list stays below a few million tasks
-    const int per = (int)std::max<long long>(1, std::min<long long>(std::min(sweeps, 32768), (1ll << 22) / nt));
+    int per = (int)std::max<long long>(1, std::min<long long>(std::min(sweeps, 32768), (1ll << 22) / nt));
     if (nt > 0x7fffffffLL / 2) return fail(ctx, IM3D_ERR_INVALID_ARG, "volume too large for the launch geometry");
-    int* state = nullptr;  // task counter, then the sweeps finished per tile
-    IM3D_TRY(tbuf<int>(ctx, "lex_state", (size_t)nt + 1, &state));
-    a.next = state;
-    a.done = state + 1;
     a.err = &ctx->ctrl_d->flag[1];
     // FP64 without a division where the spacings and dt allow it (FP32 never divides)
     auto kern = sizeof(T) == 8 && c.pow2 == 15 ? lex_tile_kernel<T, true> : lex_tile_kernel<T, false>;
@@ -831,45 +921,23 @@ int lex_sweeps(im3d_ctx* ctx, T* r, const T* b, const Dims& d, const GsCoef<T>& 
     IM3D_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kLexT * kLexT, smem));
     if (occ < 1) return fail(ctx, IM3D_ERR_UNSUPPORTED, "the lexicographic sweep does not fit an SM");
     const int pf = prof_begin(ctx, "lex_sweep");
-    for (int s0 = 0; s0 < sweeps; s0 += per) {
-        const int ns = std::min(per, sweeps - s0);
-        const int key[4] = {a.nti, a.ntj, a.ntk, ns};
-        unsigned long long* tasks = nullptr;
-        const size_t count = (size_t)nt * ns;
-        // the old list's buffer may be gone from here on, also when this call fails
-        const bool known = std::memcmp(key, ctx->lex_key, sizeof key) == 0;
-        if (!known) ctx->lex_key[0] = 0;
-        IM3D_TRY(tbuf<unsigned long long>(ctx, "lex_tasks", count, &tasks));
-        if (!known) {
-            // counting sort of (tile, sweep) by i + j + k + 2 sweep
-            const int levels = a.nti + a.ntj + a.ntk - 2 + 2 * (ns - 1);
-            std::vector<size_t> at(levels + 1, 0);
-            std::vector<unsigned long long> list(count);
-            for (int pass = 0; pass < 2; ++pass) {
-                for (int s = 0; s < ns; ++s)
-                    for (int i = 0; i < a.nti; ++i)
-                        for (int j = 0; j < a.ntj; ++j)
-                            for (int k = 0; k < a.ntk; ++k) {
-                                const int l = i + j + k + 2 * s;
-                                if (pass == 0) ++at[l + 1];
-                                else
-                                    list[at[l]++] = (unsigned long long)i | (unsigned long long)j << 16 |
-                                                    (unsigned long long)k << 32 | (unsigned long long)s << 48;
-                            }
-                if (pass == 0)
-                    for (int l = 0; l < levels; ++l) at[l + 1] += at[l];
-            }
-            IM3D_CUDA(ctx, cudaMemcpyAsync(tasks, list.data(), count * sizeof(unsigned long long),
-                                           cudaMemcpyHostToDevice, ctx->stream));
-            IM3D_TRY(sync(ctx));  // the list must outlive the copy
-            std::memcpy(ctx->lex_key, key, sizeof key);
+    const std::string err = ctx->err;
+    for (int s0 = 0; s0 < sweeps;) {
+        int ns = std::min(per, sweeps - s0);
+        int st = lex_lists(ctx, a, ns);
+        if (st == IM3D_ERR_OOM && ns > 1) st = lex_lists(ctx, a, per = ns = 1);
+        if (st == IM3D_ERR_OOM) {
+            ctx->err = err;
+            for (; s0 < sweeps; ++s0) IM3D_TRY(lex_planes(ctx, r, b, d, c));
+            break;
         }
-        a.tasks = tasks;
-        a.ntasks = (int)count;
-        IM3D_CUDA(ctx, cudaMemsetAsync(state, 0, ((size_t)nt + 1) * sizeof(int), ctx->stream));
-        const long long blocks = std::min<long long>((long long)count, (long long)occ * ctx->num_sms);
+        IM3D_TRY(st);
+        ctx->err = err;
+        IM3D_CUDA(ctx, cudaMemsetAsync(a.next, 0, ((size_t)nt + 1) * sizeof(int), ctx->stream));
+        const long long blocks = std::min<long long>(a.ntasks, (long long)occ * ctx->num_sms);
         kern<<<(unsigned)blocks, kLexT * kLexT, smem, ctx->stream>>>(r, b, d, c, a);
         IM3D_TRY(check_launch(ctx, "lex_tile"));
+        s0 += ns;
     }
     prof_end(ctx, pf);
     return IM3D_OK;

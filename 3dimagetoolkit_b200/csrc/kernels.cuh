@@ -1402,6 +1402,24 @@ __global__ void __launch_bounds__(kLexT* kLexT) lex_tile_kernel(T* r, const T* _
     }
 }
 
+// One hyperplane i + j + k = s of a lexicographic sweep: its unknowns are independent of each
+// other given the planes s - 1 (already updated) and s + 1 (not yet). Threads cover (i, j). For
+// calls that have no memory for lex_tile_kernel's list; bound by its launches, one per
+// hyperplane.
+template <typename T>
+__global__ void lex_plane_kernel(T* r, const T* __restrict__ b, Dims d, GsCoef<T> c, int s, int lo, int i_begin, int j_begin)
+{
+    const int j = j_begin + blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = i_begin + blockIdx.y * blockDim.y + threadIdx.y;
+    const int hix = d.nx - lo, hiy = d.ny - lo, hiz = d.nz - lo;
+    if (i >= hix || j >= hiy) return;
+    const int k = s - i - j;
+    if (k < lo || k >= hiz) return;
+    const long long p = d.idx(i, j, k);
+    auto rd = [&](int oi, int oj, int ok) { return r[d.idx(i + oi, j + oj, k + ok)]; };
+    r[p] = gs_value<T>(c, d, i, j, k, b[p], r[p], true, rd);
+}
+
 // Dirichlet boundary assignment of DirGaussSeidel (poisson_imp.hxx:366-391).
 template <typename T>
 __global__ void dir_faces_kernel(T* r, Dims d, T bc)

@@ -45,3 +45,25 @@ def test_list_after_a_failed_allocation(pkg, O):
         again = _sweep(c, u, b, 3)
     assert np.array_equal(first, want)
     assert np.array_equal(again, want)
+
+
+@pytest.mark.parametrize("bc_type, bc", [("dir", 0.3), ("neu", 0.3)])
+@pytest.mark.parametrize("limit", [1, 4000, 8 * 27 * 4 + 4 * 28 + 256 + 16])
+def test_sweeps_under_a_memory_limit(pkg, O, limit, bc_type, bc):
+    """On device arrays the sweeps need no memory: any limit lets them run, without the list, with
+    a list of one sweep, or with the whole one; and the list gives way to a buffer that another
+    call needs under the same limit."""
+    u, b = _case((40, 37, 48), 5)  # 27 tiles (Dirichlet and Neumann)
+    kw = dict(dt=0.7, bc=bc, bc_type=pkg.BC_NEU if bc_type == "neu" else pkg.BC_DIR, h=(0.8, 1.0, 1.3))
+    want = O.poisson_sweeps(u, b, sweeps=4, **kw)
+    with pkg.Context(0) as c:
+        c.set_option(pkg.OPT_DEVICE_MEMORY_LIMIT, limit)
+        got = _sweep(c, u, b, 4, **kw)
+        assert np.array_equal(got, want)
+        # two host arrays need two buffers of this size, and leave no room for the list
+        c.set_option(pkg.OPT_DEVICE_MEMORY_LIMIT, 2 * (u.size * 8 + 256) + 1)
+        got = u.copy()
+        c.poisson_sweeps(got, b, sweeps=4, **kw)
+        assert np.array_equal(got, want)
+        c.set_option(pkg.OPT_DEVICE_MEMORY_LIMIT, 0)
+        assert np.array_equal(_sweep(c, u, b, 4, **kw), want)
