@@ -856,8 +856,7 @@ int lex_lists(im3d_ctx* ctx, LexArgs& a, int ns)
                         const int l = i + j + k + 2 * s;
                         if (pass == 0) ++at[l + 1];
                         else
-                            list[at[l]++] = (unsigned long long)i | (unsigned long long)j << 16 |
-                                            (unsigned long long)k << 32 | (unsigned long long)s << 48;
+                            list[at[l]++] = lex_task(i, j, k, s);
                     }
         if (pass == 0)
             for (int l = 0; l < levels; ++l) at[l + 1] += at[l];
@@ -910,7 +909,7 @@ int lex_sweeps(im3d_ctx* ctx, T* r, const T* b, const Dims& d, const GsCoef<T>& 
     a.ntk = tiles(d.nz);
     const long long nt = (long long)a.nti * a.ntj * a.ntk;
     // sweeps of one launch: the list stays below a few million tasks
-    int per = (int)std::max<long long>(1, std::min<long long>(std::min(sweeps, 32768), (1ll << 22) / nt));
+    int per = (int)std::max<long long>(1, std::min<long long>(std::min(sweeps, kLexMaxSweeps), (1ll << 22) / nt));
     if (nt > 0x7fffffffLL / 2) return fail(ctx, IM3D_ERR_INVALID_ARG, "volume too large for the launch geometry");
     a.err = &ctx->ctrl_d->flag[1];
     // FP64 without a division where the spacings and dt allow it (FP32 never divides)

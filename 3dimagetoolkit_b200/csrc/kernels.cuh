@@ -1255,8 +1255,17 @@ constexpr int kLexT = 16;
 constexpr int kLexH = kLexT + 2;
 constexpr long long kLexWaitLimit = 1ll << 22;  // polls (under a microsecond each) before a wait gives up
 
+// A task's tile and sweep in one word: 12 bits for i and j (up to 65535 points), 27 for k (up to
+// 2^31 points), 13 for the sweep.
+constexpr int kLexMaxSweeps = 1 << 13;
+__host__ __device__ constexpr unsigned long long lex_task(int i, int j, int k, int sweep)
+{
+    return (unsigned long long)i | (unsigned long long)j << 12 | (unsigned long long)k << 24 |
+           (unsigned long long)sweep << 51;
+}
+
 struct LexArgs {
-    const unsigned long long* tasks;  // i | j << 16 | k << 32 | sweep << 48, in tiles
+    const unsigned long long* tasks;  // lex_task
     int ntasks;
     int* next;       // task counter
     int* done;       // sweeps finished per tile
@@ -1312,8 +1321,8 @@ __global__ void __launch_bounds__(kLexT* kLexT) lex_tile_kernel(T* r, const T* _
         __syncthreads();
         if (s_task >= a.ntasks) return;
         const unsigned long long t = a.tasks[s_task];
-        const int ti = (int)(t & 0xffff), tj = (int)(t >> 16 & 0xffff), tk = (int)(t >> 32 & 0xffff),
-                  sw = (int)(t >> 48);
+        const int ti = (int)(t & 0xfff), tj = (int)(t >> 12 & 0xfff), tk = (int)(t >> 24 & 0x7ffffff),
+                  sw = (int)(t >> 51);
         const int i0 = lo + ti * N, j0 = lo + tj * N, k0 = lo + tk * N;
         const int tile = (ti * a.ntj + tj) * a.ntk + tk;
         const int stt[3] = {a.ntj * a.ntk, a.ntk, 1}, pos[3] = {ti, tj, tk}, len[3] = {a.nti, a.ntj, a.ntk};

@@ -67,3 +67,13 @@ def test_sweeps_under_a_memory_limit(pkg, O, limit, bc_type, bc):
         assert np.array_equal(got, want)
         c.set_option(pkg.OPT_DEVICE_MEMORY_LIMIT, 0)
         assert np.array_equal(_sweep(c, u, b, 4, **kw), want)
+
+
+def test_rows_of_more_than_65536_tiles(pkg, ctx, O):
+    """A tile's k index has more than 16 bits where nz is above 2^20 (3 x 3 x 1049000)."""
+    u, b = _case((3, 3, 1049000), 7)
+    kw = dict(dt=0.7, bc=0.0, bc_type=pkg.BC_DIR, sweeps=2, h=(1.0, 1.0, 1.0))
+    want = O.poisson_sweeps(u, b, **kw)
+    got = u.copy()
+    ctx.poisson_sweeps(got, b, **kw)
+    assert np.array_equal(got, want)
