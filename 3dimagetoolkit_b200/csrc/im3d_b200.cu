@@ -1881,8 +1881,9 @@ int rsfe_apply(im3d_ctx* ctx, const T* myim_user, const T* init_user, int nx, in
             const long long cnt = lex ? n : npk2;
             double ls_err = p->ls_tol ? 1000. : -1.;
             int s;
+            constexpr int kMaxSweeps = 100000;
             for (s = 0; s < p->ls_steps || ls_err > p->ls_tol; ++s) {
-                if (s >= 100000) {
+                if (s >= kMaxSweeps) {
                     not_conv++;
                     break;
                 }
@@ -1890,8 +1891,10 @@ int rsfe_apply(im3d_ctx* ctx, const T* myim_user, const T* init_user, int nx, in
                     IM3D_CUDA(ctx, cudaMemcpyAsync(prev, work, cnt * sizeof(T), cudaMemcpyDeviceToDevice,
                                                    ctx->stream));
                 if (lex && p->ls_tol == 0) {
-                    IM3D_TRY(lex_sweeps<T>(ctx, phi, rhs, d, coef, p->ls_steps));
-                    s = p->ls_steps;
+                    // without a tolerance the number of sweeps is known
+                    s = std::min(p->ls_steps, kMaxSweeps);
+                    IM3D_TRY(lex_sweeps<T>(ctx, phi, rhs, d, coef, s));
+                    if (s < p->ls_steps) not_conv++;
                     break;
                 }
                 if (lex) IM3D_TRY(lex_sweeps<T>(ctx, phi, rhs, d, coef, 1));

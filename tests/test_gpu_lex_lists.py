@@ -77,3 +77,13 @@ def test_rows_of_more_than_65536_tiles(pkg, ctx, O):
     got = u.copy()
     ctx.poisson_sweeps(got, b, **kw)
     assert np.array_equal(got, want)
+
+
+def test_sweeps_of_an_iteration_are_bounded(pkg, ctx):
+    """At most 100000 sweeps per outer iteration, also where their number is known beforehand."""
+    u0 = pkg.synth.ellipsoids((8, 8, 8), 3, n=1, semi_axes=(2, 3))
+    phi0 = pkg.synth.sphere_phi0((8, 8, 8), 2.5)
+    params = pkg.default_params(sigma=1.0, lamda1=1.0, lamda2=1.0, epsilon=1e-3, lamda=0.5, tol=0.0, maxiter=1,
+                                ls_steps=100003, sweep=pkg.SWEEP_LEXICOGRAPHIC)
+    stats = ctx.rsfe_apply(u0, phi0, params)["stats"]
+    assert stats["total_sweeps"] == 100000 and stats["not_converged"] == 1
