@@ -1468,7 +1468,7 @@ __device__ __forceinline__ void flat_pair(const uint3 blockIdx, unsigned groups,
 // half-sweep following one in the other direction starts on the planes that are still
 // in L2.
 template <typename T, int NI>
-__global__ void __launch_bounds__(128) rb_half_vec_kernel(T* __restrict__ U, const T* __restrict__ B, Dims d, GsCoef<T> c, int color, int use_self, T omega, int reverse)
+__global__ void __launch_bounds__(128) rb_half_vec_kernel(T* __restrict__ U, const T* B, Dims d, GsCoef<T> c, int color, int use_self, T omega, int reverse)
 {
     typedef long long IX;
     typedef V16<T> VT;
@@ -1734,7 +1734,9 @@ __device__ __forceinline__ typename V16<T>::type rb_group(const GsCoef<T>& c, co
 
 // Half-sweep of the residual solve: own value and relaxation out of the way, the updated
 // colour `own` and the other colour `oth` as separate pointers, so that no store holds a
-// load back. One thread per group of W = 16/sizeof(T) packed cells of row j, marching over
+// load back. Only `own` is __restrict__: the previous launch may still be writing `oth` (and the
+// first one's, b_eff) while this one's blocks are resident, so their loads must stay ordinary
+// ones that the wait below orders. One thread per group of W = 16/sizeof(T) packed cells of row j, marching over
 // NI planes of i with the next plane's reads in flight. Every cell of a group is computed
 // by the interior formula, without a test per cell:
 //  * the k neighbours are the group itself and the group shifted by one cell (the parity of
@@ -1758,7 +1760,7 @@ __device__ __forceinline__ typename V16<T>::type rb_group(const GsCoef<T>& c, co
 // 128^3 FP64 7.5 -> 4.9 and 200^3 FP64 28.4 -> 17.9 (no division per cell, over_h2).
 template <typename T, int NI, int BC, typename IX, bool P2 = false>
 __device__ __forceinline__ void rb_march_body(const uint3 blockIdx, const dim3 gridDim, T* __restrict__ own,
-                                              const T* __restrict__ oth, const T* __restrict__ bb, const Dims& d,
+                                              const T* oth, const T* bb, const Dims& d,
                                               const GsCoef<T>& c, int color, int reverse, int first)
 {
     typedef V16<T> VT;
@@ -1831,7 +1833,7 @@ __device__ __forceinline__ void rb_march_body(const uint3 blockIdx, const dim3 g
 }
 
 template <typename T, int NI, int BC, int MINB, typename IX, bool P2>
-__global__ void __launch_bounds__(128, MINB) rb_march_kernel(T* __restrict__ own, const T* __restrict__ oth, const T* __restrict__ bb, Dims d, GsCoef<T> c, int color, int reverse, int first)
+__global__ void __launch_bounds__(128, MINB) rb_march_kernel(T* __restrict__ own, const T* oth, const T* bb, Dims d, GsCoef<T> c, int color, int reverse, int first)
 {
     rb_march_body<T, NI, BC, IX, P2>(blockIdx, gridDim, own, oth, bb, d, c, color, reverse, first);
 }
