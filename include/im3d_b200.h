@@ -352,7 +352,8 @@ int im3d_unet_train_step(im3d_ctx* ctx, im3d_unet* net, const float* x, const fl
 /* One 3x3x3 convolution (zero padding, stride 1) on the tensor cores, as the network's
  * layers run it: x BF16 channels-last (c_pitch channels per voxel, the cin used ones
  * from c_off), w FP32 [cout][cin][27], bias FP32 [cout] or NULL, out FP32 channels-last
- * [voxel][cout]; cin, cout in {16, 32, 64}; all pointers device memory. */
+ * [voxel][cout]; cin, cout in {16, 32, 64}; all pointers device memory, their contents
+ * complete or written on the legacy default stream (the call waits for that one). */
 int im3d_conv3d_bf16(im3d_ctx* ctx, const uint16_t* x, int c_pitch, int c_off, int cin, const float* w,
                      const float* bias, int cout, int nsamp, int nx, int ny, int nz, float* out);
 
