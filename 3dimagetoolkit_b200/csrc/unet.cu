@@ -901,18 +901,24 @@ int im3d_conv3d_bf16(im3d_ctx* ctx, const uint16_t* x, int c_pitch, int c_off, i
     // a caller's tensors may still be on their way on the default stream, which the context's
     // own stream does not wait for
     UN_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
-    UN_CUDA(cudaMemsetAsync(errf, 0, sizeof(int), st));
-    const int nout = nout_for(cout);
-    PackJobs jobs;
-    jobs.job[0] = PackJob{w, wpk, cout, cin, nout, 0};
-    pack_filter_kernel<<<flat_blocks(27LL * cin * cout), 256, 0, st>>>(jobs);
-    UN_TRY(launch_status(err, "pack_filter"));
-    const View v{reinterpret_cast<const bf16_t*>(x), c_pitch, nx, ny, nz, nsamp};
-    UN_TRY(conv_any<CONV_BIAS_F32>(st, cin, nout, v, c_off, wpk, cout / nout, bias, out, cout, 0, nullptr, 0, 0, errf,
-                                   err));
     int h = 0;
-    UN_CUDA(cudaMemcpyAsync(&h, errf, sizeof(int), cudaMemcpyDeviceToHost, st));
+    auto work = [&]() -> int {
+        UN_CUDA(cudaMemsetAsync(errf, 0, sizeof(int), st));
+        const int nout = nout_for(cout);
+        PackJobs jobs;
+        jobs.job[0] = PackJob{w, wpk, cout, cin, nout, 0};
+        pack_filter_kernel<<<flat_blocks(27LL * cin * cout), 256, 0, st>>>(jobs);
+        UN_TRY(launch_status(err, "pack_filter"));
+        const View v{reinterpret_cast<const bf16_t*>(x), c_pitch, nx, ny, nz, nsamp};
+        UN_TRY(conv_any<CONV_BIAS_F32>(st, cin, nout, v, c_off, wpk, cout / nout, bias, out, cout, 0, nullptr, 0, 0,
+                                       errf, err));
+        UN_CUDA(cudaMemcpyAsync(&h, errf, sizeof(int), cudaMemcpyDeviceToHost, st));
+        return IM3D_OK;
+    };
+    // the caller's arrays are its own again when the call returns, with an error too
+    const int s = work();
     UN_CUDA(cudaStreamSynchronize(st));
+    if (s != IM3D_OK) return s;
     if (h) {
         err = "conv3d: a wait gave up";
         return IM3D_ERR_CUDA;

@@ -36,3 +36,19 @@ def test_inputs_written_on_a_side_stream(ctx):
         b2.copy_(bd)
         got = ctx.conv3d_bf16(x2, w2, b2)
     assert rel(got.cpu().double().numpy(), _want(x, w, b)) <= 1e-5
+
+
+@pytest.mark.parametrize("nz", [24, 144])
+def test_refused_width_leaves_nothing_running(pkg, nz):
+    """A width without a tiling is refused, and nothing queued by the call still reads its
+    arguments: the context's stream, busy before the call, is idle after it."""
+    x, w, b = (t.cuda() for t in _inputs(2, dims=(3, 4, nz)))
+    with pkg.Context(0) as c:
+        stream = torch.cuda.Stream()
+        c.set_stream(stream.cuda_stream)
+        with torch.cuda.stream(stream):
+            torch.cuda._sleep(20_000_000)  # about 10 ms of clock cycles
+        with pytest.raises(pkg.Im3dError):
+            c.conv3d_bf16(x, w, b)
+        assert stream.query()
+        c.set_stream(None)
