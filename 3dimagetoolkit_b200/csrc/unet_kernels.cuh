@@ -147,6 +147,7 @@ __global__ void __launch_bounds__(kMarchThreads, 1) conv3_march_kernel(const __g
     uint64_t* drained = ready + kMarchSlots; // ... and read out
     uint32_t* tslot = reinterpret_cast<uint32_t*>(drained + kMarchSlots);
     __shared__ volatile int s_fail;
+    __shared__ uint64_t s_last[kMarchIssuers];  // a failed issuer's MMAs have ended
     __shared__ float s_bias[NOUT];
     const int nb = blockIdx.y;  // block of NOUT output channels
 
@@ -165,6 +166,7 @@ __global__ void __launch_bounds__(kMarchThreads, 1) conv3_march_kernel(const __g
             tc::mbar_init(ready + q, kMarchIssuers);
             tc::mbar_init(drained + q, kMarchDrains);
         }
+        for (int q = 0; q < kMarchIssuers; ++q) tc::mbar_init(s_last + q, 1);
         tc::fence_mbar_init();
         s_fail = 0;
     }
@@ -293,6 +295,11 @@ __global__ void __launch_bounds__(kMarchThreads, 1) conv3_march_kernel(const __g
                         if (++sa == g.slots) sa = 0;
                     }
                 }
+            }
+            // after a failure the MMAs issued so far end before their operands and TMEM are given back
+            if (!ok) {
+                tc::mma_commit(s_last + warp - 1);
+                tc::mbar_wait(s_last + warp - 1, 0, 1000000000ull);
             }
         }
     } else {
