@@ -970,10 +970,10 @@ dim3 grid_rb_flat(const Dims& d, dim3 blk, int zmul = 1, int ni = kNV)
 // planes per thread of the residual check: 4 on large grids, 2 where 4 leave fewer than 16
 // blocks per SM (us with 2 and 4: 171x203x117 27 / 31, 256^3 50 / 47.5, 512x512x320 227 / 202)
 template <typename T>
-int res_planes(const Dims& d)
+int res_planes(const im3d_ctx* ctx, const Dims& d)
 {
     const dim3 g = grid_rb_flat<T>(d, kBlkVec, 2, kNVres);
-    return (long long)g.x * g.z >= 16 * 148 ? kNVres : 2;
+    return (long long)g.x * g.z >= 16ll * ctx->num_sms ? kNVres : 2;
 }
 
 // natural-layout vectorised kernels: (vector group, row) pairs flattened over x blocks
@@ -1217,7 +1217,7 @@ template <typename T>
 int rb_check(im3d_ctx* ctx, const T* U, const T* B, const Dims& d, const GsCoef<T>& c,
              double* beff2, double* rel)
 {
-    const int ni = res_planes<T>(d);
+    const int ni = res_planes<T>(ctx, d);
     const dim3 grid = grid_rb_flat<T>(d, kBlkVec, 2, ni);
     const int nvals = *beff2 < 0 ? 2 : 1;
     double* part = nullptr;
@@ -2560,7 +2560,7 @@ int worklist_group(im3d_ctx* ctx, const std::vector<int>& ids, const im3d_volume
                                  dsc.nx, dsc.ny, dsc.nz, dsc.hx, dsc.hy, dsc.hz, p, nullptr, nullptr,
                                  nullptr, nullptr, nullptr);
         const Dims& d = V[q].d;
-        const dim3 gr = grid_rb_flat<T>(d, kBlkVec, 2, res_planes<T>(d));
+        const dim3 gr = grid_rb_flat<T>(d, kBlkVec, 2, res_planes<T>(ctx, d));
         const bool vec = d.nz % V16<T>::W == 0;
         const dim3 gc = vec ? grid_vec<T>(d, kBlkVec) : grid_col(d, kBlkVol);
         if (st == IM3D_OK)
@@ -2642,7 +2642,7 @@ int worklist_group(im3d_ctx* ctx, const std::vector<int>& ids, const im3d_volume
             jrd[c].h.push_back({RbD{v.upk, v.bpk, d, v.coef, c, c}, gpk});
             jrn[c].h.push_back({RbN{v.upk, v.bpk, d, v.coef, c, c}, gpk});
         }
-        const int ni = res_planes<T>(d);
+        const int ni = res_planes<T>(ctx, d);
         const dim3 gr = grid_rb_flat<T>(d, kBlkVec, 2, ni);
         jres.h.push_back({Res{v.upk, v.bpk, d, v.coef, part_res[q], ni}, gr});
         fin_res[q] = FinalizeJob{part_res[q], (long long)gr.x * gr.y * gr.z, ctrl[q].sum};

@@ -16,7 +16,7 @@ have positive terms, and what remains are the gradients' own FP32 sums:
 
 A wrong tap, a dropped row or plane, or a tile counted twice moves an element by 1e-3 and more.
 Shapes: rows past the last tile of 8, 4, 2 rows, every tile width, two samples, chains of several
-tiles (up to 14 at 64 x 100 x 64), more rows than the rings hold."""
+tiles (up to 12 at 64 x 100 x 64, with 96 rows through rings of 8 and 5)."""
 import numpy as np
 import pytest
 
