@@ -968,7 +968,8 @@ dim3 grid_rb_flat(const Dims& d, dim3 blk, int zmul = 1, int ni = kNV)
 }
 
 // planes per thread of the residual check: 4 on large grids, 2 where 4 leave fewer than 16
-// blocks per SM (us with 2 and 4: 171x203x117 27 / 31, 256^3 50 / 47.5, 512x512x320 227 / 202)
+// blocks per SM (us with 2 and 4: 48x44x40 8.2 / 8.5, 171x203x117 31 / 31, 256^3 54 / 51,
+// 512x512x320 240 / 222)
 template <typename T>
 int res_planes(const im3d_ctx* ctx, const Dims& d)
 {

@@ -1974,8 +1974,8 @@ __global__ void __launch_bounds__(kRbClThreads, 1) rb_cluster_kernel(T* __restri
 // rb_group and c_a = 1, and cells that are no unknowns (Dirichlet faces, padding) count 0.
 // What bounds it: conversions to FP64 (about 5 per cell; a value is converted once and kept
 // for the planes that read it) and the reads. us against per-cell face tests with a generic
-// boundary path (88 instructions per cell): 256^3 66 -> 49, 512x512x320 300 -> 214, 171x203x117
-// Neumann 38 -> 30 (6 blocks of 128 threads per SM; unlimited and 8 measured slower).
+// boundary path (88 instructions per cell): 256^3 66 -> 51, 512x512x320 300 -> 222, 171x203x117
+// Neumann 38 -> 31 (6 blocks of 128 threads per SM; unlimited and 8 measured slower).
 template <typename T, int NI, bool NEU, typename IX = long long>
 __device__ __forceinline__ void rb_residual_vec_body(const uint3 blockIdx, const dim3 gridDim, const T* __restrict__ U, const T* __restrict__ B, const Dims& d, const GsCoef<T>& c, double* part, int want_beff, int ni)
 {

@@ -142,8 +142,8 @@ int plan_zc(int D, long long cols, int ctas)
 }
 
 // Tiling of a 3x3x3 convolution: 4 tile rows where two staged planes, the filter and four
-// output planes fit (measured at 128^3, 16 -> 16 channels: 8, 4, 2, 1 rows take 79, 79, 123,
-// 183 us; 64 -> 32 at 64^3: 4, 2, 1 take 71, 87, 138), else fewer; output planes per unit zc
+// output planes fit (16 -> 16 channels at 128^3 take 1, 1, 1.56 and 2.3 times as long with 8, 4, 2
+// and 1 rows, 64 -> 32 at 64^3 1, 1.2 and 1.9 times with 4, 2 and 1), else fewer; output planes per unit zc
 // such that the busiest CTA streams the fewest planes.
 template <int CIN, int NOUT>
 bool plan_march(int D, int H, int W, int nsamp, int nblocks, MarchGeom* g, int* smem)

@@ -17,7 +17,7 @@
 // no im2col buffer, one read of each plane per tile. M = 128 output positions of the
 // padded tile, N = the output channels of the launch (16 or 32) of the three output planes
 // that the input plane feeds, K = 16 input channels per instruction; the FP32 accumulators
-// live in TMEM and are drained by 4 warps (bias + ReLU or the ReLU mask of the data
+// live in TMEM and are drained by 8 warps (bias + ReLU or the ReLU mask of the data
 // gradient, BF16 store). The weight gradient (wgrad_mma_kernel) streams rows of the
 // activations and of the output's gradient, with its accumulators in registers (mma.sync: its M
 // fits 16 and 32 output channels).
@@ -125,7 +125,7 @@ __device__ __forceinline__ int mtile_start(int TW, int m)
 // 3800 cycles per plane of 4 x 128 voxels of 16 channels, against 36 + N / 4 cycles per MMA
 // (measured, M = 128, K = 16: its operands go through shared memory), about 2000. Three dz taps
 // per MMA cost little more than one, and each plane is loaded once instead of three times.
-// 16-byte cp.async from 4 warps instead of the TMA measured slower (119 against 79 us).
+// 16-byte cp.async from 4 warps instead of the TMA measured 1.5 times slower.
 // Measured against one block of three planes per output plane, load, MMAs (N = NOUT) and drain
 // in turn (us): 16 -> 16 channels at 128^3 139 -> 74, 32 -> 16 406 -> 124, 64 -> 32 at 64^3
 // 154 + 154 (N = 16) -> 67.
@@ -506,7 +506,8 @@ __device__ __forceinline__ void wgrad_row(float (&acc)[3][MB][2][4], const uint3
 // smallest M (64) multiplies three quarters or half of it for nothing.
 // us (output x input channels): 16 x 16 at 128^3 124, 16 x 32 at 128^3 261, 32 x 32 at 64^3 60,
 // 32 x 16 at 64^3 37; the same chains on tcgen05, load and multiply in turn: 929, 950, 420 for
-// the first three. Consecutive tiles of a chain lie in other rows and planes, so X is read for each of
+// the first three. What bounds it: the reads of the fragments from shared memory (its port busy
+// 36 to 61 % of the time) and the fixed latency of mma.sync, whose pipe is busy 28 to 46 %. Consecutive tiles of a chain lie in other rows and planes, so X is read for each of
 // its three planes anew; chains marching along z (90, 157, 48, 32 us) are other sums.
 template <int CO>
 __global__ void __launch_bounds__(kWgThreads, 1) wgrad_mma_kernel(const __grid_constant__ CUtensorMap xmap,
