@@ -1037,7 +1037,11 @@ int rb_march_launch(im3d_ctx* ctx, T* U, const T* B, const Dims& d, const GsCoef
     // red walks the planes forward, black backward: each half-sweep starts on the planes
     // the previous one wrote last, which are still in L2
     constexpr int MINB = BC == RB_NEU ? 1 : kRbMinB;
-    auto kern = rb_march_kernel<T, NI, BC, MINB, IX, false>;
+    // FP64 with divisions on a grid that does not fill the GPU: registers for the divisions
+    // instead of blocks per SM (us with 8 and unlimited: 90x80x71 3.44 / 3.09, 128x96x100 5.70 /
+    // 5.21, 200^3 on 4 planes 27.5 / 35.0)
+    constexpr int MINB_DIV = sizeof(T) == 8 && NI == 2 ? 1 : MINB;
+    auto kern = rb_march_kernel<T, NI, BC, MINB_DIV, IX, false>;
     if constexpr (sizeof(T) == 8)  // no division where the spacings allow it
         if ((c.pow2 & 7) == 7) kern = rb_march_kernel<T, NI, BC, MINB, IX, true>;
     return launch_dependent(ctx, kern, grid_rb_flat<T>(d, kBlkVec, 1, NI), kBlkVec, U + (color ? npk : 0),
@@ -1068,10 +1072,13 @@ int rb_sweep(im3d_ctx* ctx, T* U, const T* B, const Dims& d, const GsCoef<T>& c,
     const bool self = use_self || omega != 1.0;
     for (int color = 0; color < 2; ++color) {
         const int pf = prof_begin(ctx, "rb_half");
-        if (self)
-            IM3D_TRY(launch_dependent(ctx, rb_half_vec_kernel<T, kNV>, grid_rb_flat<T>(d, kBlkVec), kBlkVec, U, B, d,
-                                      c, color, use_self, (T)omega, color));
-        else if (fits_int32(d))
+        if (self) {
+            auto kern = rb_half_vec_kernel<T, kNV, false>;
+            if constexpr (sizeof(T) == 8)  // no division where the spacings (and dt, if used) allow it
+                if ((c.pow2 & 7) == 7 && (!use_self || c.pow2 == 15)) kern = rb_half_vec_kernel<T, kNV, true>;
+            IM3D_TRY(launch_dependent(ctx, kern, grid_rb_flat<T>(d, kBlkVec), kBlkVec, U, B, d, c, color, use_self,
+                                      (T)omega, color));
+        } else if (fits_int32(d))
             IM3D_TRY((rb_march<T, int>(ctx, U, B, d, c, color, first && !color)));
         else
             IM3D_TRY((rb_march<T, long long>(ctx, U, B, d, c, color, first && !color)));

@@ -1159,26 +1159,27 @@ struct GsCoef {
 };
 
 // The neighbour terms of the FP64 update divide by h^2, the own value by dt
-// (poisson_imp.hxx:400). Where those are powers of two (pow2, or P2: all of them, known at
-// compile time) the product with the (exact) reciprocal is the same number.
-template <int AXIS, bool P2 = false, typename T>
+// (poisson_imp.hxx:400). Where all of those are powers of two (P2, which the host picks by
+// GsCoef::pow2) the product with the (exact) reciprocal is the same number. One form per
+// kernel: both behind a test per axis cost more than the divisions themselves.
+template <int AXIS, bool P2, typename T>
 __device__ __forceinline__ double over_h2(double x, const GsCoef<T>& c)
 {
     const double h = AXIS == 0 ? c.hx : AXIS == 1 ? c.hy : c.hz;
     const double r = AXIS == 0 ? c.ihx2d : AXIS == 1 ? c.ihy2d : c.ihz2d;
-    return P2 || (c.pow2 >> AXIS & 1) ? x * r : x / (h * h);
+    return P2 ? x * r : x / (h * h);
 }
 
-template <bool P2 = false, typename T>
+template <bool P2, typename T>
 __device__ __forceinline__ double over_dt(double x, const GsCoef<T>& c)
 {
-    return P2 || (c.pow2 & 8) ? x * c.idtd : x / c.dt;
+    return P2 ? x * c.idtd : x / c.dt;
 }
 
 // One Gauss-Seidel point value (sum of neighbour terms + b + self/dt) * htilde;
 // `self_dt` is self/dt (beff mode folds u_in/dt into b and passes 0).
 // r(o_i, o_j, o_k) returns the current value of a neighbour.
-template <typename T, bool P2 = false, class R>
+template <typename T, bool P2, class R>
 __device__ __forceinline__ T gs_value(const GsCoef<T>& c, const Dims& d, int i, int j, int k,
                                       T b, T self, bool use_self, R r)
 {
@@ -1426,7 +1427,7 @@ __global__ void lex_plane_kernel(T* r, const T* __restrict__ b, Dims d, GsCoef<T
     if (k < lo || k >= hiz) return;
     const long long p = d.idx(i, j, k);
     auto rd = [&](int oi, int oj, int ok) { return r[d.idx(i + oi, j + oj, k + ok)]; };
-    r[p] = gs_value<T>(c, d, i, j, k, b[p], r[p], true, rd);
+    r[p] = gs_value<T, false>(c, d, i, j, k, b[p], r[p], true, rd);
 }
 
 // Dirichlet boundary assignment of DirGaussSeidel (poisson_imp.hxx:366-391).
@@ -1466,9 +1467,10 @@ __device__ __forceinline__ void flat_pair(const uint3 blockIdx, unsigned groups,
 // rules; the residual solve with omega 1 runs rb_march_kernel instead.
 // reverse: the blocks take the planes of i from the last to the first, so that a
 // half-sweep following one in the other direction starts on the planes that are still
-// in L2.
-template <typename T, int NI>
-__global__ void __launch_bounds__(128) rb_half_vec_kernel(T* __restrict__ U, const T* B, Dims d, GsCoef<T> c, int color, int use_self, T omega, int reverse)
+// in L2. (Without the lower bound of one block per SM the compiler keeps to fewer registers:
+// 200^3 FP64 36.0 -> 36.5 us, Neumann 60.9 -> 62.2.)
+template <typename T, int NI, bool P2>
+__global__ void __launch_bounds__(128, 1) rb_half_vec_kernel(T* __restrict__ U, const T* B, Dims d, GsCoef<T> c, int color, int use_self, T omega, int reverse)
 {
     typedef long long IX;
     typedef V16<T> VT;
@@ -1554,8 +1556,8 @@ __global__ void __launch_bounds__(128) rb_half_vec_kernel(T* __restrict__ U, con
                 const T sf = VT::get(self, cc);
                 T v;
                 if (std::is_same<T, double>::value) {
-                    double acc = over_h2<0>(sx, c) + over_h2<1>(sy, c) + over_h2<2>(sz, c) + b;
-                    if (use_self) acc = acc + over_dt(sf, c);
+                    double acc = over_h2<0, P2>(sx, c) + over_h2<1, P2>(sy, c) + over_h2<2, P2>(sz, c) + b;
+                    if (use_self) acc = acc + over_dt<P2>(sf, c);
                     v = T(acc * (double)c.htilde[7]);
                 } else {
                     T acc = fma(sx, c.ihx2, fma(sy, c.ihy2, fma(sz, c.ihz2, b)));
@@ -1584,7 +1586,7 @@ __global__ void __launch_bounds__(128) rb_half_vec_kernel(T* __restrict__ U, con
                 if (rowint && k >= 1 && k <= d.nz - 2) continue;
                 auto rd = [&](int oi, int oj, int ok) { return oth[d.pidx(i + oi, j + oj, k + ok)]; };
                 const T sf = own[q + cc];
-                T v = gs_value<T>(c, d, i, j, k, bb[q + cc], sf, use_self != 0, rd);
+                T v = gs_value<T, P2>(c, d, i, j, k, bb[q + cc], sf, use_self != 0, rd);
                 if (relax) v = sf + omega * (v - sf);
                 own[q + cc] = v;
             }
@@ -1602,7 +1604,7 @@ struct RbRow<float> {
     static __device__ __forceinline__ float4 update(const GsCoef<float>& c, const float4& xm, const float4& xp,
                                                     const float4& ym, const float4& yp, const float4& zc,
                                                     const float4& zn, const float4& b, const float (&ht)[4],
-                                                    const float (&hl)[4])
+                                                    const float (&hl)[4], const bool (&)[4])
     {
         auto pair = [&](float2 a0, float2 a1, float2 b0, float2 b1, float2 c0, float2 c1, float2 bv, float2 h,
                         float2 l) {
@@ -1627,12 +1629,20 @@ struct RbRow<double> {
     static __device__ __forceinline__ double2 update(const GsCoef<double>& c, const double2& xm, const double2& xp,
                                                      const double2& ym, const double2& yp, const double2& zc,
                                                      const double2& zn, const double2& b, const double (&ht)[2],
-                                                     const double (&)[2])
+                                                     const double (&)[2], const bool (&live)[2])
     {
-        double2 o;
-        o.x = (over_h2<0, P2>(xm.x + xp.x, c) + over_h2<1, P2>(ym.x + yp.x, c) + over_h2<2, P2>(zc.x + zn.x, c) + b.x) * ht[0];
-        o.y = (over_h2<0, P2>(xm.y + xp.y, c) + over_h2<1, P2>(ym.y + yp.y, c) + over_h2<2, P2>(zc.y + zn.y, c) + b.y) * ht[1];
-        return o;
+        auto one = [&](double sx, double sy, double sz, double bv, double h, bool lv) {
+            // (the neighbours of a cell on a face or past the row are often 0, which the division
+            // takes a slow path for)
+            if constexpr (!P2) {
+                sx = lv ? sx : 1.;
+                sy = lv ? sy : 1.;
+                sz = lv ? sz : 1.;
+            }
+            return (over_h2<0, P2>(sx, c) + over_h2<1, P2>(sy, c) + over_h2<2, P2>(sz, c) + bv) * h;
+        };
+        return make_double2(one(xm.x + xp.x, ym.x + yp.x, zc.x + zn.x, b.x, ht[0], live[0]),
+                            one(xm.y + xp.y, ym.y + yp.y, zc.y + zn.y, b.y, ht[1], live[1]));
     }
 };
 
@@ -1723,12 +1733,14 @@ __device__ __forceinline__ typename V16<T>::type rb_group(const GsCoef<T>& c, co
             }
         }
     }
-    VV v = RbRow<T>::template update<P2>(c, xm, xp, ym, yp, zc, zn, bv, ht, hl);
+    bool live[W];  // cells that keep the formula's value
 #pragma unroll
-    for (int cc = 0; cc < W; ++cc) {
-        if (!NEU && ((cc == 0 && first_k) || (last_k && cc == last))) VT::set(v, cc, c.bc);
-        if (cc > last) VT::set(v, cc, T(0));
-    }
+    for (int cc = 0; cc < W; ++cc)
+        live[cc] = cc <= last && (NEU || !((cc == 0 && first_k) || (last_k && cc == last)));
+    VV v = RbRow<T>::template update<P2>(c, xm, xp, ym, yp, zc, zn, bv, ht, hl, live);
+#pragma unroll
+    for (int cc = 0; cc < W; ++cc)
+        if (!live[cc]) VT::set(v, cc, NEU || cc > last ? T(0) : c.bc);
     return v;
 }
 
@@ -1757,7 +1769,8 @@ __device__ __forceinline__ typename V16<T>::type rb_group(const GsCoef<T>& c, co
 // around a block), DRAM for b_eff. Measured us per half-sweep in sequence, against the
 // general kernel's form of it (54 instructions per cell): 256^3 FP32 17.0 -> 14.0,
 // 512x512x320 88.6 -> 83.4, 160^3 5.2 -> 4.0, 171x203x117 FP32 Neumann 14.0 -> 5.7,
-// 128^3 FP64 7.5 -> 4.9 and 200^3 FP64 28.4 -> 17.9 (no division per cell, over_h2).
+// 128^3 FP64 7.5 -> 4.7 and 200^3 FP64 28.4 -> 17.3 (no division per cell, over_h2), with
+// spacings that need the divisions 7.6 -> 7.2 and 28.4 -> 27.8.
 template <typename T, int NI, int BC, typename IX, bool P2 = false>
 __device__ __forceinline__ void rb_march_body(const uint3 blockIdx, const dim3 gridDim, T* __restrict__ own,
                                               const T* oth, const T* bb, const Dims& d,

@@ -130,8 +130,12 @@ struct RbHalfJob {
     __device__ __forceinline__ void operator()(uint3 b, dim3 g, int flag) const
     {
         const long long npk = d.npk();
-        rb_march_body<T, NI, BC, long long>(b, g, U + (color ? npk : 0), U + (color ? 0 : npk), B + (color ? npk : 0),
-                                            d, c, color, reverse, flag);
+        T* own = U + (color ? npk : 0);
+        const T *oth = U + (color ? 0 : npk), *bb = B + (color ? npk : 0);
+        if (sizeof(T) == 8 && (c.pow2 & 7) == 7)
+            rb_march_body<T, NI, BC, long long, true>(b, g, own, oth, bb, d, c, color, reverse, flag);
+        else
+            rb_march_body<T, NI, BC, long long, false>(b, g, own, oth, bb, d, c, color, reverse, flag);
     }
 };
 
