@@ -1090,10 +1090,9 @@ __device__ __forceinline__ void div_body(const uint3 blockIdx, const dim3 gridDi
         if (jint && i >= 1 && i <= d.nx - 2) {
             const T tx = over_two_h<0>(x[t + 2] - x[t], hs);
             const T ty = over_two_h<1>(yp[t] - ym[t], hs);
-            const T mid = over_two_h<2>(z0[t] - z1[t], hs);
-            const T lo = over_two_h<2>(T(4) * z0[t] - T(3) * zc[t] - z1[t], hs);
-            const T hi = over_two_h<2>(T(3) * zc[t] - T(4) * z0[t] + z1[t], hs);
-            r = tx + ty + (k == 0 ? lo : (k == d.nz - 1 ? hi : mid));
+            // one division for the three forms of the z term
+            const T lo = T(4) * z0[t] - T(3) * zc[t] - z1[t], hi = T(3) * zc[t] - T(4) * z0[t] + z1[t];
+            r = tx + ty + over_two_h<2>(k == 0 ? lo : (k == d.nz - 1 ? hi : z0[t] - z1[t]), hs);
         } else {
             r = div_point(f0, f1, f2, d, i, j, k, hs);
         }
