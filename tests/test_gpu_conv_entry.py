@@ -52,3 +52,12 @@ def test_refused_width_leaves_nothing_running(pkg, nz):
             c.conv3d_bf16(x, w, b)
         assert stream.query()
         c.set_stream(None)
+
+
+@pytest.mark.parametrize("cout, dims", [(32, (3, 6, 112)), (64, (6, 12, 128)), (32, (2, 5, 256)), (64, (9, 3, 96))])
+def test_64_channels_on_wide_rows(ctx, cout, dims):
+    """64 staged channels and 32 outputs per block leave room for one tile row only on rows of
+    112 and more."""
+    x, w, b = _inputs(3, dims=dims, cin=64, cout=cout)
+    got = ctx.conv3d_bf16(x.cuda(), w, b)
+    assert rel(got.cpu().double().numpy(), _want(x, w, b)) <= 1e-5
