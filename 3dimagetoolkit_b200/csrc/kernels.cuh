@@ -1733,14 +1733,16 @@ __device__ __forceinline__ typename V16<T>::type rb_group(const GsCoef<T>& c, co
             }
         }
     }
-    bool live[W];  // cells that keep the formula's value
+    bool live[W];  // cells that keep the formula's value (read by the form with divisions only)
 #pragma unroll
     for (int cc = 0; cc < W; ++cc)
         live[cc] = cc <= last && (NEU || !((cc == 0 && first_k) || (last_k && cc == last)));
     VV v = RbRow<T>::template update<P2>(c, xm, xp, ym, yp, zc, zn, bv, ht, hl, live);
 #pragma unroll
-    for (int cc = 0; cc < W; ++cc)
-        if (!live[cc]) VT::set(v, cc, NEU || cc > last ? T(0) : c.bc);
+    for (int cc = 0; cc < W; ++cc) {
+        if (!NEU && ((cc == 0 && first_k) || (last_k && cc == last))) VT::set(v, cc, c.bc);
+        if (cc > last) VT::set(v, cc, T(0));
+    }
     return v;
 }
 
