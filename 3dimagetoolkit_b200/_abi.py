@@ -299,7 +299,10 @@ class Context:
         b = None if bias is None else bias.to(device=x.device, dtype=torch.float32).contiguous()
         out = torch.empty((nsamp, D, H, W, cout), dtype=torch.float32, device=x.device)
         # the convolution runs on the context's own stream, x, w and b are written on torch's
-        torch.cuda.current_stream(x.device).synchronize()
+        # (the library itself waits for the default stream)
+        stream = torch.cuda.current_stream(x.device)
+        if stream.cuda_stream:
+            stream.synchronize()
         self._check(lib().im3d_conv3d_bf16(self._h, C.c_void_p(x.data_ptr()), C.c_int(pitch), C.c_int(c_off),
                                            C.c_int(cin), C.c_void_p(w.data_ptr()),
                                            C.c_void_p(b.data_ptr() if b is not None else 0), C.c_int(cout),
